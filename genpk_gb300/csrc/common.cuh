@@ -6,6 +6,37 @@
 
 namespace genpk {
 
+// A pass's constants from its total mass m and its largest |mass| mref: the
+// shift s of the 2^-s mass units, which maps mref into [2^27, 2^28) units, so
+// that one CIC weight is below 2^28 (32-bit accumulators carry at most once
+// per 2^4 adds) and 64-bit cell sums hold 2^35 full-mass particles; and the
+// mean in those units, rounded to 24 significant bits (exactly representable in
+// FP32 after the final 2^-s scaling).  On the host for a uniform mass, on the
+// device for others: the same IEEE operations in the same order, the same bits.
+struct PassConsts {
+    double mass;
+    int fx_shift;
+    long long mean_fixed;
+};
+
+__host__ __device__ inline PassConsts pass_consts(double m, float mref, double inv_cells)
+{
+    int s = 0;
+    if (mref > 0.f && isfinite(mref))
+        s = 27 - ilogbf(mref);
+    s = s < -100 ? -100 : s > 100 ? 100 : s;
+    const double mf = m * inv_cells * ldexp(1.0, s);
+    long long mean_fixed;
+    const double amf = fabs(mf);
+    if (amf >= 16777216.0) {
+        const double q = ldexp(1.0, ilogb(amf) - 23);
+        mean_fixed = (long long)(rint(mf / q) * q);
+    } else {
+        mean_fixed = llrint(mf);
+    }
+    return {m, s, mean_fixed};
+}
+
 // Position -> (wrapped cell, fraction) for one axis, as fieldize.cpp:66-76
 // computes it in FP64: x = pos*units, f = floor(x), d = x - f, f wrapped mod N.
 //
@@ -192,6 +223,53 @@ __device__ __forceinline__ AxisQ split_q28_unwrapped(float p, float xh, float uh
     const int carry = q >> kFracBits;
     u = fmaf(2.f, (float)carry, u);
     return {(int)f + carry, (uint32_t)q & (kFracOne - 1u), u, xl};
+}
+
+// split_q28 of the three axes of a particle whose floor(xh) lies in [0, dims)
+// on each axis and whose fraction does not carry into another cell: the same
+// cells, fractions, u and xl.  Returns false (a undefined) for every other
+// particle (outside the box, carries, non-finite positions), which takes
+// split_q28 itself.
+//   * xh + 1.5 * 2^23 rounded down holds floor(xh) in its low bits (0 <= xh <
+//     2^22), so the cell needs no float-to-int conversion; any xh outside that
+//     range, infinite or NaN leaves a bit pattern outside [0, dims).
+//   * xl * 2^28 + 1.5 * 2^23 holds round(xl * 2^28) in its low bits: |xl| <=
+//     xh * 2^-23, so |xl * 2^28| < 2^22 up to 2^17 cells.
+//   * a = xh - floor(xh) is exact, and 1 - 2a rounds only in cell 0; its
+//     rounding error goes into xl as split_q28 puts it there (CORNER: u and xl
+//     are wanted).
+// 13 instructions an axis (9 without u) and one conversion, against 18 with
+// three conversions (which run at a quarter rate) and the carry.
+constexpr int kMagicBits = 0x4b400000;  // 1.5 * 2^23 as a float's bits
+
+template <bool CORNER>
+__device__ __forceinline__ void split_axis_fast(float p, float uh, float ul, AxisQ &o)
+{
+    const float xh = __fmul_rn(p, uh);
+    const float xe = fmaf(p, uh, -xh);
+    const float xl = fmaf(p, ul, xe);
+    const float r = __fadd_rd(xh, 12582912.f);
+    const float a = __fsub_rn(xh, __fsub_rn(r, 12582912.f));
+    o.q = (uint32_t)(__float2int_rn(a * 268435456.f) +
+                     (__float_as_int(fmaf(xl, 268435456.f, 12582912.f)) - kMagicBits));
+    o.cell = __float_as_int(r) - kMagicBits;
+    if (CORNER) {
+        o.u = fmaf(-2.f, a, 1.f);
+        const float err = fmaf(-2.f, a, __fsub_rn(1.f, o.u));  // (1 - 2a) - u, exact
+        o.xl = fmaf(-0.5f, err, xl);
+    }
+}
+
+template <bool CORNER>
+__device__ __forceinline__ bool split3_fast(float x, float y, float z, float uh, float ul, int dims,
+                                            AxisQ a[3])
+{
+    split_axis_fast<CORNER>(x, uh, ul, a[0]);
+    split_axis_fast<CORNER>(y, uh, ul, a[1]);
+    split_axis_fast<CORNER>(z, uh, ul, a[2]);
+    return max((uint32_t)a[0].cell, max((uint32_t)a[1].cell, (uint32_t)a[2].cell)) <
+               (uint32_t)dims &&
+           ((a[0].q | a[1].q | a[2].q) >> kFracBits) == 0u;
 }
 
 __device__ __forceinline__ int wrap_cell(int fi, int dims)

@@ -89,32 +89,6 @@ struct WinParams {
     double *field_mass, *field_sub;
 };
 
-// The pass constants of k_window_prep, on the host for a uniform mass (the
-// same IEEE operations in the same order: the same bits).
-struct PassConsts {
-    double mass;
-    int fx_shift;
-    long long mean_fixed;
-};
-
-__host__ __device__ inline PassConsts pass_consts(double m, float mref, double inv_cells)
-{
-    int s = 0;
-    if (mref > 0.f && isfinite(mref))
-        s = 27 - ilogbf(mref);
-    s = max(-100, min(100, s));
-    const double mf = m * inv_cells * ldexp(1.0, s);
-    long long mean_fixed;
-    const double amf = fabs(mf);
-    if (amf >= 16777216.0) {
-        const double q = ldexp(1.0, ilogb(amf) - 23);
-        mean_fixed = (long long)(rint(mf / q) * q);
-    } else {
-        mean_fixed = llrint(mf);
-    }
-    return {m, s, mean_fixed};
-}
-
 // Thread 0 of CTA 0: the host-computed constants into the status words and
 // the grid's running sums (a uniform-mass pass without k_window_prep).
 __device__ __forceinline__ void store_host_prep(const WinParams &p, DeviceStatus *st)

@@ -99,9 +99,8 @@ struct genpk_ctx {
         int band = 0;
         bool var = false;
         bool with_stream = false;         // the stream engine was among the trials
-        int engine = GENPK_ENGINE_SORTED;  // the faster: SORTED (tile, per_sm) or STREAM
+        int engine = GENPK_ENGINE_SORTED;  // the faster: SORTED (with this tile) or STREAM
         TileShape tile{16, 16, 16};
-        int per_sm = 1;
     };
     static constexpr int kTuned = 16;
     Tuned tuned[kTuned];
@@ -122,6 +121,10 @@ struct genpk_ctx {
     // 64-bit accumulator: the forward transform reads it from there (the
     // conversion pass is skipped); anything else converts it first.
     int acc_pending = -1;
+    // A field whose latest (clean) sorted-engine pass is headed for the own z, y
+    // and x passes (own_transform_limit); any later pass on the context ends
+    // that, as it would convert a pending accumulator.
+    int own_pending = -1;
     // The accumulator holds zeros (the transform's x pass cleared it after its
     // contents were used), so the next window pass skips its clear;
     // acc_spent: its contents were used (converted or read by the z pass) and
@@ -143,6 +146,7 @@ struct genpk_ctx {
         int64_t n = -1;
         double boxsize = 0.0;
         int engine = 0, chunk = 0;
+        bool no_order = false;  // the particles showed no spatial order: tuned
     };
     static constexpr int kChoices = 32;  // species of a loop, or a batch of boxes per grid size
     Choice choices[kChoices];
@@ -297,8 +301,9 @@ const float *mapped_host(const float *p)
     return (const float *)a.devicePointer;
 }
 
+// zeroed: the new memory is cleared (for buffers that every pass leaves zero).
 template <typename T>
-int grow(genpk_ctx *ctx, T **ptr, size_t *cap, size_t need)
+int grow(genpk_ctx *ctx, T **ptr, size_t *cap, size_t need, bool zeroed = false)
 {
     if (*cap >= need)
         return GENPK_OK;
@@ -310,6 +315,8 @@ int grow(genpk_ctx *ctx, T **ptr, size_t *cap, size_t need)
     }
     GENPK_CUDA(cudaMalloc((void **)ptr, sizeof(T) * need));
     *cap = need;
+    if (zeroed)
+        GENPK_CUDA(cudaMemsetAsync(*ptr, 0, sizeof(T) * need, ctx->stream));
     return GENPK_OK;
 }
 
@@ -423,26 +430,35 @@ DepositGeom deposit_geom(genpk_ctx *ctx, double boxsize)
 
 int ensure_stage(genpk_ctx *ctx, int64_t need);
 
-// Scratch of one sorted-engine pass of n particles with geometry g.
-int grow_sorted_scratch(genpk_ctx *ctx, const DepositGeom &g, int64_t n, int sort_ctas)
+// Scratch of one sorted-engine pass of n particles with geometry g (nbox boxes
+// of a grouped pass, n particles in all).
+int grow_sorted_scratch(genpk_ctx *ctx, const DepositGeom &g, int64_t n, int sort_ctas, int nbox,
+                        size_t hdr_words)
 {
     DepositScratch &s = ctx->dscr;
-    if (deposit_shared_hist(g)) {
-        GENPK_TRY(grow(ctx, &s.hist, &s.hist_cap, (size_t)sort_ctas * g.ntiles));
+    const size_t nb = (size_t)nbox;
+    if (deposit_binned(g)) {
+        GENPK_TRY(grow(ctx, &s.hdr, &s.hdr_cap, std::max<size_t>(hdr_words, 1)));
     } else {
-        GENPK_TRY(grow(ctx, &s.cursor, &s.cursor_cap, (size_t)g.ntiles));
+        GENPK_TRY(grow(ctx, &s.tile_start, &s.tile_start_cap, nb * (g.ntiles + 1)));
+        GENPK_TRY(grow(ctx, &s.totals, &s.tile_cap, nb * g.ntiles, true));
+        GENPK_TRY(grow(ctx, &s.cursor, &s.cursor_cap, nb * deposit_cursor_words(g)));
     }
-    GENPK_TRY(grow(ctx, &s.tile_start, &s.tile_start_cap, (size_t)g.ntiles + 1));
-    GENPK_TRY(grow(ctx, &s.totals, &s.tile_cap, (size_t)g.ntiles + 1));
+    GENPK_TRY(grow(ctx, &s.ticket, &s.ticket_cap, (size_t)kMaxGroupBoxes, true));
     GENPK_TRY(grow(ctx, &s.sorted, &s.sorted_cap, (size_t)std::max<int64_t>(n, 1)));
     size_t nface = 0, nhalo = 0;
     deposit_scratch_sizes(g, &nface, &nhalo);
-    GENPK_TRY(grow(ctx, &s.faces, &s.faces_cap, nface));
-    GENPK_TRY(grow(ctx, &s.halo, &s.halo_cap, nhalo));
+    GENPK_TRY(grow(ctx, &s.faces, &s.faces_cap, nface * nb));
+    GENPK_TRY(grow(ctx, &s.halo, &s.halo_cap, nhalo * nb));
     size_t mp = (size_t)s.mass_part_cap;
-    GENPK_TRY(grow(ctx, &s.mass_part, &mp, (size_t)sort_ctas));
+    GENPK_TRY(grow(ctx, &s.mass_part, &mp, (size_t)2 * sort_ctas));  // + corner partials
     s.mass_part_cap = (int)mp;
     return GENPK_OK;
+}
+
+int grow_sorted_scratch(genpk_ctx *ctx, const DepositGeom &g, int64_t n, int sort_ctas)
+{
+    return grow_sorted_scratch(ctx, g, n, sort_ctas, 1, deposit_header_words(g, n, sort_ctas));
 }
 
 // Particle-density band of a pass: half octaves of particles per cell.
@@ -459,9 +475,8 @@ constexpr int kTuneReps = 2;
 
 // The deposit autotuner for particle orders without spatial coherence.  On
 // the first clean pass of a density band (and mass kind) it runs the pass once
-// per candidate -- the sorted engine with tiles 8^3, 16x16x8 and 16^3, each
-// with up to 1, 2 and 4 sort CTAs per SM, and (with_stream) the stream
-// engine, whose reductions go straight to the accumulator -- timed with CUDA
+// per candidate -- the sorted engine with tiles 8^3, 16x16x8 and 16^3, and
+// (with_stream) the stream engine, whose reductions go straight to the accumulator -- timed with CUDA
 // events, and keeps the fastest.  (Measured on uniform random particles: the
 // stream engine is 2-2.6x faster at 1e6 particles, where the sort's fixed
 // costs dominate, about even at 3e7 on a 128^3 grid, and 1.75x slower at 3e7
@@ -474,10 +489,6 @@ int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, boo
                 const genpk_ctx::Tuned **out)
 {
     static const TileShape tiles[] = {{8, 8, 8}, {16, 16, 8}, {16, 16, 16}};
-    // sort CTAs per SM: fewer CTAs give each (CTA, tile) run of the scatter
-    // more particles, so its 16-byte records share sectors in the L2; more
-    // shorten a CTA's range (two waves of 1024-thread CTAs)
-    static const int pers[] = {1, 2};
     const size_t stash = 0;  // the error counters are kept in the probe buffer meanwhile
     GENPK_TRY(grow(ctx, &ctx->d_probe, &ctx->probe_cap, (size_t)4));
     GENPK_CUDA(cudaMemcpyAsync(ctx->d_probe + stash, ctx->d_status, 2 * sizeof(long long),
@@ -549,38 +560,31 @@ int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, boo
     for (const TileShape &t : tiles) {
         if (!deposit_tile_supported(t.tx, t.ty, t.tz))
             continue;
-        int last_ctas = -1;
-        for (int per : pers) {
-            const DepositGeom g = deposit_geom(ctx, boxsize, t);
-            const int ctas = deposit_sort_ctas(g, a.n, ctx->num_sms, per);
-            if (ctas == last_ctas)  // capped to the same count: nothing new to try
-                continue;
-            last_ctas = ctas;
-            GENPK_TRY(grow_sorted_scratch(ctx, g, a.n, ctas));
-            float ms = 1e30f;
-            for (int rep = 0; rep < kTuneReps; rep++) {
-                GENPK_TRY(reset_field());
-                GENPK_CUDA(cudaEventRecord(e0, ctx->stream));
-                GENPK_CUDA(deposit_pass(g, a, ctx->dscr, ctx->d_status, ctas, ctx->stream,
-                                        &ctx->launches, nullptr, nullptr));
-                GENPK_CUDA(cudaEventRecord(e1, ctx->stream));
-                GENPK_CUDA(cudaEventSynchronize(e1));
-                float t = 0.f;
-                GENPK_CUDA(cudaEventElapsedTime(&t, e0, e1));
-                ms = std::min(ms, t);
-            }
-            if (ctx->ntrials < genpk_ctx::kMaxTrials) {
-                ctx->trial_tile[ctx->ntrials] = t;
-                ctx->trial_ctas[ctx->ntrials] = ctas;
-                ctx->trial_ms[ctx->ntrials] = ms;
-                ctx->ntrials++;
-            }
-            if (ms < best_ms) {
-                best_ms = ms;
-                best.engine = GENPK_ENGINE_SORTED;
-                best.tile = t;
-                best.per_sm = per;
-            }
+        const DepositGeom g = deposit_geom(ctx, boxsize, t);
+        const int ctas = deposit_sort_ctas(g, a.n, ctx->num_sms);
+        GENPK_TRY(grow_sorted_scratch(ctx, g, a.n, ctas));
+        float ms = 1e30f;
+        for (int rep = 0; rep < kTuneReps; rep++) {
+            GENPK_TRY(reset_field());
+            GENPK_CUDA(cudaEventRecord(e0, ctx->stream));
+            GENPK_CUDA(deposit_pass(g, a, ctx->dscr, ctx->d_status, ctas, ctx->stream,
+                                    &ctx->launches, nullptr, nullptr));
+            GENPK_CUDA(cudaEventRecord(e1, ctx->stream));
+            GENPK_CUDA(cudaEventSynchronize(e1));
+            float x = 0.f;
+            GENPK_CUDA(cudaEventElapsedTime(&x, e0, e1));
+            ms = std::min(ms, x);
+        }
+        if (ctx->ntrials < genpk_ctx::kMaxTrials) {
+            ctx->trial_tile[ctx->ntrials] = t;
+            ctx->trial_ctas[ctx->ntrials] = ctas;
+            ctx->trial_ms[ctx->ntrials] = ms;
+            ctx->ntrials++;
+        }
+        if (ms < best_ms) {
+            best_ms = ms;
+            best.engine = GENPK_ENGINE_SORTED;
+            best.tile = t;
         }
     }
     GENPK_TRY(reset_field());
@@ -602,6 +606,21 @@ const genpk_ctx::Tuned *find_tuned(const genpk_ctx *ctx, int64_t n, bool var, bo
             ctx->tuned[i].with_stream == with_stream)
             return &ctx->tuned[i];
     return nullptr;
+}
+
+// A pass of particles without spatial order takes the own z, y and x transform
+// passes where it has fewer particles than this (and at least
+// kTuneMinParticles), else the batched cuFFT ones, whichever engine deposits it:
+// the two transforms round differently, and with the transform tied to the
+// engine, whose choice is timed, a spectrum's last bits changed from run to run.
+// The line lies where the stream mode with the own passes and the sorted engine
+// with cuFFT took equal time (uniform random particles, ms of the deposit):
+// 0.069 and 0.079 at 2^20 particles on 128^3, 0.111 and 0.097 at 2^21; 0.131 and
+// 0.141 at 2^19 on 256^3, 0.175 and 0.155 at 2^20; 0.67 and 0.83 at 2^20 on
+// 512^3, 0.88 and 0.86 at 2^21.
+int64_t own_transform_limit(int64_t dims)
+{
+    return dims <= 128 ? (int64_t)3 << 19 : dims <= 256 ? (int64_t)3 << 18 : (int64_t)1 << 21;
 }
 
 // One deposit pass from device particle arrays, or (host_mapped) from pinned
@@ -700,6 +719,7 @@ int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const f
     const genpk_ctx::Tuned *tuned = nullptr;
     const bool auto_sorted = ctx->engine == GENPK_ENGINE_AUTO && engine == GENPK_ENGINE_SORTED &&
                              !ctx->tile_fixed && !host_mapped;
+    const bool no_order = auto_sorted || (reuse && hit->no_order);
     if (auto_sorted || (engine == GENPK_ENGINE_SORTED && !ctx->tile_fixed && !host_mapped)) {
         tuned = find_tuned(ctx, n, masses != nullptr, auto_sorted);
         if (!tuned && a.clean && n >= kTuneMinParticles) {
@@ -719,6 +739,7 @@ int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const f
             c.boxsize = boxsize;
             c.engine = engine;
             c.chunk = chunk;
+            c.no_order = no_order;
         }
         stage_event(ctx, "probe");
     }
@@ -761,14 +782,17 @@ int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const f
     a.host_mapped = host_mapped;
     ctx->last_engine = engine;
     timing_touch(ctx);
+    // A clean grid headed for the own z/y/x transform keeps a window or stream
+    // pass in the accumulator: the z pass converts it on the fly.
+    bool own = a.clean && chunked && (use_xfft(ctx) || use_kz(ctx));
+    if (no_order && use_xfft(ctx))
+        own = a.clean && n >= kTuneMinParticles && n < own_transform_limit(ctx->dims);
     if (chunked) {
         const int mass_ctas = ctx->num_sms * 4;
         size_t mp = (size_t)s.mass_part_cap;
         GENPK_TRY(grow(ctx, &s.mass_part, &mp, (size_t)mass_ctas));
         s.mass_part_cap = (int)mp;
-        // A clean grid headed for the own z/y/x transform keeps the pass in the
-        // accumulator: the z pass converts it on the fly.
-        const bool defer = a.clean && (use_xfft(ctx) || use_kz(ctx));
+        const bool defer = own;
         // (a pass that fails part-way must not leave the accumulator marked clear)
         const size_t clear = ctx->acc_zero ? 0 : ctx->acc_dirty_bytes ? ctx->acc_dirty_bytes
                                                                        : acc_bytes(ctx);
@@ -781,19 +805,16 @@ int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const f
         if (defer)
             ctx->acc_pending = f;
     } else {
-        TileShape tile = ctx->tile;
-        int per_sm = 1;
-        if (tuned) {
-            tile = tuned->tile;
-            per_sm = tuned->per_sm;
-        }
+        const TileShape tile = tuned ? tuned->tile : ctx->tile;
         const DepositGeom gs = deposit_geom(ctx, boxsize, tile);
-        const int sort_ctas = deposit_sort_ctas(gs, n, ctx->num_sms, per_sm);
+        const int sort_ctas = deposit_sort_ctas(gs, n, ctx->num_sms);
         GENPK_TRY(grow_sorted_scratch(ctx, gs, n, sort_ctas));
         ctx->last_tile = tile;
         ctx->last_sort_ctas = sort_ctas;
         GENPK_CUDA(deposit_pass(gs, a, s, ctx->d_status, sort_ctas, ctx->stream, &ctx->launches,
                                 hook, ctx));
+        if (own && use_xfft(ctx))
+            ctx->own_pending = f;
     }
     ctx->state[(size_t)f] = F_DENSITY;
     ctx->auto_valid[(size_t)f] = false;
@@ -803,6 +824,7 @@ int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const f
 // The pending accumulator (if any) into its FP32 grid.
 int flush_acc(genpk_ctx *ctx)
 {
+    ctx->own_pending = -1;
     if (ctx->acc_pending < 0)
         return GENPK_OK;
     const int f = ctx->acc_pending;
@@ -1120,8 +1142,9 @@ int to_spectrum(genpk_ctx *ctx, const std::vector<int> &need, FusedAuto *fused =
     // by the own z pass (which reads the accumulator) and y pass; other runs of
     // consecutive fields take one batched 2-D cuFFT over their x-planes.  Both
     // then run the x pass.
-    const int pend = planes ? ctx->acc_pending : -1;
-    if (ctx->acc_pending >= 0 && (pend < 0 || std::find(todo.begin(), todo.end(), pend) == todo.end()))
+    const int pend = !planes ? -1 : ctx->own_pending >= 0 ? ctx->own_pending : ctx->acc_pending;
+    if ((ctx->acc_pending >= 0 || ctx->own_pending >= 0) &&
+        (pend < 0 || std::find(todo.begin(), todo.end(), pend) == todo.end()))
         GENPK_TRY(flush_acc(ctx));
     timing_touch(ctx);
     stage_event(ctx, "host");
@@ -1135,10 +1158,15 @@ int to_spectrum(genpk_ctx *ctx, const std::vector<int> &need, FusedAuto *fused =
         float *base = grid_of(ctx, todo[i]);
         if (planes) {
             if (todo[i] == pend) {
-                GENPK_CUDA(zfft_pass(ctx->gg, base, ctx->dscr.win_acc, ctx->d_xtw, ctx->d_status,
-                                     ctx->num_sms, ctx->stream, &ctx->launches));
-                ctx->acc_pending = -1;
-                ctx->acc_spent = true;
+                const bool from_acc = ctx->own_pending < 0;
+                GENPK_CUDA(zfft_pass(ctx->gg, base, from_acc ? ctx->dscr.win_acc : nullptr,
+                                     ctx->d_xtw, ctx->d_status, ctx->num_sms, ctx->stream,
+                                     &ctx->launches));
+                ctx->own_pending = -1;
+                if (from_acc) {
+                    ctx->acc_pending = -1;
+                    ctx->acc_spent = true;
+                }
                 stage_event(ctx, "zfft");
                 GENPK_CUDA(yfft_pass(ctx->gg, base, 1, ctx->d_xtw, ctx->num_sms, ctx->stream,
                                      &ctx->launches));
@@ -1246,8 +1274,9 @@ int power_impl(genpk_ctx *ctx, int np, const int *pairs, const double *pair_mass
     // The auto spectra of consecutive fields still to be transformed in one
     // batch (a batch's grouped boxes): each binned inside the x pass, one
     // histogram per field.
+    const int single = ctx->own_pending >= 0 ? ctx->own_pending : ctx->acc_pending;
     bool autos = np > 1 && use_xfft(ctx) && xfft_bin_supported(ctx->dims, nrb) &&
-                 (ctx->acc_pending < pairs[0] || ctx->acc_pending >= pairs[0] + np);
+                 (single < pairs[0] || single >= pairs[0] + np);
     for (int q = 0; autos && q < np; q++)
         autos = pairs[2 * q] == pairs[0] + q && pairs[2 * q + 1] == pairs[2 * q] &&
                 pair_mass[2 * q] == pair_mass[2 * q + 1] &&
@@ -1411,6 +1440,7 @@ uint64_t issue_digest(const genpk_ctx *ctx)
     for (bool v : ctx->kzmajor)
         mix(v);
     mix((uint64_t)ctx->acc_pending);
+    mix((uint64_t)ctx->own_pending);
     mix(ctx->acc_zero);
     mix(ctx->acc_spent);
     mix(ctx->acc_dirty_bytes);
@@ -1429,8 +1459,9 @@ uint64_t issue_digest(const genpk_ctx *ctx)
     mix(ctx->r2c.size());
     for (const void *q : {(const void *)ctx->grids, (const void *)ctx->d_field_mass,
                           (const void *)ctx->d_status, (const void *)ctx->d_xtw, (const void *)ctx->fft_work,
-                          (const void *)ctx->dscr.hist, (const void *)ctx->dscr.tile_start,
-                          (const void *)ctx->dscr.totals, (const void *)ctx->dscr.cursor,
+                          (const void *)ctx->dscr.tile_start, (const void *)ctx->dscr.totals,
+                          (const void *)ctx->dscr.cursor, (const void *)ctx->dscr.ticket,
+                          (const void *)ctx->dscr.hdr,
                           (const void *)ctx->dscr.sorted, (const void *)ctx->dscr.faces,
                           (const void *)ctx->dscr.halo, (const void *)ctx->dscr.mass_part,
                           (const void *)ctx->dscr.win_acc, (const void *)ctx->d_probe,
@@ -1448,7 +1479,7 @@ struct IssueState {
     std::vector<bool> corner_valid, kzmajor, auto_valid;
     std::vector<double> auto_mass;
     std::vector<std::vector<double>> auto_power;
-    int acc_pending = -1;
+    int acc_pending = -1, own_pending = -1;
     bool acc_zero = false, acc_spent = false;
     size_t acc_dirty_bytes = 0;
     int last_engine = 0;
@@ -1457,7 +1488,7 @@ struct IssueState {
     explicit IssueState(const genpk_ctx *c)
         : state(c->state), corner_valid(c->corner_valid), kzmajor(c->kzmajor),
           auto_valid(c->auto_valid), auto_mass(c->auto_mass), auto_power(c->auto_power),
-          acc_pending(c->acc_pending), acc_zero(c->acc_zero), acc_spent(c->acc_spent),
+          acc_pending(c->acc_pending), own_pending(c->own_pending), acc_zero(c->acc_zero), acc_spent(c->acc_spent),
           acc_dirty_bytes(c->acc_dirty_bytes), last_engine(c->last_engine), deferred(c->deferred)
     {
     }
@@ -1470,6 +1501,7 @@ struct IssueState {
         c->auto_mass = auto_mass;
         c->auto_power = auto_power;
         c->acc_pending = acc_pending;
+        c->own_pending = own_pending;
         c->acc_zero = acc_zero;
         c->acc_spent = acc_spent;
         c->acc_dirty_bytes = acc_dirty_bytes;
@@ -1534,7 +1566,8 @@ void genpk_ctx_destroy(genpk_ctx *ctx)
     cudaFree(ctx->bdev.thr);
     cudaFree(ctx->bdev.iw);
     cudaFree(ctx->bdev.count);
-    cudaFree(ctx->dscr.hist);
+    cudaFree(ctx->dscr.ticket);
+    cudaFree(ctx->dscr.hdr);
     cudaFree(ctx->dscr.tile_start);
     cudaFree(ctx->dscr.totals);
     cudaFree(ctx->dscr.sorted);
@@ -1664,6 +1697,8 @@ int genpk_zero(genpk_ctx *ctx, int field)
         ctx->acc_pending = -1;  // its accumulator is not needed any more
         ctx->acc_spent = true;
     }
+    if (ctx->own_pending == field)
+        ctx->own_pending = -1;
     ctx->state[(size_t)field] = F_CLEAN;
     ctx->auto_valid[(size_t)field] = false;
     ctx->kzmajor[(size_t)field] = false;
@@ -2279,7 +2314,6 @@ struct genpk_batch {
         bool tuned = false;
         std::vector<int64_t> tuned_n;  // the particle counts it was tuned for
         TileShape tile = {16, 16, 16};
-        int per_sm = 1;
     };
     std::vector<Group> groups;
 
@@ -2420,38 +2454,21 @@ bool groupable(const genpk_batch *b, const double *boxsize, const float *const *
     return true;
 }
 
-// Scratch of a grouped pass in the group context's sorted-engine buffers.
-int grow_group_scratch(genpk_ctx *ctx, const DepositGeom &g, const GroupLayout &lay)
-{
-    DepositScratch &s = ctx->dscr;
-    const int nb = lay.nbox;
-    const int ctas = lay.cta0[nb];
-    GENPK_TRY(grow(ctx, &s.hist, &s.hist_cap, std::max<size_t>(1, (size_t)ctas * g.ntiles)));
-    GENPK_TRY(grow(ctx, &s.tile_start, &s.tile_start_cap, (size_t)nb * (g.ntiles + 1)));
-    GENPK_TRY(grow(ctx, &s.totals, &s.tile_cap, (size_t)nb * g.ntiles + 1));
-    GENPK_TRY(grow(ctx, &s.sorted, &s.sorted_cap, (size_t)std::max<int64_t>(lay.rec0[nb], 1)));
-    size_t nface = 0, nhalo = 0;
-    deposit_scratch_sizes(g, &nface, &nhalo);
-    GENPK_TRY(grow(ctx, &s.faces, &s.faces_cap, nface * nb));
-    GENPK_TRY(grow(ctx, &s.halo, &s.halo_cap, nhalo * nb));
-    size_t mp = (size_t)s.mass_part_cap;
-    GENPK_TRY(grow(ctx, &s.mass_part, &mp, (size_t)std::max(ctas, 1)));
-    s.mass_part_cap = (int)mp;
-    return GENPK_OK;
-}
-
 // One grouped pass of every box of group g into its field (which must be
 // clean, with zero field sums).
-int group_pass(genpk_batch::Group &g, const std::vector<GroupBox> &gb, TileShape tile, int per_sm)
+int group_pass(genpk_batch::Group &g, const std::vector<GroupBox> &gb, TileShape tile)
 {
     genpk_ctx *ctx = g.ctx;
     int64_t total = 0;
     for (const GroupBox &x : gb)
         total += x.n;
     const DepositGeom geo = deposit_geom(ctx, 1.0, tile);
-    const int ctas = deposit_sort_ctas(geo, std::max<int64_t>(total, 1), ctx->num_sms, per_sm);
+    const int ctas = deposit_sort_ctas(geo, std::max<int64_t>(total, 1), ctx->num_sms);
     const GroupLayout lay = deposit_group_layout((int)gb.size(), gb.data(), ctas);
-    GENPK_TRY(grow_group_scratch(ctx, geo, lay));
+    size_t words = 0;
+    for (int b = 0; b < lay.nbox; b++)
+        words += deposit_header_words(geo, gb[(size_t)b].n, lay.cta0[b + 1] - lay.cta0[b]);
+    GENPK_TRY(grow_sorted_scratch(ctx, geo, total, lay.cta0[lay.nbox], lay.nbox, words));
     GENPK_CUDA(deposit_group_pass(geo, lay, gb.data(), ctx->grids, ctx->gg.nfloat, ctx->d_field_mass,
                                   ctx->d_field_mass + ctx->nfields, ctx->d_field_mass + 2 * ctx->nfields,
                                   ctx->dscr, g.d_st, g.bad_dev, ctx->stream, &ctx->launches));
@@ -2461,13 +2478,12 @@ int group_pass(genpk_batch::Group &g, const std::vector<GroupBox> &gb, TileShape
     return GENPK_OK;
 }
 
-// The group's tile shape and sort CTAs per SM, timed as tune_sorted times
+// The group's tile shape, timed as tune_sorted times
 // the single-box candidates (the best of kTuneReps passes each); the trials
 // are kept in the group context (genpk_deposit_trials).
 int tune_group(genpk_batch::Group &g, const std::vector<GroupBox> &gb)
 {
     static const TileShape tiles[] = {{8, 8, 8}, {16, 16, 8}, {16, 16, 16}};
-    static const int pers[] = {1, 2};
     genpk_ctx *ctx = g.ctx;
     int64_t total = 0;
     for (const GroupBox &x : gb)
@@ -2489,34 +2505,26 @@ int tune_group(genpk_batch::Group &g, const std::vector<GroupBox> &gb)
         const DepositGeom geo = deposit_geom(ctx, 1.0, t);
         if (!deposit_shared_hist(geo))
             continue;
-        int last_ctas = -1;
-        for (int per : pers) {
-            const int ctas = deposit_sort_ctas(geo, std::max<int64_t>(total, 1), ctx->num_sms, per);
-            if (ctas == last_ctas)
-                continue;
-            last_ctas = ctas;
-            float ms = 1e30f;
-            for (int rep = 0; rep < kTuneReps; rep++) {
-                GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass, 0, sums, ctx->stream));
-                GENPK_CUDA(cudaEventRecord(e0, ctx->stream));
-                GENPK_TRY(group_pass(g, gb, t, per));
-                GENPK_CUDA(cudaEventRecord(e1, ctx->stream));
-                GENPK_CUDA(cudaEventSynchronize(e1));
-                float x = 0.f;
-                GENPK_CUDA(cudaEventElapsedTime(&x, e0, e1));
-                ms = std::min(ms, x);
-            }
-            if (ctx->ntrials < genpk_ctx::kMaxTrials) {
-                ctx->trial_tile[ctx->ntrials] = t;
-                ctx->trial_ctas[ctx->ntrials] = ctas;
-                ctx->trial_ms[ctx->ntrials] = ms;
-                ctx->ntrials++;
-            }
-            if (ms < best_ms) {
-                best_ms = ms;
-                g.tile = t;
-                g.per_sm = per;
-            }
+        float ms = 1e30f;
+        for (int rep = 0; rep < kTuneReps; rep++) {
+            GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass, 0, sums, ctx->stream));
+            GENPK_CUDA(cudaEventRecord(e0, ctx->stream));
+            GENPK_TRY(group_pass(g, gb, t));
+            GENPK_CUDA(cudaEventRecord(e1, ctx->stream));
+            GENPK_CUDA(cudaEventSynchronize(e1));
+            float x = 0.f;
+            GENPK_CUDA(cudaEventElapsedTime(&x, e0, e1));
+            ms = std::min(ms, x);
+        }
+        if (ctx->ntrials < genpk_ctx::kMaxTrials) {
+            ctx->trial_tile[ctx->ntrials] = t;
+            ctx->trial_ctas[ctx->ntrials] = ctx->last_sort_ctas;
+            ctx->trial_ms[ctx->ntrials] = ms;
+            ctx->ntrials++;
+        }
+        if (ms < best_ms) {
+            best_ms = ms;
+            g.tile = t;
         }
     }
     GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass, 0, sums, ctx->stream));
@@ -2559,7 +2567,7 @@ int group_issue(genpk_batch::Group &g, const double *boxsize, const float *const
         GENPK_TRY(tune_group(g, gb));
         g.tuned_n = counts;
     }
-    GENPK_TRY(group_pass(g, gb, g.tile, g.per_sm));
+    GENPK_TRY(group_pass(g, gb, g.tile));
     std::vector<int> pairs((size_t)2 * nf);
     std::vector<double> pm((size_t)2 * nf);
     for (int f = 0; f < nf; f++) {

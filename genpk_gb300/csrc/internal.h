@@ -52,14 +52,16 @@ struct DepositGeom {
 
 // Scratch the deposit pass needs; owned by the context, grown on demand.
 struct DepositScratch {
-    uint32_t *hist = nullptr;        // [sort_ctas][ntiles]; becomes the scatter offsets
-    size_t hist_cap = 0;             // elements
-    uint32_t *tile_start = nullptr;  // [ntiles + 1]
+    uint32_t *tile_start = nullptr;  // [ntiles + 1] per box
     size_t tile_start_cap = 0;
-    uint32_t *totals = nullptr;      // [ntiles]
+    uint32_t *totals = nullptr;      // [ntiles] per box; zero between passes
     size_t tile_cap = 0;
-    uint32_t *cursor = nullptr;      // [ntiles] scatter cursors (global-counter mode)
+    uint32_t *cursor = nullptr;      // [deposit_cursor_words] per box: next free slot of each tile
     size_t cursor_cap = 0;
+    uint32_t *ticket = nullptr;      // [kMaxGroupBoxes] finished sort CTAs; zero between passes
+    size_t ticket_cap = 0;
+    uint16_t *hdr = nullptr;         // binned passes: [chunk][tiles + 1, rounded up] run offsets
+    size_t hdr_cap = 0;
     uint4 *sorted = nullptr;         // [cap] packed tile-local particles (x,y,z words, mass bits)
     size_t sorted_cap = 0;           // particles
     long long *faces = nullptr;      // [ntiles][face cells] 64-bit low-face sums
@@ -80,6 +82,7 @@ struct DeviceStatus {
     long long alt_sum;                 // sum over cells of (-1)^(x+y+z) * cell, fixed point
     int fx_shift;                      // weights are accumulated as round(w * 2^fx_shift)
     unsigned max_mass_bits;            // max |mass| of the pass, as float bits
+    unsigned long long pass_bad;       // particles the current binned pass has skipped
 };
 
 struct DepositArgs {
@@ -106,10 +109,17 @@ struct TileShape {
 };
 bool deposit_tile_supported(int tx, int ty, int tz);
 TileShape deposit_default_tile(int dims, int64_t n);
-// Sort CTAs of a pass: up to max_per_sm per SM (fewer where the per-CTA tile
-// histogram leaves no room), and no more than one per 4096 particles.
-int deposit_sort_ctas(const DepositGeom &g, int64_t n, int num_sms, int max_per_sm = 1);
+// Particles a sort CTA takes at a time.
+constexpr int kSortChunkParticles = 4096;
+// Sort CTAs of a pass: two per SM (one where the per-CTA tile histogram leaves
+// no room for two), and no more than one per chunk.
+int deposit_sort_ctas(const DepositGeom &g, int64_t n, int num_sms);
 size_t deposit_hist_smem(const DepositGeom &g);
+size_t deposit_cursor_words(const DepositGeom &g);
+// True when a pass sorts chunks in shared memory (deposit.cu k_bin_sort); the
+// 16-bit words of chunk headers it needs for n particles on `ctas` sort CTAs.
+bool deposit_binned(const DepositGeom &g);
+size_t deposit_header_words(const DepositGeom &g, int64_t n, int ctas);
 // True when the per-CTA tile histogram fits in shared memory (else the pass
 // uses global counters).
 bool deposit_shared_hist(const DepositGeom &g);
@@ -147,12 +157,12 @@ struct GroupLayout {
     int64_t rec0[kMaxGroupBoxes + 1];
 };
 // The pass's sort CTAs (deposit_sort_ctas over all the boxes' particles)
-// shared out in proportion to the boxes' particles: at least one for a box
-// with particles, none for an empty box, at most one per 4096 particles.
+// shared out in proportion to the boxes' particles: at least one for each box,
+// at most one per chunk.
 GroupLayout deposit_group_layout(int nbox, const GroupBox *boxes, int sort_ctas);
 // Scratch elements a grouped pass needs beyond deposit_scratch_sizes per box:
-// hist cta0[nbox] x ntiles, tile_start nbox x (ntiles + 1), totals
-// nbox x ntiles, sorted rec0[nbox], mass_part cta0[nbox].  Requires
+// tile_start nbox x (ntiles + 1), totals nbox x ntiles (zeroed once), cursor
+// nbox x deposit_cursor_words, sorted rec0[nbox], mass_part cta0[nbox].  Requires
 // deposit_shared_hist(g), nbox <= kMaxGroupBoxes and rec0[nbox] < 2^32.
 // bad_out (device-visible, one word per box, may be null) receives each box's
 // count of skipped particles, and the status word is zeroed for the next pass.
@@ -263,7 +273,8 @@ int xfft_bin_ctas(int dims, int nbatch, int num_sms);
 // The z and y transforms of every x-plane for xfft_supported sizes (xfft.cu):
 // zfft_pass is the length-N r2c along z of one grid, read from the window
 // engine's 64-bit accumulator (converted as its conversion pass does, with the
-// pass's mean and scale in dstat) and written to `grid`; yfft_pass is the
+// pass's mean and scale in dstat) and written to `grid`, or (acc null) in place
+// from the FP32 density in `grid`; yfft_pass is the
 // complex length-N pass along y.  Followed by xfft_pass they leave the 3-D r2c
 // transform.  xfft_pass also stores zeros over `zero_bytes` (a multiple of 16)
 // at `zero`, when not null, spread over its tiles: the accumulator's clear for

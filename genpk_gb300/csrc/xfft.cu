@@ -701,10 +701,12 @@ __global__ void __launch_bounds__(kXThreads, kXCtasPerSm)
 //      R < 8, five radix-2 shuffle stages across the warp;
 //   3. X[k] = E[k] + W_N^k O[k], k = 0..M, with E = (Z[k] + conj Z[M-k]) / 2
 //      and O = (Z[k] - conj Z[M-k]) / 2i.
-// The input is the window engine's 64-bit accumulator, converted as
+// The input (T) is the window engine's 64-bit accumulator, converted as
 // k_window_convert does (accumulator minus the fixed-point mean, rounded
-// once), so that pass is skipped; the output is the FP32 grid's row.  Rows are
-// prefetched one row ahead by 16-byte asynchronous copies into a per-warp
+// once), so that pass is skipped, or the FP32 grid itself, in place (the
+// sorted engine's passes); the output is the FP32 grid's row, with the same
+// bits from either.  Rows are prefetched one row ahead by 16-byte (FP32 rows,
+// which are 8-byte aligned: 8-byte) asynchronous copies into a per-warp
 // buffer; each lane copies and later reads only its own chunks, so the buffer
 // needs no warp synchronisation.
 constexpr int kZThreads = 256;
@@ -714,6 +716,33 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src)
                  : "memory");
 }
+
+__device__ __forceinline__ void cp_async8(void *dst, const void *src, unsigned src_bytes)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src),
+                 "r"(src_bytes)
+                 : "memory");
+}
+
+// Two consecutive reals of a row, as k_zfft reads them.
+template <typename T>
+struct ZPair;
+template <>
+struct ZPair<unsigned long long> {
+    typedef longlong2 V;
+    static __device__ __forceinline__ void copy(V *dst, const V *src) { cp_async16(dst, src); }
+    static __device__ __forceinline__ float2 value(const V &a, long long mean, float inv_scale)
+    {
+        return make_float2(i64_to_f32_rn(a.x - mean) * inv_scale,
+                           i64_to_f32_rn(a.y - mean) * inv_scale);
+    }
+};
+template <>
+struct ZPair<float> {
+    typedef float2 V;
+    static __device__ __forceinline__ void copy(V *dst, const V *src) { cp_async8(dst, src, 8u); }
+    static __device__ __forceinline__ float2 value(const V &a, long long, float) { return a; }
+};
 
 __device__ __forceinline__ int zpad(int i)
 {
@@ -729,27 +758,28 @@ __device__ __forceinline__ float2 dif_shfl(float2 v, int s, bool upper, float2 w
     return upper ? cmul(csub(q, v), w) : cadd(v, q);
 }
 
-template <int N>
+template <int N, typename T>
 __global__ void __launch_bounds__(kZThreads)
-    k_zfft(const unsigned long long *__restrict__ acc, float *grid, int64_t nrows,
-           int row_floats, const float2 *__restrict__ tw_g, const DeviceStatus *__restrict__ st)
+    k_zfft(const T *in, float *grid, int64_t nrows, int row_floats,
+           const float2 *__restrict__ tw_g, const DeviceStatus *__restrict__ st)
 {
+    typedef typename ZPair<T>::V V;
     constexpr int M = N / 2;
     constexpr int R = M / 32;
     __shared__ float2 tw[N];
     __shared__ float2 zs_all[kZThreads / 32][M + M / 32];  // Z[k] (or exchange) at zpad(k)
-    extern __shared__ __align__(16) unsigned char zdyn[];  // [warps][M] longlong2
+    extern __shared__ __align__(16) unsigned char zdyn[];  // [warps][M] V
     for (int i = threadIdx.x; i < N; i += blockDim.x)
         tw[i] = tw_g[i];
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float2 *zs = zs_all[wid];
-    longlong2 *pre = reinterpret_cast<longlong2 *>(zdyn) + wid * M;
+    V *pre = reinterpret_cast<V *>(zdyn) + wid * M;
     auto prefetch = [&](int64_t r) {
-        const longlong2 *src = reinterpret_cast<const longlong2 *>(acc + (size_t)r * row_floats);
+        const V *src = reinterpret_cast<const V *>(in + (size_t)r * row_floats);
 #pragma unroll
         for (int m = 0; m < R; m++)
-            cp_async16(pre + lane + 32 * m, src + lane + 32 * m);
+            ZPair<T>::copy(pre + lane + 32 * m, src + lane + 32 * m);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const long long mean = st->mean_fixed;
@@ -766,11 +796,8 @@ __global__ void __launch_bounds__(kZThreads)
         float2 v[R];
         asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-        for (int m = 0; m < R; m++) {
-            const longlong2 a = pre[lane + 32 * m];
-            v[m] = make_float2(i64_to_f32_rn(a.x - mean) * inv_scale,
-                               i64_to_f32_rn(a.y - mean) * inv_scale);
-        }
+        for (int m = 0; m < R; m++)
+            v[m] = ZPair<T>::value(pre[lane + 32 * m], mean, inv_scale);
         // the values are in registers: this lane's chunks of the buffer are free
         if (row + nw < nrows)
             prefetch(row + nw);
@@ -1082,13 +1109,6 @@ __global__ void __launch_bounds__(256)
 // buffer for the stages to alternate between, halving the barriers, made the
 // pass slower: 100 KB of shared memory per CTA leaves the 8-byte copies, which
 // go through L1, too little of it.)
-__device__ __forceinline__ void cp_async8(void *dst, const void *src, unsigned src_bytes)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src),
-                 "r"(src_bytes)
-                 : "memory");
-}
-
 template <int N>
 __global__ void __launch_bounds__(kXThreads, kXCtasPerSm)
     k_yfft(float2 *spec, int hc, int tiles_per_plane, int64_t ntiles,
@@ -1318,29 +1338,31 @@ cudaError_t xfft_grad_pass(const GridGeom &g, float *grid, const float2 *tw, con
                        launches);
 }
 
-cudaError_t zfft_pass(const GridGeom &g, float *grid, const unsigned long long *acc,
-                      const float2 *tw, const DeviceStatus *dstat, int num_sms,
-                      cudaStream_t stream, int64_t *launches)
+namespace {
+
+template <typename T>
+cudaError_t launch_zfft(const GridGeom &g, const T *in, float *grid, const float2 *tw,
+                        const DeviceStatus *dstat, int num_sms, cudaStream_t stream,
+                        int64_t *launches)
 {
     const int n = g.dims;
     const int64_t nrows = (int64_t)n * n;
     const int ctas = (int)std::min<int64_t>((nrows + 7) / 8, (int64_t)num_sms * 8);
-    // prefetch buffers of the accumulator rows: one row per warp
-    const int pre = (int)(sizeof(longlong2) * (kZThreads / 32) * (n / 2));
-    void (*kern)(const unsigned long long *, float *, int64_t, int, const float2 *,
-                 const DeviceStatus *) = nullptr;
+    // prefetch buffers of the input rows: one row per warp
+    const int pre = (int)(sizeof(typename ZPair<T>::V) * (kZThreads / 32) * (n / 2));
+    void (*kern)(const T *, float *, int64_t, int, const float2 *, const DeviceStatus *) = nullptr;
     switch (n) {
     case 64:
-        kern = k_zfft<64>;
+        kern = k_zfft<64, T>;
         break;
     case 128:
-        kern = k_zfft<128>;
+        kern = k_zfft<128, T>;
         break;
     case 256:
-        kern = k_zfft<256>;
+        kern = k_zfft<256, T>;
         break;
     case 512:
-        kern = k_zfft<512>;
+        kern = k_zfft<512, T>;
         break;
     default:
         return cudaErrorNotSupported;
@@ -1348,9 +1370,21 @@ cudaError_t zfft_pass(const GridGeom &g, float *grid, const unsigned long long *
     cudaError_t err;
     if ((err = ensure_dynamic_smem(kern, (size_t)pre)) != cudaSuccess)
         return err;
-    kern<<<ctas, kZThreads, pre, stream>>>(acc, grid, nrows, g.row, tw, dstat);
+    kern<<<ctas, kZThreads, pre, stream>>>(in, grid, nrows, g.row, tw, dstat);
     (*launches)++;
     return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t zfft_pass(const GridGeom &g, float *grid, const unsigned long long *acc,
+                      const float2 *tw, const DeviceStatus *dstat, int num_sms,
+                      cudaStream_t stream, int64_t *launches)
+{
+    if (!acc)
+        return launch_zfft(g, static_cast<const float *>(grid), grid, tw, dstat, num_sms, stream,
+                           launches);
+    return launch_zfft(g, acc, grid, tw, dstat, num_sms, stream, launches);
 }
 
 bool zfft_kz_supported(int dims)

@@ -197,10 +197,9 @@ int genpk_deposit_config(const genpk_ctx *ctx, int *tile_x, int *tile_y, int *ti
 /* The deposit autotuner, for passes whose particle order has no spatial
  * coherence: on the first clean pass of each particle density band (half
  * octaves of particles per cell) and mass kind, the pass runs twice per
- * candidate -- the sorted engine with tiles 8^3, 16x16x8 and 16^3, each with
- * 1 and 2 sort CTAs per SM, and, when the engine is automatic,
- * the stream engine -- timed with CUDA events, and the fastest is kept for
- * that band.  Every candidate writes the same grid.  This returns the latest
+ * candidate -- the sorted engine with tiles 8^3, 16x16x8 and 16^3, and, when
+ * the engine is automatic, the stream engine -- timed with CUDA events, and the
+ * fastest is kept for that band.  Every candidate writes the same grid.  This returns the latest
  * tuning's trials (at most cap, the number written): tile edges (0 x 0 x 0
  * for the stream engine), sort CTA count (0 for the stream engine) and
  * milliseconds each.  No reference counterpart (the reference's deposit has
@@ -312,7 +311,7 @@ int64_t genpk_batch_graph_replays(const genpk_batch *b);
  * grouped sorted-engine pass -- one launch of each kernel of the pass for all
  * of them: the sort CTAs shared out over the boxes' particles by a table of
  * (box, particle range, record range), the per-tile kernels indexed by box --
- * with a tile shape and sort CTAs per SM tuned per group on its first call
+ * with a tile shape tuned per group on its first call
  * (trials as for genpk_deposit_trials, on the group's context); then one
  * batched 2-D R2C over every x-plane of the group, and one x pass that bins
  * every box's auto spectrum (a histogram per box).  A call qualifies when
