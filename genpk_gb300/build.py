@@ -28,7 +28,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 CU_SOURCES = ["deposit.cu", "deposit_window.cu", "spectrum.cu", "xfft.cu", "adjoint.cu",
               "noalloc.cu"]
-CXX_SOURCES = {"genpk.cpp": ["-O2"], "tables.cpp": ["-O2", "-ffast-math"]}
+CXX_SOURCES = {"genpk.cpp": ["-O2", "-ftree-vectorize", "-fopenmp"], "tables.cpp": ["-O2", "-ffast-math"]}
 COMPAT_SOURCE = "compat.cpp"
 # The gen-pk command line (format-II reader + driver) over the C ABI.
 CLI_SOURCES = ["gadget2.cpp", "bigfile.cpp", "gen_pk_gb300.cpp"]
@@ -94,7 +94,7 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False) 
         for text in ex.map(_run, jobs):
             out.append(text)
     if jobs or not os.path.exists(LIB):
-        out.append(_run([NVCC, *ARCH, "-shared", "-o", LIB, *objs, "-lcufft",
+        out.append(_run([NVCC, *ARCH, "-shared", "-o", LIB, *objs, "-lcufft", "-lgomp",
                          f"-L{CUDA_HOME}/lib64", "-Xlinker", f"-rpath,{CUDA_HOME}/lib64"]))
     if jobs or not os.path.exists(COMPAT_LIB):
         out.append(_run(["g++", "-shared", "-o", COMPAT_LIB, cobj, f"-L{LIBDIR}", "-lgenpk_gb300",

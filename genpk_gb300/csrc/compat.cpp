@@ -5,7 +5,6 @@
 #include <map>
 #include <mutex>
 #include <utility>
-#include <vector>
 
 #include "../../include/genpk_compat.h"
 
@@ -71,19 +70,10 @@ int fieldize(double boxsize, int dims, double *out, int64_t segment_particles, f
     int rc = genpk_zero(ctx, 0);
     if (rc == GENPK_OK)
         rc = genpk_deposit(ctx, 0, boxsize, positions, masses, mass, segment_particles);
-    const size_t row = 2 * (size_t)(dims / 2 + 1);
-    std::vector<double> g((size_t)dims * dims * row);
-    if (rc == GENPK_OK)
-        rc = genpk_read_field(ctx, 0, g.data());
-    if (rc != GENPK_OK)
-        return rc;
     // fieldize.cpp:48-51: rows of fdims = 2*(dims/2 + extra) doubles.
-    const size_t fdims = 2 * (size_t)(dims / 2 + extra);
-    for (int x = 0; x < dims; x++)
-        for (int y = 0; y < dims; y++)
-            for (int z = 0; z < dims; z++)
-                out[((size_t)x * dims + y) * fdims + z] += g[((size_t)x * dims + y) * row + z];
-    return GENPK_OK;
+    if (rc == GENPK_OK)
+        rc = genpk_add_field(ctx, 0, out, 2 * (int64_t)(dims / 2 + extra));
+    return rc;
 }
 
 extern "C" {

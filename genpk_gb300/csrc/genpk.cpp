@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <cufft.h>
 #include <math.h>
+#include <omp.h>
 #include <stddef.h>
 #include <string.h>
 
@@ -210,6 +211,13 @@ struct genpk_ctx {
         std::vector<double> mass;
         int np = 0;
     } step;
+
+    // host grids in and out: a ring of pinned buffers that device grids come
+    // back through, and a device buffer that host spectra go through
+    float *ring = nullptr;
+    cudaEvent_t ring_ev[2] = {};
+    double *d_wide = nullptr;
+    size_t wide_cap = 0;  // doubles
 
     // adjoint scratch
     float *d_gcoef = nullptr;
@@ -1510,6 +1518,66 @@ struct IssueState {
     }
 };
 
+// Ring slots of kRingFloats; a header (the grid's subtracted mean, the status
+// words) behind them.
+constexpr size_t kRingFloats = (size_t)1 << 20;
+struct RingHead {
+    double mean;
+    DeviceStatus status;
+};
+
+RingHead *ring_head(genpk_ctx *ctx)
+{
+    return reinterpret_cast<RingHead *>(ctx->ring + 2 * kRingFloats);
+}
+
+int ensure_ring(genpk_ctx *ctx)
+{
+    if (!ctx->ring)
+        GENPK_CUDA(cudaHostAlloc((void **)&ctx->ring,
+                                 sizeof(float) * 2 * kRingFloats + sizeof(RingHead),
+                                 cudaHostAllocDefault));
+    for (auto &e : ctx->ring_ev)
+        if (!e)
+            GENPK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return GENPK_OK;
+}
+
+// A density grid's rows to the host through the ring: each slot of whole rows
+// is handed to f(first row, rows, floats) while the next one is on its way.
+template <class F>
+int read_rows(genpk_ctx *ctx, int field, F &&f)
+{
+    const size_t row = (size_t)ctx->gg.row, rows = (size_t)ctx->dims * (size_t)ctx->dims;
+    const size_t per = std::max<size_t>(1, kRingFloats / row);
+    const float *grid = grid_of(ctx, field);
+    auto fetch = [&](size_t k) -> int {
+        const size_t r0 = k * per;
+        if (r0 >= rows)
+            return GENPK_OK;
+        GENPK_CUDA(cudaMemcpyAsync(ctx->ring + (k & 1) * kRingFloats, grid + r0 * row,
+                                   sizeof(float) * row * std::min(per, rows - r0),
+                                   cudaMemcpyDeviceToHost, ctx->stream));
+        GENPK_CUDA(cudaEventRecord(ctx->ring_ev[k & 1], ctx->stream));
+        return GENPK_OK;
+    };
+    GENPK_TRY(fetch(0));
+    GENPK_TRY(fetch(1));
+    for (size_t k = 0; k * per < rows; k++) {
+        GENPK_CUDA(cudaEventSynchronize(ctx->ring_ev[k & 1]));
+        f(k * per, std::min(per, rows - k * per), ctx->ring + (k & 1) * kRingFloats);
+        GENPK_TRY(fetch(k + 2));
+    }
+    return GENPK_OK;
+}
+
+// Threads for a host loop over n grid values (one below a quarter million: a
+// thread's start costs more than it takes over).
+int host_threads(size_t n)
+{
+    return n < ((size_t)1 << 18) ? 1 : std::min(8, omp_get_max_threads());
+}
+
 // Device copies of particle arrays for the adjoint when the caller passed host memory.
 int adj_stage(genpk_ctx *ctx, size_t floats)
 {
@@ -1584,6 +1652,11 @@ void genpk_ctx_destroy(genpk_ctx *ctx)
     cudaFree(ctx->adj_buf);
     cudaFree(ctx->d_probe);
     cudaFreeHost(ctx->res_host);
+    cudaFreeHost(ctx->ring);
+    cudaFree(ctx->d_wide);
+    for (auto &e : ctx->ring_ev)
+        if (e)
+            cudaEventDestroy(e);
     for (auto &e : ctx->ev)
         if (e)
             cudaEventDestroy(e);
@@ -1973,12 +2046,19 @@ int genpk_load_spectrum(genpk_ctx *ctx, int field, const double *spectrum)
     cudaSetDevice(ctx->device);
     if (ctx->pend.active && ctx->pend.field == field)
         GENPK_TRY(flush_pending(ctx));
+    // The doubles go to the device as they are (through a buffer of at most 64
+    // MB) and are rounded to floats there: a host loop over them took 0.8 of the
+    // 1.1 ms of a 128^3 spectrum.
     const size_t nc = (size_t)ctx->gg.nfloat;  // 2 floats per complex value
-    std::vector<float> tmp(nc);
-    for (size_t i = 0; i < nc; i++)
-        tmp[i] = (float)spectrum[i];
-    GENPK_CUDA(cudaMemcpyAsync(grid_of(ctx, field), tmp.data(), sizeof(float) * nc,
-                               cudaMemcpyHostToDevice, ctx->stream));
+    const size_t per = std::min<size_t>(nc, (size_t)1 << 23);
+    GENPK_TRY(grow(ctx, &ctx->d_wide, &ctx->wide_cap, per));
+    for (size_t i = 0; i < nc; i += per) {
+        const size_t n = std::min(per, nc - i);
+        GENPK_CUDA(cudaMemcpyAsync(ctx->d_wide, spectrum + i, sizeof(double) * n,
+                                   cudaMemcpyHostToDevice, ctx->stream));
+        GENPK_CUDA(doubles_to_floats(ctx->d_wide, grid_of(ctx, field) + i, n, ctx->num_sms,
+                                     ctx->stream, &ctx->launches));
+    }
     GENPK_CUDA(cudaStreamSynchronize(ctx->stream));
     ctx->state[(size_t)field] = F_SPECTRUM;
     ctx->auto_valid[(size_t)field] = false;
@@ -2020,19 +2100,55 @@ int genpk_read_field(genpk_ctx *ctx, int field, double *out)
     }
     if (st != F_DENSITY)
         return fail(ctx, GENPK_ERR_STATE, "genpk_read_field: field is not a density");
-    std::vector<float> tmp(nf);
-    double mean = 0.0;  // the exact sum of the (fixed-point) means subtracted by the passes
-    GENPK_CUDA(cudaMemcpyAsync(tmp.data(), grid_of(ctx, field), sizeof(float) * nf,
-                               cudaMemcpyDeviceToHost, ctx->stream));
-    GENPK_CUDA(cudaMemcpyAsync(&mean, ctx->d_field_mass + ctx->nfields + field, sizeof(double),
+    GENPK_TRY(ensure_ring(ctx));
+    // the exact sum of the (fixed-point) means subtracted by the passes
+    GENPK_CUDA(cudaMemcpyAsync(&ring_head(ctx)->mean, ctx->d_field_mass + ctx->nfields + field,
+                               sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    const size_t row = (size_t)ctx->gg.row, dims = (size_t)ctx->dims;
+    const int rc = read_rows(ctx, field, [&](size_t r0, size_t rows, const float *g) {
+        const double mean = ring_head(ctx)->mean;
+#pragma omp parallel for num_threads(host_threads(rows * row))
+        for (size_t r = 0; r < rows; r++) {
+            double *o = out + (r0 + r) * row;
+            for (size_t z = 0; z < dims; z++)
+                o[z] = (double)g[r * row + z] + mean;
+            for (size_t z = dims; z < row; z++)
+                o[z] = 0.0;
+        }
+    });
+    return rc != GENPK_OK ? rc : collect_status(ctx);
+}
+
+int genpk_add_field(genpk_ctx *ctx, int field, double *out, int64_t row_out)
+{
+    GENPK_TRY(check_field(ctx, field));
+    if (!out || row_out < ctx->dims)
+        return fail(ctx, GENPK_ERR_INVALID, "genpk_add_field: null output or short rows");
+    cudaSetDevice(ctx->device);
+    GENPK_TRY(flush_pending(ctx));
+    const int st = ctx->state[(size_t)field];
+    if (st == F_CLEAN)
+        return collect_status(ctx);
+    if (st != F_DENSITY)
+        return fail(ctx, GENPK_ERR_STATE, "genpk_add_field: field is not a density");
+    GENPK_TRY(ensure_ring(ctx));
+    RingHead *head = ring_head(ctx);
+    GENPK_CUDA(cudaMemcpyAsync(&head->mean, ctx->d_field_mass + ctx->nfields + field,
+                               sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    GENPK_CUDA(cudaMemcpyAsync(&head->status, ctx->d_status, sizeof(DeviceStatus),
                                cudaMemcpyDeviceToHost, ctx->stream));
     GENPK_CUDA(cudaStreamSynchronize(ctx->stream));
-    const int row = ctx->gg.row, dims = (int)ctx->dims;
-    for (size_t i = 0; i < nf; i++) {
-        const int z = (int)(i % (size_t)row);
-        out[i] = z < dims ? (double)tmp[i] + mean : 0.0;
-    }
-    return collect_status(ctx);
+    GENPK_TRY(report_status(ctx, head->status));
+    const size_t row = (size_t)ctx->gg.row, dims = (size_t)ctx->dims;
+    const double mean = head->mean;
+    return read_rows(ctx, field, [&](size_t r0, size_t rows, const float *g) {
+#pragma omp parallel for num_threads(host_threads(rows * row))
+        for (size_t r = 0; r < rows; r++) {
+            double *o = out + (r0 + r) * (size_t)row_out;
+            for (size_t z = 0; z < dims; z++)
+                o[z] += (double)g[r * row + z] + mean;
+        }
+    });
 }
 
 int genpk_adjoint(genpk_ctx *ctx, int field, double boxsize, const float *pos, const float *masses,

@@ -377,6 +377,9 @@ cudaError_t bin_spectrum_kz(const GridGeom &g, const BinTables &t, const BinDevi
                             const float2 *spec, const double *corner, double *partial, int ctas,
                             int warps, size_t smem, void *zero, int64_t zero_bytes,
                             cudaStream_t stream, int64_t *launches);
+// n doubles rounded to floats (both on the device).
+cudaError_t doubles_to_floats(const double *in, float *out, size_t n, int num_sms,
+                              cudaStream_t stream, int64_t *launches);
 cudaError_t bin_spectra(const GridGeom &g, const BinTables &t, const BinDevice &d,
                         const BinLaunch &l, double *partial, double *out_power, int ctas,
                         int warps, size_t smem, cudaStream_t stream, int64_t *launches,

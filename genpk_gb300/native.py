@@ -39,6 +39,7 @@ ABI = {
     "genpk_bin_of": (ctypes.c_int, [c_void_p, ctypes.c_int64]),
     "genpk_sync": (ctypes.c_int, [c_void_p]),
     "genpk_read_field": (ctypes.c_int, [c_void_p, ctypes.c_int, c_f64p]),
+    "genpk_add_field": (ctypes.c_int, [c_void_p, ctypes.c_int, c_f64p, ctypes.c_int64]),
     "genpk_adjoint": (ctypes.c_int, [c_void_p, ctypes.c_int, ctypes.c_double, c_void_p, c_void_p,
                                      ctypes.c_double, ctypes.c_int64, ctypes.c_double, c_f64p,
                                      c_void_p, c_void_p, c_f64p, ctypes.c_int]),

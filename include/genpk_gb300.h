@@ -164,6 +164,12 @@ int genpk_sync(genpk_ctx *ctx);
  * Intended for tests; flushes pending deposits. */
 int genpk_read_field(genpk_ctx *ctx, int field, double *out);
 
+/* Add grid `field` (density form) to a host grid of dims*dims rows of `row`
+ * doubles, row >= dims: the first dims values of each row, as fieldize() adds
+ * to its caller's grid (fieldize.cpp:104-113).  Flushes pending deposits.  An
+ * error (a skipped particle among them) leaves `out` as it was. */
+int genpk_add_field(genpk_ctx *ctx, int field, double *out, int64_t row);
+
 /* Gradient of a P(k) loss with respect to particle positions and masses
  * (no reference counterpart).  For the auto spectrum of grid `field` built from
  * the n particles (pos, masses|NULL, mass) with normalisation mass_norm:
