@@ -14,6 +14,7 @@
 // k_mode_gradient here serves the other sizes.
 #include "common.cuh"
 #include "internal.h"
+#include "launch.cuh"
 
 #include <algorithm>
 
@@ -43,6 +44,9 @@ __global__ void __launch_bounds__(256)
     extern __shared__ uint32_t thr[];
     for (int i = threadIdx.x; i <= p.nrbins; i += blockDim.x)
         thr[i] = thr_g[i];
+    wait_previous();
+    spec = fresh(spec);
+    gcoef = fresh(gcoef);
     __syncthreads();
     const bool even = (p.dims & 1) == 0;
     const int lane = threadIdx.x & 31;
@@ -105,6 +109,9 @@ __global__ void __launch_bounds__(256)
     extern __shared__ uint32_t thr[];
     for (int i = threadIdx.x; i <= p.nrbins; i += blockDim.x)
         thr[i] = thr_g[i];
+    wait_previous();
+    spec = fresh(spec);
+    gcoef = fresh(gcoef);
     __syncthreads();
     const bool even = (p.dims & 1) == 0;
     const int lane = threadIdx.x & 31;
@@ -204,6 +211,8 @@ __global__ void __launch_bounds__(256)
     k_gather(GatherParams p, const float *__restrict__ grid, const float *__restrict__ pos,
              const float *__restrict__ masses, float *__restrict__ gpos, float *__restrict__ gmass)
 {
+    wait_previous();
+    grid = fresh(grid);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const float x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
@@ -242,6 +251,8 @@ __global__ void __launch_bounds__(256)
     k_gather4(GatherParams p, const float *__restrict__ grid, const float *__restrict__ pos,
               const float *__restrict__ masses, float *__restrict__ gpos, float *__restrict__ gmass)
 {
+    wait_previous();
+    grid = fresh(grid);
     const int64_t groups = p.n >> 2;
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (int64_t q = tid; q < groups; q += (int64_t)gridDim.x * blockDim.x) {
@@ -295,9 +306,9 @@ cudaError_t adjoint_mode_gradient_kz(const GridGeom &g, const BinTables &t, cons
     cudaError_t err;
     if ((err = ensure_dynamic_smem(k_mode_gradient_kz, smem)) != cudaSuccess)
         return err;
-    k_mode_gradient_kz<<<num_sms * 8, 256, smem, stream>>>(p, spec, d.thr, d.iw, gcoef_dev);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(k_mode_gradient_kz, num_sms * 8, 256, smem, stream, p, spec, d.thr, d.iw,
+                        gcoef_dev);
 }
 
 cudaError_t adjoint_mode_gradient_coef(const GridGeom &g, const BinTables &t, const BinDevice &d,
@@ -312,10 +323,9 @@ cudaError_t adjoint_mode_gradient_coef(const GridGeom &g, const BinTables &t, co
     p.bpu_half = (float)(0.5 * t.binsperunit);
     // one warp per row of kz modes; 4 CTAs of 8 warps per SM (46 registers)
     const int blocks = (int)std::min<int64_t>(((int64_t)g.dims * g.dims + 7) / 8, 152 * 4);
-    k_mode_gradient<<<blocks, 256, sizeof(uint32_t) * (t.nrbins + 1), stream>>>(p, spec, d.thr,
-                                                                              d.iw, gcoef_dev);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(k_mode_gradient, blocks, 256, sizeof(uint32_t) * (t.nrbins + 1), stream, p,
+                        spec, d.thr, d.iw, gcoef_dev);
 }
 
 cudaError_t adjoint_gather(const GridGeom &g, float units_hi, float units_lo, const float *grid,
@@ -343,20 +353,14 @@ cudaError_t adjoint_gather(const GridGeom &g, float units_hi, float units_lo, co
                      (!masses || (aligned16(masses) && aligned16(grad_mass)));
     if (vec) {
         const int blocks4 = (int)std::min<int64_t>(std::max<int64_t>((n / 4 + 255) / 256, 1), 152 * 32);
-        if (masses)
-            k_gather4<true><<<blocks4, 256, 0, stream>>>(p, grid, pos, masses, grad_pos, grad_mass);
-        else
-            k_gather4<false><<<blocks4, 256, 0, stream>>>(p, grid, pos, masses, grad_pos, grad_mass);
         (*launches)++;
-        return cudaGetLastError();
+        return launch_after(masses ? k_gather4<true> : k_gather4<false>, blocks4, 256, 0, stream, p,
+                            grid, pos, masses, grad_pos, grad_mass);
     }
     const int blocks = (int)std::min<int64_t>((n + 255) / 256, 152 * 32);
-    if (masses)
-        k_gather<true><<<blocks, 256, 0, stream>>>(p, grid, pos, masses, grad_pos, grad_mass);
-    else
-        k_gather<false><<<blocks, 256, 0, stream>>>(p, grid, pos, masses, grad_pos, grad_mass);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(masses ? k_gather<true> : k_gather<false>, blocks, 256, 0, stream, p, grid,
+                        pos, masses, grad_pos, grad_mass);
 }
 
 }  // namespace genpk

@@ -37,6 +37,15 @@ __host__ __device__ inline PassConsts pass_consts(double m, float mref, double i
     return {m, s, mean_fixed};
 }
 
+// The pass joins a grid's running mass and the sum of the means subtracted from
+// it; a clean grid's first pass starts them (no memset comes before it).
+__device__ __forceinline__ void add_pass_sums(const PassConsts &k, bool clean, double *field_mass,
+                                              double *field_sub)
+{
+    *field_mass = (clean ? 0.0 : *field_mass) + k.mass;
+    *field_sub = (clean ? 0.0 : *field_sub) + ldexp((double)k.mean_fixed, -k.fx_shift);
+}
+
 // Position -> (wrapped cell, fraction) for one axis, as fieldize.cpp:66-76
 // computes it in FP64: x = pos*units, f = floor(x), d = x - f, f wrapped mod N.
 //

@@ -46,6 +46,7 @@
 #include "bulk.cuh"
 #include "common.cuh"
 #include "internal.h"
+#include "launch.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -148,6 +149,7 @@ struct ScanOut {
     uint32_t *ticket;      // one per box; zero between passes
     double *mass_part;     // [sort CTAs]
     double inv_cells;
+    bool clean;
     double *field_mass, *field_sub;
 };
 
@@ -276,14 +278,14 @@ __device__ __forceinline__ void load_half(const SortParams &p, int64_t i0, Pos3 
 
 // A pass's constants into the status words and the grid's running sums, by one
 // thread.
-__device__ __forceinline__ void store_pass_consts(const PassConsts &k, double *field_mass,
-                                                  double *field_sub, DeviceStatus *st)
+__device__ __forceinline__ void store_pass_consts(const PassConsts &k, bool clean,
+                                                  double *field_mass, double *field_sub,
+                                                  DeviceStatus *st)
 {
     st->pass_mass = k.mass;
     st->fx_shift = k.fx_shift;
     st->mean_fixed = k.mean_fixed;
-    *field_mass += k.mass;
-    *field_sub += ldexp((double)k.mean_fixed, -k.fx_shift);
+    add_pass_sums(k, clean, field_mass, field_sub);
 }
 
 // Exclusive scan of box `box`'s tile totals and its per-pass constants, by the
@@ -364,7 +366,7 @@ __device__ __forceinline__ void scan_box(const ScanOut &o, const ScanBoxes &boxe
         const float mref = !boxes.var[box] ? (float)fabs(boxes.umass[box])
                                            : __uint_as_float(__ldcg(&st->max_mass_bits));
         st->max_mass_bits = 0u;  // read: zero again for the next pass
-        store_pass_consts(pass_consts(m, mref, o.inv_cells), o.field_mass + box,
+        store_pass_consts(pass_consts(m, mref, o.inv_cells), o.clean, o.field_mass + box,
                           o.field_sub + box, st);
         o.ticket[box] = 0u;
     }
@@ -393,6 +395,7 @@ __global__ void __launch_bounds__(kSortThreads)
         __syncthreads();
     }
     uint32_t *counts = GLOBAL ? totals : sh_hist;
+    wait_previous();
     float msum = 0.f, mc = 0.f, mmax = 0.f;
     unsigned bad = 0;
     for (int64_t c0 = (int64_t)cta * kSortChunkParticles; c0 < p.n;
@@ -499,6 +502,7 @@ struct BinOut {
     double *corner_part;  // per sort CTA: its share of the corner mode (over a uniform mass)
     uint32_t *ticket;     // one per box; zero between passes
     double inv_cells;
+    bool clean;
     double *field_mass, *field_sub;
 };
 
@@ -577,6 +581,7 @@ __global__ void __launch_bounds__(kBinThreads, 1)
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nt4 = (p.ntiles + 3) >> 2;
     const bool var = p.masses != nullptr;
+    wait_previous();
 
     f2sum alt = {0.f, 0.f};
     double corner = 0.0;
@@ -767,7 +772,7 @@ __global__ void __launch_bounds__(kBinThreads, 1)
     if (threadIdx.x == 0) {
         const float mref = __uint_as_float(__ldcg(&st->max_mass_bits));
         st->max_mass_bits = 0u;  // read: zero again for the next pass
-        store_pass_consts(pass_consts(m, mref, out.inv_cells), out.field_mass + box,
+        store_pass_consts(pass_consts(m, mref, out.inv_cells), out.clean, out.field_mass + box,
                           out.field_sub + box, st);
         out.ticket[box] = 0u;
     }
@@ -811,6 +816,9 @@ __global__ void __launch_bounds__(kSortThreads, 2)
     }
     const uint32_t mx = (1u << p.lx) - 1u, my = (1u << p.ly) - 1u, mz = (1u << p.lz) - 1u;
     const int lane = threadIdx.x & 31;
+    wait_previous();
+    cursor = fresh(cursor);
+    st = fresh(st);
     // Corner terms in 2^-(s+4) mass units (|term| < 2^32), summed per thread as
     // a float pair and converted to an integer once per warp.
     const float mscale = ldexpf(1.f, st->fx_shift + 4);
@@ -1043,7 +1051,7 @@ struct RangeWalk {
     uint32_t s0, s1;
     __device__ __forceinline__ void begin(const RangeRecords &r, int box, int ntiles, int t)
     {
-        const uint32_t *start = r.tile_start + (size_t)box * (ntiles + 1);
+        const uint32_t *start = fresh(r.tile_start) + (size_t)box * (ntiles + 1);
         s0 = start[t];
         s1 = start[t + 1];
     }
@@ -1079,7 +1087,7 @@ struct ChunkWalk {
         len = r.len[box];
         nchunks = r.nchunks[box];
         rec0 = r.rec0[box];
-        hdr = r.hdr + (size_t)r.hdr0[box] * (size_t)stride + t;
+        hdr = fresh(r.hdr) + (size_t)r.hdr0[box] * (size_t)stride + t;
         group = r.group[box];
         c = wid * group + lane;
         load();
@@ -1137,8 +1145,6 @@ __global__ void __launch_bounds__(kTileThreads, 4)
     unsigned *lo = acc_words, *hi = acc_words + L::NACC;
     const TileOfBlock tb = tile_of_block(p, 0);
     const int ntiles = p.ntx * p.nty * p.ntz;
-    typename WalkOf<Records>::T records_walk;
-    records_walk.begin(records, tb.box, ntiles, tb.t);
     st += tb.box;
     grid += (size_t)tb.box * (size_t)grid_stride;
     const size_t slot = (size_t)tb.box * ntiles + tb.t;
@@ -1146,6 +1152,11 @@ __global__ void __launch_bounds__(kTileThreads, 4)
     const int ex = min(TX, p.dims - x0), ey = min(TY, p.dims - y0), ez = min(TZ, p.dims - z0);
     for (int i = threadIdx.x; i < (2 * L::NACC + 3) / 4; i += blockDim.x)
         reinterpret_cast<uint4 *>(acc_words)[i] = make_uint4(0u, 0u, 0u, 0u);
+    wait_previous();
+    sorted = fresh(sorted);
+    st = fresh(st);
+    typename WalkOf<Records>::T records_walk;
+    records_walk.begin(records, tb.box, ntiles, tb.t);
     __syncthreads();
 
     const int s = consts.host[tb.box] ? consts.fx_shift[tb.box] : st->fx_shift;
@@ -1197,7 +1208,8 @@ __global__ void __launch_bounds__(kTileThreads, 4)
         const PassConsts pc = box_consts(consts, tb.box, st);
         const long long mean = pc.mean_fixed;
         if (consts.host[tb.box] && tb.t == 0 && threadIdx.x == 0)
-            store_pass_consts(pc, consts.field_mass + tb.box, consts.field_sub + tb.box, st);
+            store_pass_consts(pc, CLEAN, consts.field_mass + tb.box, consts.field_sub + tb.box,
+                              st);
         const int z = threadIdx.x % TZ, y = (threadIdx.x / TZ) % TY;
         int x = threadIdx.x / (TY * TZ);
         x += x == 0 ? NXP : 0;
@@ -1263,6 +1275,7 @@ struct PassEnd {
     int first[kMaxGroupBoxes + 1];   // each box's partials
     double unit_mass[kMaxGroupBoxes];  // what they are in units of
     double *field_corner;
+    bool clean;  // the grid's first pass: its sums start here
     unsigned long long *bad_out;
 };
 
@@ -1272,7 +1285,7 @@ __device__ __forceinline__ void end_pass(const PassEnd &e, int box, DeviceStatus
     double corner = 0.0;
     if (e.corner_part) {
         for (int i = e.first[box] + threadIdx.x; i < e.first[box + 1]; i += blockDim.x)
-            corner += e.corner_part[i];
+            corner += fresh(e.corner_part)[i];
         corner = block_sum_d(corner, sh) * e.unit_mass[box];
     }
     if (threadIdx.x != 0)
@@ -1282,7 +1295,7 @@ __device__ __forceinline__ void end_pass(const PassEnd &e, int box, DeviceStatus
         corner = ldexp((double)st->alt_sum, -(st->fx_shift + 4));
         st->alt_sum = 0;
     }
-    e.field_corner[box] += corner;
+    e.field_corner[box] = (e.clean ? 0.0 : e.field_corner[box]) + corner;
     if (e.bad_out) {
         e.bad_out[box] = st->bad_particles;
         st->bad_particles = 0;
@@ -1296,6 +1309,10 @@ __global__ void __launch_bounds__(256)
                   DeviceStatus *st, float *__restrict__ grid, int64_t grid_stride)
 {
     using L = TileLayout<TX, TY, TZ>;
+    wait_previous();
+    faces = fresh(faces);
+    halo = fresh(halo);
+    st = fresh(st);
     if (blockIdx.z == 0) {
         const int nbox = ((int)gridDim.z - 1) / p.ntx;
         for (int b = blockIdx.y * gridDim.x + blockIdx.x; b < nbox; b += gridDim.x * gridDim.y)
@@ -1421,12 +1438,12 @@ cudaError_t launch_tile_kernels(const DepositGeom &g, const TileTarget &a, const
     cudaError_t err;
 #define GENPK_TILE_LAUNCH(V, C)                                                                \
     do {                                                                                       \
-        auto kern = k_tile_deposit<TX, TY, TZ, V, C, Records>;                                          \
+        auto kern = k_tile_deposit<TX, TY, TZ, V, C, Records>;                                 \
         err = ensure_dynamic_smem(kern, smem);                                                 \
         if (err != cudaSuccess)                                                                \
             return err;                                                                        \
-        kern<<<tiles, kTileThreads, smem, stream>>>(tp, s.sorted, records, a.consts, dstat,    \
-                                                   a.grid, s.faces, s.halo, a.grid_stride);    \
+        err = launch_after(kern, tiles, kTileThreads, smem, stream, tp, s.sorted, records,     \
+                           a.consts, dstat, a.grid, s.faces, s.halo, a.grid_stride);           \
     } while (0)
     if (var && a.clean)
         GENPK_TILE_LAUNCH(true, true);
@@ -1440,18 +1457,15 @@ cudaError_t launch_tile_kernels(const DepositGeom &g, const TileTarget &a, const
     (*launches)++;
     if (hook)
         hook(hook_user, "dep_tile");
-    if ((err = cudaGetLastError()) != cudaSuccess)
+    if (err != cudaSuccess)
         return err;
-    if (a.clean)
-        k_face_gather<TX, TY, TZ, true><<<slices, 256, 0, stream>>>(
-            tp, s.faces, s.halo, a.end, dstat, a.grid, a.grid_stride);
-    else
-        k_face_gather<TX, TY, TZ, false><<<slices, 256, 0, stream>>>(
-            tp, s.faces, s.halo, a.end, dstat, a.grid, a.grid_stride);
+    auto face = a.clean ? k_face_gather<TX, TY, TZ, true> : k_face_gather<TX, TY, TZ, false>;
+    err = launch_after(face, slices, 256, 0, stream, tp, s.faces, s.halo, a.end, dstat, a.grid,
+                       a.grid_stride);
     (*launches)++;
     if (hook)
         hook(hook_user, "dep_faces");
-    return cudaGetLastError();
+    return err;
 }
 
 template <class Records>
@@ -1491,8 +1505,8 @@ SortParams sort_params(const DepositGeom &g, const float *pos, const float *mass
 // The histogram (and scan) and scatter launches of a pass over `ctas` sort CTAs.
 template <class Src>
 cudaError_t launch_sort(const DepositGeom &g, const Src &src, const ScanBoxes &sb, DepositScratch &s,
-                        double *field_mass, double *field_sub, DeviceStatus *dstat, int ctas,
-                        cudaStream_t stream, int64_t *launches, StageHook hook, void *hook_user)
+                        const TileTarget &t, DeviceStatus *dstat, int ctas, cudaStream_t stream,
+                        int64_t *launches, StageHook hook, void *hook_user)
 {
     auto mark = [&](const char *name) {
         (*launches)++;
@@ -1506,9 +1520,10 @@ cudaError_t launch_sort(const DepositGeom &g, const Src &src, const ScanBoxes &s
     out.cursor_stride = deposit_shared_hist(g) ? kCursorStride : 1;
     out.ticket = s.ticket;
     out.mass_part = s.mass_part;
-    out.inv_cells = 1.0 / ((double)g.grid.dims * g.grid.dims * g.grid.dims);
-    out.field_mass = field_mass;
-    out.field_sub = field_sub;
+    out.inv_cells = t.consts.inv_cells;
+    out.clean = t.clean;
+    out.field_mass = t.consts.field_mass;
+    out.field_sub = t.consts.field_sub;
     // (max_mass_bits and alt_sum are zero here: the pass that used them last
     // zeroed them, in scan_box / k_window_prep and the finishing kernels)
     const bool shared_hist = deposit_shared_hist(g);
@@ -1518,15 +1533,15 @@ cudaError_t launch_sort(const DepositGeom &g, const Src &src, const ScanBoxes &s
     cudaError_t err;
     if ((err = ensure_dynamic_smem(hist, hsmem)) != cudaSuccess)
         return err;
-    hist<<<ctas, kSortThreads, hsmem, stream>>>(src, out, sb, dstat);
-    mark("dep_hist");
-    if ((err = cudaGetLastError()) != cudaSuccess)
+    if ((err = launch_after(hist, ctas, kSortThreads, hsmem, stream, src, out, sb, dstat)) !=
+        cudaSuccess)
         return err;
+    mark("dep_hist");
     if ((err = ensure_dynamic_smem(scatter, hsmem)) != cudaSuccess)
         return err;
-    scatter<<<ctas, kSortThreads, hsmem, stream>>>(src, s.cursor, s.sorted, dstat);
+    err = launch_after(scatter, ctas, kSortThreads, hsmem, stream, src, s.cursor, s.sorted, dstat);
     mark("dep_scatter");
-    return cudaGetLastError();
+    return err;
 }
 
 // Chunk length and count of a binned pass over n particles on `ctas` CTAs:
@@ -1580,6 +1595,7 @@ cudaError_t launch_bins(const DepositGeom &g, const Src &src, const ChunkRecords
     out.corner_part = s.mass_part + ctas;
     out.ticket = s.ticket;
     out.inv_cells = t.consts.inv_cells;
+    out.clean = t.clean;
     out.field_mass = t.consts.field_mass;
     out.field_sub = t.consts.field_sub;
     const size_t smem = sizeof(uint4) * (size_t)stage_len + 4 * (size_t)((g.ntiles + 3) & ~3);
@@ -1587,11 +1603,11 @@ cudaError_t launch_bins(const DepositGeom &g, const Src &src, const ChunkRecords
     cudaError_t err;
     if ((err = ensure_dynamic_smem(kern, smem)) != cudaSuccess)
         return err;
-    kern<<<ctas, kBinThreads, smem, stream>>>(src, out, stage_len, dstat);
+    err = launch_after(kern, ctas, kBinThreads, smem, stream, src, out, stage_len, dstat);
     (*launches)++;
     if (hook)
         hook(hook_user, "dep_bins");
-    return cudaGetLastError();
+    return err;
 }
 
 }  // namespace
@@ -1668,6 +1684,7 @@ cudaError_t deposit_pass(const DepositGeom &g, const DepositArgs &a, DepositScra
     t.consts.field_mass = a.field_mass;
     t.consts.field_sub = a.field_sub;
     t.end.field_corner = a.field_corner;
+    t.end.clean = a.clean;
     if (deposit_binned(g)) {
         OneBin one = {};
         one.b.s = src.p;
@@ -1692,8 +1709,8 @@ cudaError_t deposit_pass(const DepositGeom &g, const DepositArgs &a, DepositScra
     sb.first[1] = sort_ctas;
     sb.var[0] = a.masses ? 1 : 0;
     sb.umass[0] = (double)a.mass;
-    cudaError_t err = launch_sort(g, src, sb, s, a.field_mass, a.field_sub, dstat, sort_ctas,
-                                  stream, launches, hook, hook_user);
+    cudaError_t err = launch_sort(g, src, sb, s, t, dstat, sort_ctas, stream, launches, hook,
+                                  hook_user);
     if (err != cudaSuccess)
         return err;
     return launch_tile_pass(g, t, RangeRecords{s.tile_start}, s, dstat, stream, launches, hook, hook_user);
@@ -1742,6 +1759,7 @@ cudaError_t deposit_group_pass(const DepositGeom &g, const GroupLayout &lay, con
     t.consts.field_mass = field_mass0;
     t.consts.field_sub = field_sub0;
     t.end.field_corner = field_corner0;
+    t.end.clean = true;
     t.end.bad_out = bad_out;
     if (deposit_binned(g)) {
         BinGroup src = {};
@@ -1795,8 +1813,8 @@ cudaError_t deposit_group_pass(const DepositGeom &g, const GroupLayout &lay, con
         sb.umass[b] = (double)x.mass;
         sb.rec0[b] = (long long)lay.rec0[b];
     }
-    const cudaError_t err = launch_sort(g, src, sb, s, field_mass0, field_sub0, st0,
-                                        lay.cta0[nbox], stream, launches, nullptr, nullptr);
+    const cudaError_t err = launch_sort(g, src, sb, s, t, st0, lay.cta0[nbox], stream, launches,
+                                        nullptr, nullptr);
     if (err != cudaSuccess)
         return err;
     return launch_tile_pass(g, t, RangeRecords{s.tile_start}, s, st0, stream, launches, nullptr,

@@ -45,6 +45,7 @@
 #include "bulk.cuh"
 #include "common.cuh"
 #include "internal.h"
+#include "launch.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -87,6 +88,7 @@ struct WinParams {
     double pass_mass;
     long long mean_fixed;
     double *field_mass, *field_sub;
+    int clean;  // the grid's first pass
 };
 
 // Thread 0 of CTA 0: the host-computed constants into the status words and
@@ -97,8 +99,8 @@ __device__ __forceinline__ void store_host_prep(const WinParams &p, DeviceStatus
         st->pass_mass = p.pass_mass;
         st->fx_shift = p.fx_shift;
         st->mean_fixed = p.mean_fixed;
-        *p.field_mass += p.pass_mass;
-        *p.field_sub += ldexp((double)p.mean_fixed, -p.fx_shift);
+        add_pass_sums(PassConsts{p.pass_mass, p.fx_shift, p.mean_fixed}, p.clean != 0, p.field_mass,
+                      p.field_sub);
     }
 }
 
@@ -363,6 +365,8 @@ __global__ void __launch_bounds__(kWinThreads, 1)
         fence_mbar_init();
         fence_proxy_async();
     }
+    wait_previous();
+    st = fresh(st);
     __syncthreads();
 
     // Weights in 2^-s mass units, s = 154 - emax (common.cuh pair_w / z_mass /
@@ -587,6 +591,8 @@ __global__ void __launch_bounds__(kWinThreads, 1)
         fence_mbar_init();
         fence_proxy_async();
     }
+    wait_previous();
+    st = fresh(st);
     __syncthreads();
 
     store_host_prep(p, st);
@@ -765,6 +771,7 @@ __global__ void __launch_bounds__(256)
     k_mass_reduce(const float *__restrict__ masses, int64_t n, double *__restrict__ mass_part,
                   DeviceStatus *st)
 {
+    wait_previous();
     float s = 0.f, cmp = 0.f, mx = 0.f;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -807,9 +814,11 @@ __global__ void __launch_bounds__(256)
 // rounded to 24 significant bits (an empty cell then reads back exactly 0).
 // nparts = 0: uniform mass umass; else the sum of nparts partial sums.
 __global__ void k_window_prep(const double *__restrict__ mass_part, int nparts, double umass,
-                              int64_t n, double inv_cells, double *field_mass, double *field_sub,
-                              DeviceStatus *st)
+                              int64_t n, double inv_cells, bool clean, double *field_mass,
+                              double *field_sub, DeviceStatus *st)
 {
+    wait_previous();
+    mass_part = fresh(mass_part);
     double m = 0.0;
     float mref;
     if (nparts == 0) {
@@ -825,8 +834,7 @@ __global__ void k_window_prep(const double *__restrict__ mass_part, int nparts, 
     st->pass_mass = k.mass;
     st->fx_shift = k.fx_shift;
     st->mean_fixed = k.mean_fixed;
-    *field_mass += k.mass;
-    *field_sub += ldexp((double)k.mean_fixed, -k.fx_shift);
+    add_pass_sums(k, clean, field_mass, field_sub);
 }
 
 // Accumulator minus the mean, rounded once to FP32 and stored (clean grid) or
@@ -840,6 +848,9 @@ __global__ void __launch_bounds__(256)
                      int64_t npairs, int clean, const DeviceStatus *__restrict__ st)
 {
     constexpr int U = 4;
+    wait_previous();
+    acc = fresh(acc);
+    st = fresh(st);
     const long long mean = st->mean_fixed;
     const float inv_scale = ldexpf(1.f, -st->fx_shift);
     const int half_row = row >> 1;
@@ -878,9 +889,12 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-__global__ void k_window_finish(DeviceStatus *__restrict__ st, double *field_corner)
+__global__ void k_window_finish(DeviceStatus *st, double *field_corner, bool clean)
 {
-    *field_corner += ldexp((double)st->alt_sum, -(st->fx_shift + 4));
+    wait_previous();
+    st = fresh(st);
+    *field_corner = (clean ? 0.0 : *field_corner) +
+                    ldexp((double)st->alt_sum, -(st->fx_shift + 4));
     st->alt_sum = 0;  // zero for the next pass
 }
 
@@ -987,6 +1001,7 @@ WinParams make_win_params(const DepositGeom &g, const DepositArgs &a, int chunk)
     p.pass_mass = 0.0;
     p.mean_fixed = 0;
     p.field_mass = p.field_sub = nullptr;
+    p.clean = a.clean ? 1 : 0;
     return p;
 }
 
@@ -1026,10 +1041,9 @@ cudaError_t window_convert(const GridGeom &g, const unsigned long long *acc, flo
                            bool clean, const DeviceStatus *dstat, int num_sms,
                            cudaStream_t stream, int64_t *launches)
 {
-    k_window_convert<<<num_sms * 8, 256, 0, stream>>>(acc, grid, g.dims, g.row, g.nfloat / 2,
-                                                      clean ? 1 : 0, dstat);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(k_window_convert, num_sms * 8, 256, 0, stream, acc, grid, g.dims, g.row,
+                        g.nfloat / 2, clean ? 1 : 0, dstat);
 }
 
 cudaError_t deposit_window_pass(const DepositGeom &g, const DepositArgs &a, int chunk,
@@ -1050,12 +1064,16 @@ cudaError_t deposit_window_pass(const DepositGeom &g, const DepositArgs &a, int 
     const double n3 = (double)g.grid.dims * g.grid.dims * g.grid.dims;
     WinParams p = make_win_params(g, a, chunk);
     if (a.masses) {
-        k_mass_reduce<<<mass_ctas, 256, 0, stream>>>(a.masses, a.n, mass_part, dstat);
+        if ((err = launch_after(k_mass_reduce, mass_ctas, 256, 0, stream, a.masses, a.n, mass_part,
+                                dstat)) != cudaSuccess)
+            return err;
         mark("win_mass");
     }
     if (a.masses || p.nchunks == 0) {
-        k_window_prep<<<1, 1, 0, stream>>>(mass_part, a.masses ? mass_ctas : 0, (double)a.mass,
-                                           a.n, 1.0 / n3, a.field_mass, a.field_sub, dstat);
+        if ((err = launch_after(k_window_prep, 1, 1, 0, stream, mass_part,
+                                a.masses ? mass_ctas : 0, (double)a.mass, a.n, 1.0 / n3, a.clean,
+                                a.field_mass, a.field_sub, dstat)) != cudaSuccess)
+            return err;
         mark("win_prep");
     } else {
         // a uniform mass: the constants need nothing from the device, and the
@@ -1100,22 +1118,20 @@ cudaError_t deposit_window_pass(const DepositGeom &g, const DepositArgs &a, int 
                                         : k_stream_deposit<false, false, true>);
         if ((err = ensure_dynamic_smem(kern, (size_t)smem)) != cudaSuccess)
             return err;
-        kern<<<ctas, kWinThreads, smem, stream>>>(p, dstat, acc);
-        mark(stream_mode ? "stream_deposit" : "win_deposit");
-        if ((err = cudaGetLastError()) != cudaSuccess)
+        if ((err = launch_after(kern, ctas, kWinThreads, (size_t)smem, stream, p, dstat, acc)) !=
+            cudaSuccess)
             return err;
+        mark(stream_mode ? "stream_deposit" : "win_deposit");
     }
     if (!defer_convert) {
-        k_window_convert<<<num_sms * 8, 256, 0, stream>>>(acc, a.grid, g.grid.dims, g.grid.row,
-                                                          g.grid.nfloat / 2, a.clean ? 1 : 0,
-                                                          dstat);
-        mark("win_convert");
-        if ((err = cudaGetLastError()) != cudaSuccess)
+        if ((err = launch_after(k_window_convert, num_sms * 8, 256, 0, stream, acc, a.grid,
+                                g.grid.dims, g.grid.row, g.grid.nfloat / 2, a.clean ? 1 : 0,
+                                dstat)) != cudaSuccess)
             return err;
+        mark("win_convert");
     }
-    k_window_finish<<<1, 1, 0, stream>>>(dstat, a.field_corner);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(k_window_finish, 1, 1, 0, stream, dstat, a.field_corner, a.clean);
 }
 
 

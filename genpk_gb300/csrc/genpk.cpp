@@ -490,7 +490,7 @@ constexpr int kTuneReps = 2;
 // costs dominate, about even at 3e7 on a 128^3 grid, and 1.75x slower at 3e7
 // on a 256^3 grid, whose accumulator exceeds the L2.)  Every candidate writes
 // the same grid (the sums are exact), so the trials only cost time: each
-// overwrites the clean grid, and the field's running sums and the error
+// overwrites the clean grid and starts the field's running sums, and the error
 // counters are put back before the next.  The chosen candidate then runs as
 // the real pass.
 int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, bool with_stream,
@@ -511,14 +511,6 @@ int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, boo
         cudaEvent_t a, b;
         ~Ev() { cudaEventDestroy(a); cudaEventDestroy(b); }
     } ev{e0, e1};
-    auto reset_field = [&]() -> int {
-        GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass + f, 0, sizeof(double), ctx->stream));
-        GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass + ctx->nfields + f, 0, sizeof(double),
-                                   ctx->stream));
-        GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass + 2 * ctx->nfields + f, 0, sizeof(double),
-                                   ctx->stream));
-        return GENPK_OK;
-    };
     genpk_ctx::Tuned best;
     best.band = density_band(ctx, a.n);
     best.var = a.masses != nullptr;
@@ -541,7 +533,6 @@ int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, boo
         ctx->dscr.mass_part_cap = (int)mp;
         float ms = 1e30f;
         for (int rep = 0; rep < kTuneReps; rep++) {
-            GENPK_TRY(reset_field());
             GENPK_CUDA(cudaEventRecord(e0, ctx->stream));
             GENPK_CUDA(deposit_window_pass(g, a,
                                            stream_chunk(a.n, a.masses != nullptr, ctx->num_sms),
@@ -573,7 +564,6 @@ int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, boo
         GENPK_TRY(grow_sorted_scratch(ctx, g, a.n, ctas));
         float ms = 1e30f;
         for (int rep = 0; rep < kTuneReps; rep++) {
-            GENPK_TRY(reset_field());
             GENPK_CUDA(cudaEventRecord(e0, ctx->stream));
             GENPK_CUDA(deposit_pass(g, a, ctx->dscr, ctx->d_status, ctas, ctx->stream,
                                     &ctx->launches, nullptr, nullptr));
@@ -595,7 +585,6 @@ int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, boo
             best.tile = t;
         }
     }
-    GENPK_TRY(reset_field());
     GENPK_CUDA(cudaMemcpyAsync(ctx->d_status, ctx->d_probe + stash, 2 * sizeof(long long),
                                cudaMemcpyDeviceToDevice, ctx->stream));
     genpk_ctx::Tuned &slot = ctx->tuned[ctx->ntuned % genpk_ctx::kTuned];
@@ -1107,6 +1096,9 @@ int to_spectrum(genpk_ctx *ctx, const std::vector<int> &need, FusedAuto *fused =
         if (st == F_CLEAN) {
             GENPK_CUDA(cudaMemsetAsync(grid_of(ctx, f), 0, sizeof(float) * ctx->gg.nfloat,
                                        ctx->stream));
+            for (int k = 0; k < 3; k++)  // an empty grid's sums
+                GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass + k * ctx->nfields + f, 0,
+                                           sizeof(double), ctx->stream));
             ctx->state[(size_t)f] = F_DENSITY;
         }
         if (ctx->state[(size_t)f] == F_DENSITY)
@@ -1775,11 +1767,6 @@ int genpk_zero(genpk_ctx *ctx, int field)
     ctx->state[(size_t)field] = F_CLEAN;
     ctx->auto_valid[(size_t)field] = false;
     ctx->kzmajor[(size_t)field] = false;
-    GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass + field, 0, sizeof(double), ctx->stream));
-    GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass + ctx->nfields + field, 0, sizeof(double),
-                               ctx->stream));
-    GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass + 2 * ctx->nfields + field, 0, sizeof(double),
-                               ctx->stream));
     return GENPK_OK;
 }
 
@@ -2191,11 +2178,6 @@ int genpk_adjoint(genpk_ctx *ctx, int field, double boxsize, const float *pos, c
     if (recompute || !have) {
         ctx->state[(size_t)field] = F_CLEAN;
         ctx->kzmajor[(size_t)field] = false;
-        GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass + field, 0, sizeof(double), ctx->stream));
-        GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass + ctx->nfields + field, 0, sizeof(double),
-                                   ctx->stream));
-        GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass + 2 * ctx->nfields + field, 0,
-                                   sizeof(double), ctx->stream));
         GENPK_TRY(run_deposit(ctx, field, boxsize, dpos, dmass, (float)mass, n));
         GENPK_TRY(genpk_power(ctx, field, field, mass_norm, mass_norm, pw.data(), nullptr, nullptr));
     } else {
@@ -2571,7 +2553,7 @@ bool groupable(const genpk_batch *b, const double *boxsize, const float *const *
 }
 
 // One grouped pass of every box of group g into its field (which must be
-// clean, with zero field sums).
+// clean).
 int group_pass(genpk_batch::Group &g, const std::vector<GroupBox> &gb, TileShape tile)
 {
     genpk_ctx *ctx = g.ctx;
@@ -2614,7 +2596,6 @@ int tune_group(genpk_batch::Group &g, const std::vector<GroupBox> &gb)
         cudaEvent_t a, b;
         ~Ev() { cudaEventDestroy(a); cudaEventDestroy(b); }
     } ev{e0, e1};
-    const size_t sums = sizeof(double) * 3 * (size_t)ctx->nfields;
     float best_ms = 1e30f;
     ctx->ntrials = 0;
     for (const TileShape &t : tiles) {
@@ -2623,7 +2604,6 @@ int tune_group(genpk_batch::Group &g, const std::vector<GroupBox> &gb)
             continue;
         float ms = 1e30f;
         for (int rep = 0; rep < kTuneReps; rep++) {
-            GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass, 0, sums, ctx->stream));
             GENPK_CUDA(cudaEventRecord(e0, ctx->stream));
             GENPK_TRY(group_pass(g, gb, t));
             GENPK_CUDA(cudaEventRecord(e1, ctx->stream));
@@ -2643,7 +2623,6 @@ int tune_group(genpk_batch::Group &g, const std::vector<GroupBox> &gb)
             g.tile = t;
         }
     }
-    GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass, 0, sums, ctx->stream));
     g.tuned = true;
     return GENPK_OK;
 }
@@ -2677,8 +2656,6 @@ int group_issue(genpk_batch::Group &g, const double *boxsize, const float *const
         ctx->kzmajor[(size_t)f] = false;
         ctx->corner_valid[(size_t)f] = false;
     }
-    GENPK_CUDA(cudaMemsetAsync(ctx->d_field_mass, 0, sizeof(double) * 3 * (size_t)ctx->nfields,
-                               ctx->stream));
     if (!g.tuned || g.tuned_n != counts) {
         GENPK_TRY(tune_group(g, gb));
         g.tuned_n = counts;

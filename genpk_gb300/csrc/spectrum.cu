@@ -23,6 +23,7 @@
 // from the host tables.
 #include "common.cuh"
 #include "internal.h"
+#include "launch.cuh"
 
 #include <algorithm>
 
@@ -205,6 +206,12 @@ __global__ void __launch_bounds__(256)
         whist[i] = 0.0;
         rhist[i] = 0.f;
     }
+    wait_previous();
+#pragma unroll
+    for (int f = 0; f < NF; f++) {
+        p.f[f] = fresh(p.f[f]);
+        p.corner[f] = fresh(p.corner[f]);
+    }
     __syncthreads();
 
     const int64_t nrows = (int64_t)p.dims * p.dims;
@@ -386,6 +393,9 @@ __global__ void __launch_bounds__(256)
         whist[i] = 0.0;
         rhist[i] = 0.f;
     }
+    wait_previous();
+    p.f = fresh(p.f);
+    p.corner = fresh(p.corner);
     __syncthreads();
 
     const int64_t nrows = (int64_t)2 * p.hc * p.dims;  // half-rows
@@ -518,6 +528,9 @@ __global__ void __launch_bounds__(kFinalizeThreads)
                    const double *__restrict__ count, NormParams mn, double *__restrict__ power,
                    const DeviceStatus *__restrict__ st_in, DeviceStatus *__restrict__ st_out)
 {
+    wait_previous();
+    partial = fresh(partial);
+    st_in = fresh(st_in);
     if (st_out && blockIdx.x == 0 && threadIdx.x == 0)
         *st_out = *st_in;  // the pass's status words, beside the results
     __shared__ double sh[kFinalizeThreads];
@@ -629,7 +642,7 @@ cudaError_t bin_spectra(const GridGeom &g, const BinTables &t, const BinDevice &
         auto kern = k_bin<NF, CROSS1>;                                                        \
         if ((err = ensure_dynamic_smem(kern, smem)) != cudaSuccess)                           \
             return err;                                                                       \
-        kern<<<ctas, 32 * warps, smem, stream>>>(p, d.thr, d.iw, partial);                    \
+        err = launch_after(kern, ctas, 32 * warps, smem, stream, p, d.thr, d.iw, partial);    \
     } while (0)
     if (s.nf == 1)
         GENPK_BIN_LAUNCH(1, false);
@@ -643,7 +656,7 @@ cudaError_t bin_spectra(const GridGeom &g, const BinTables &t, const BinDevice &
         GENPK_BIN_LAUNCH(4, false);
 #undef GENPK_BIN_LAUNCH
     (*launches)++;
-    if ((err = cudaGetLastError()) != cudaSuccess)
+    if (err != cudaSuccess)
         return err;
     NormParams mn;
     mn.npc = s.np;
@@ -655,10 +668,9 @@ cudaError_t bin_spectra(const GridGeom &g, const BinTables &t, const BinDevice &
         mn.src[q] = s.cross1 ? 0 : pair_slot(s.nf, a, b);
     }
     const int k = l.npairs * t.nrbins;
-    k_bin_finalize<<<k, kFinalizeThreads, 0, stream>>>(partial, ctas, t.nrbins, d.count, mn,
-                                                        out_power, st_in, st_out);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(k_bin_finalize, k, kFinalizeThreads, 0, stream, partial, ctas, t.nrbins,
+                        d.count, mn, out_power, st_in, st_out);
 }
 
 int bin_kz_ctas(const GridGeom &g, int nrbins, int num_sms, int *warps, size_t *smem)
@@ -699,9 +711,8 @@ cudaError_t bin_spectrum_kz(const GridGeom &g, const BinTables &t, const BinDevi
     cudaError_t err;
     if ((err = ensure_dynamic_smem(k_bin_kz, smem)) != cudaSuccess)
         return err;
-    k_bin_kz<<<ctas, 32 * warps, smem, stream>>>(p, d.thr, d.iw, partial);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(k_bin_kz, ctas, 32 * warps, smem, stream, p, d.thr, d.iw, partial);
 }
 
 cudaError_t finalize_power(const double *partial, int ctas, int nrbins, const double *count,
@@ -715,10 +726,9 @@ cudaError_t finalize_power(const double *partial, int ctas, int nrbins, const do
         mn.mb[q] = q == 0 ? mb : 1.0;
         mn.src[q] = 0;
     }
-    k_bin_finalize<<<nrbins, kFinalizeThreads, 0, stream>>>(partial, ctas, nrbins, count, mn,
-                                                            out, st_in, st_out);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(k_bin_finalize, nrbins, kFinalizeThreads, 0, stream, partial, ctas, nrbins,
+                        count, mn, out, st_in, st_out);
 }
 
 cudaError_t finalize_powers(const double *partial, int ctas, int nrbins, int nfields,
@@ -735,11 +745,11 @@ cudaError_t finalize_powers(const double *partial, int ctas, int nrbins, int nfi
             mn.src[q] = q < k ? f0 + q : 0;
         }
         const bool last = f0 + k >= nfields;
-        k_bin_finalize<<<k * nrbins, kFinalizeThreads, 0, stream>>>(
-            partial, ctas, nrbins, count, mn, out + (size_t)f0 * nrbins, st_in,
-            last ? st_out : nullptr);
         (*launches)++;
-        cudaError_t err = cudaGetLastError();
+        const cudaError_t err = launch_after(k_bin_finalize, k * nrbins, kFinalizeThreads, 0, stream,
+                                             partial, ctas, nrbins, count, mn,
+                                             out + (size_t)f0 * nrbins, st_in,
+                                             last ? st_out : nullptr);
         if (err != cudaSuccess)
             return err;
     }

@@ -38,6 +38,7 @@
 //             the CTA partials.
 #include "common.cuh"
 #include "internal.h"
+#include "launch.cuh"
 
 #include <cuda.h>
 
@@ -468,14 +469,18 @@ __global__ void __launch_bounds__(kXThreads, kXCtasPerSm)
     if (BIN || GRAD)
         for (int i = tid; i <= p.nrbins; i += kXThreads)
             thr[i] = p.thr[i];
-    if (GRAD)
-        for (int i = tid; i < p.nrbins; i += kXThreads)
-            gco[i] = p.gcoef[i];
     if (tid == 0) {
         mbar_init(&bar[0]);
         mbar_init(&bar[1]);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_proxy_async();
+    }
+    wait_previous();
+    p.corner = fresh(p.corner);
+    if (GRAD) {
+        const float *gcoef = fresh(p.gcoef);
+        for (int i = tid; i < p.nrbins; i += kXThreads)
+            gco[i] = gcoef[i];
     }
     __syncthreads();
     // Binning each field of a batch: a CTA's tiles run through the fields in
@@ -771,6 +776,9 @@ __global__ void __launch_bounds__(kZThreads)
     extern __shared__ __align__(16) unsigned char zdyn[];  // [warps][M] V
     for (int i = threadIdx.x; i < N; i += blockDim.x)
         tw[i] = tw_g[i];
+    wait_previous();
+    in = fresh(in);
+    st = fresh(st);
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float2 *zs = zs_all[wid];
@@ -922,6 +930,9 @@ __global__ void __launch_bounds__(kTThreads)
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t row0 = (int64_t)blockIdx.x * kTRows;
     const int x = (int)(row0 / N), y0 = (int)(row0 - (int64_t)x * N);
+    wait_previous();
+    acc = fresh(acc);
+    st = fresh(st);
     const long long mean = st->mean_fixed;
     const float inv_scale = ldexpf(1.f, -st->fx_shift);
 
@@ -1005,6 +1016,8 @@ __global__ void __launch_bounds__(kTThreads)
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t row0 = (int64_t)blockIdx.x * kTRows;
     const int x = (int)(row0 / N), y0 = (int)(row0 - (int64_t)x * N);
+    wait_previous();
+    spec = fresh(spec);
     {
         // every load of this thread in flight before any store (the runs are
         // kTRows values of one kz plane, planes N^2 values apart)
@@ -1123,6 +1136,8 @@ __global__ void __launch_bounds__(kXThreads, kXCtasPerSm)
     const int c = tid % TZ, g = tid / TZ;
     for (int i = tid; i < N; i += kXThreads)
         tw_s[i] = tw_g[i];
+    wait_previous();
+    spec = fresh(spec);
     auto fetch = [&](int64_t t, float2 *dst) {
         const int64_t plane = t / tiles_per_plane;
         const int kz0 = (int)(t - plane * tiles_per_plane) * TZ;
@@ -1315,9 +1330,8 @@ cudaError_t launch_xfft(const GridGeom &g, float *grids, int nbatch, const float
     cudaError_t err;
     if ((err = ensure_dynamic_smem(kern, smem)) != cudaSuccess)
         return err;
-    kern<<<ctas, kXThreads, smem, stream>>>(map, p, dstat);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(kern, ctas, kXThreads, smem, stream, map, p, dstat);
 }
 
 }  // namespace
@@ -1370,9 +1384,8 @@ cudaError_t launch_zfft(const GridGeom &g, const T *in, float *grid, const float
     cudaError_t err;
     if ((err = ensure_dynamic_smem(kern, (size_t)pre)) != cudaSuccess)
         return err;
-    kern<<<ctas, kZThreads, pre, stream>>>(in, grid, nrows, g.row, tw, dstat);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(kern, ctas, kZThreads, (size_t)pre, stream, in, grid, nrows, g.row, tw, dstat);
 }
 
 }  // namespace
@@ -1403,10 +1416,9 @@ cudaError_t zfft_kz_pass(const GridGeom &g, float *grid, const unsigned long lon
     if ((err = ensure_dynamic_smem(k_zfft_t1024, smem)) != cudaSuccess)
         return err;
     const int64_t nrows = (int64_t)g.dims * g.dims;
-    k_zfft_t1024<<<(unsigned)(nrows / kTRows), kTThreads, smem, stream>>>(
-        acc, reinterpret_cast<float2 *>(grid), g.row, tw, dstat);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(k_zfft_t1024, (unsigned)(nrows / kTRows), kTThreads, smem, stream, acc,
+                        reinterpret_cast<float2 *>(grid), g.row, tw, dstat);
 }
 
 cudaError_t zifft_kz_pass(const GridGeom &g, const float *kz_major, float *out, const float2 *tw,
@@ -1420,10 +1432,9 @@ cudaError_t zifft_kz_pass(const GridGeom &g, const float *kz_major, float *out, 
     if ((err = ensure_dynamic_smem(k_zifft_t1024, smem)) != cudaSuccess)
         return err;
     const int64_t nrows = (int64_t)g.dims * g.dims;
-    k_zifft_t1024<<<(unsigned)(nrows / kTRows), kTThreads, smem, stream>>>(
-        reinterpret_cast<const float2 *>(kz_major), out, g.row, tw);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(k_zifft_t1024, (unsigned)(nrows / kTRows), kTThreads, smem, stream,
+                        reinterpret_cast<const float2 *>(kz_major), out, g.row, tw);
 }
 
 cudaError_t kz_to_rows(const GridGeom &g, const float2 *kz_major, float2 *rows,
@@ -1464,10 +1475,9 @@ cudaError_t yfft_pass(const GridGeom &g, float *grids, int nbatch, const float2 
     cudaError_t err;
     if ((err = ensure_dynamic_smem(kern, smem)) != cudaSuccess)
         return err;
-    kern<<<ctas, kXThreads, smem, stream>>>(reinterpret_cast<float2 *>(grids), g.hc, per_plane,
-                                            ntiles, tw);
     (*launches)++;
-    return cudaGetLastError();
+    return launch_after(kern, ctas, kXThreads, smem, stream, reinterpret_cast<float2 *>(grids), g.hc,
+                        per_plane, ntiles, tw);
 }
 
 int xfft_bin_ctas(int dims, int nbatch, int num_sms)
