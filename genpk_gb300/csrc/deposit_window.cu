@@ -309,9 +309,8 @@ __device__ __noinline__ void carry_corners(const WinParams &p, acc_t *acc, const
             acc_add_global(acc, corner_index(p, c, k), (long long)sign << 32);
 }
 
-// Block epilogue of both deposit kernels: the warps' shares of the exact
-// corner mode (fixed point, 2^-(s+4) units) and the invalid-particle and
-// wait-timeout counts.
+// Block epilogue of the windowed mode: the warps' shares of the exact corner mode
+// (fixed point, 2^-(s+4) units) and the invalid-particle and wait-timeout counts.
 template <bool VARMASS, bool CORNER>
 __device__ __forceinline__ void report_block(const WinParams &p, DeviceStatus *st, f2sum alt,
                                              unsigned bad, unsigned timeouts, float mscale)
@@ -341,6 +340,84 @@ __device__ __forceinline__ void report_block(const WinParams &p, DeviceStatus *s
         atomicAdd(&st->bad_particles, (unsigned long long)bad);
     if (lane == 0 && timeouts)
         atomicAdd(&st->timeouts, (unsigned long long)timeouts);
+}
+
+// The exact corner mode of a stream pass, in integers, so that it does not
+// depend on which CTA works a chunk.  Terms have magnitude <= 1 (a uniform mass
+// is factored out, others are scaled to the pass's largest); a thread's terms of
+// one chunk (at most 8) are summed as a float pair, which is rounded to
+// hi * 2^-18 + lo * 2^-40, the two limbs summed in 64 bits.  The rounding, 2^-41
+// a chunk and thread, leaves 5e-10 over 512^3 particles (2e-8 when each warp's
+// total over the pass was rounded to 2^-32).
+struct CornerSum {
+    long long hi, lo;
+};
+
+__device__ __forceinline__ void corner_add_chunk(CornerSum &c, f2sum v)
+{
+    v = two_sum(v.hi, v.lo);  // (the terms' low parts reach 2^-11 on the largest grids)
+    const float t = fmaf(v.hi, 262144.f, 12582912.f);
+    const float r = fmaf(-__fsub_rn(t, 12582912.f), 1.f / 262144.f, v.hi);  // exact
+    c.hi += __float_as_int(t) - kMagicBits;
+    c.lo += __float_as_int(fmaf(__fadd_rn(r, v.lo), 1099511627776.f, 12582912.f)) - kMagicBits;
+}
+
+// Block epilogue of the stream mode: the warps' corner sums and the
+// invalid-particle and wait-timeout counts.
+template <bool CORNER>
+__device__ __forceinline__ void report_stream_block(DeviceStatus *st, CornerSum c, unsigned bad,
+                                             unsigned timeouts)
+{
+    const int lane = threadIdx.x & 31;
+    if (CORNER) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            c.hi += __shfl_xor_sync(0xffffffffu, c.hi, o);
+            c.lo += __shfl_xor_sync(0xffffffffu, c.lo, o);
+        }
+        if (lane == 0) {
+            atomicAdd((unsigned long long *)&st->alt_hi, (unsigned long long)c.hi);
+            atomicAdd((unsigned long long *)&st->alt_lo, (unsigned long long)c.lo);
+        }
+    }
+    bad = __reduce_add_sync(0xffffffffu, bad);
+    timeouts = __reduce_add_sync(0xffffffffu, timeouts);
+    if (lane == 0 && bad)
+        atomicAdd(&st->bad_particles, (unsigned long long)bad);
+    if (lane == 0 && timeouts)
+        atomicAdd(&st->timeouts, (unsigned long long)timeouts);
+}
+
+// The stream mode hands out its chunks in order: a CTA's first two are fixed, the others come
+// from a pass-wide counter as it starts copying them.  With chunks b, b + CTAs,
+// ... the CTAs drifted apart by their speed (the two dies see the memory
+// differently), and the accumulator lines that neighbouring chunks share left
+// the L2 between their adds (512^3 lattice: +10 % DRAM reads, +28 % writes; the
+// kernel 1.24 -> 1.10 ms, 1024^3 11.1 -> 8.35).  (The windowed mode, whose
+// chunks flush few lines, is no faster for it.)
+struct ChunkFeed {
+    int cur, next;   // this chunk and the one being copied
+    int after;       // thread 0: the one after that
+};
+
+__device__ __forceinline__ ChunkFeed feed_start(DeviceStatus *st)
+{
+    ChunkFeed f;
+    f.cur = blockIdx.x;
+    f.next = f.cur + gridDim.x;
+    f.after = 0;
+    if (threadIdx.x == 0)
+        f.after = 2 * (int)gridDim.x + (int)atomicAdd(&st->next_chunk, 1u);
+    return f;
+}
+
+// Thread 0, while chunk `cur` is worked: the chunk after `next`, for everyone to
+// read behind the next barrier, and a request for one more (its answer is not
+// needed before the next call).
+__device__ __forceinline__ void feed_ahead(ChunkFeed &f, int *slot, DeviceStatus *st)
+{
+    *slot = f.after;
+    f.after = 2 * (int)gridDim.x + (int)atomicAdd(&st->next_chunk, 1u);
 }
 
 template <bool VARMASS, bool CORNER>
@@ -568,7 +645,12 @@ __global__ void __launch_bounds__(kWinThreads, 1)
 // each) and lane l skips those four reductions, so each such cell takes one
 // reduction for both.  The lower-z reductions of a warp cover consecutive
 // cells.  One barrier per chunk; the L2 holds the few x-planes that the
-// resident chunks touch.
+// resident chunks touch, as long as the chunks are worked in order (ChunkFeed).
+//
+// Bound by the SM's request port to the L2: about 58 sectors of reductions per
+// 32 particles, one a cycle, 76 % of its peak, at 220 instructions per 32
+// particles (257 with the general split's conversions and carries).  512^3
+// lattice 1.29 -> 1.10 ms, 1024^3 10.15 -> 8.35 ms.
 // Accumulator element of cell (x, y, z): 32-bit arithmetic where the grid has
 // fewer than 2^32 elements (WIDE = false), else 64-bit.
 template <bool WIDE>
@@ -584,6 +666,7 @@ __global__ void __launch_bounds__(kWinThreads, 1)
     float *pbuf = reinterpret_cast<float *>(win_smem);  // [2][chunk * 3]
     float *mbuf = pbuf + 6 * p.chunk;                   // [2][chunk] (VARMASS)
     __shared__ __align__(8) unsigned long long bar[2];
+    __shared__ int sh_next[2];
     const int lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         mbar_init(&bar[0], 1);
@@ -602,17 +685,17 @@ __global__ void __launch_bounds__(kWinThreads, 1)
     const unsigned umant = (ubits & 0x7fffffu) | 0x800000u;
     const int uef = (int)((ubits >> 23) & 0xffu);
     const bool uneg = (ubits >> 31) != 0u;
-    const float mscale = ldexpf(1.f, fxs + 4);
+    const float mscale = ldexpf(1.f, fxs - 28);  // the largest mass scales below 1
 
-    f2sum alt = {0.f, 0.f};
+    CornerSum corner = {0, 0};
     unsigned bad = 0, timeouts = 0;
     bool broken = false;  // a wait ran out: plain loads from then on
-    const int64_t c0 = blockIdx.x;
-    if (threadIdx.x == 0 && c0 < p.nchunks && chunk_by_bulk(p, c0))
-        issue_chunk<VARMASS>(p, c0, pbuf, mbuf, &bar[0]);
+    ChunkFeed feed = feed_start(st);
+    if (threadIdx.x == 0 && feed.cur < p.nchunks && chunk_by_bulk(p, feed.cur))
+        issue_chunk<VARMASS>(p, feed.cur, pbuf, mbuf, &bar[0]);
 
-    int k = 0;
-    for (int64_t c = c0; c < p.nchunks; c += gridDim.x, k++) {
+    for (int k = 0; feed.cur < p.nchunks; k++) {
+        const int64_t c = feed.cur;
         const int buf = k & 1;
         float *P = pbuf + buf * 3 * p.chunk;
         float *M = mbuf + buf * p.chunk;
@@ -620,11 +703,16 @@ __global__ void __launch_bounds__(kWinThreads, 1)
         // The chunk is in place, and every thread is done with the other buffer.
         arrive_chunk<VARMASS>(p, c, cnt, !broken && chunk_by_bulk(p, c), P, M, &bar[buf],
                               (unsigned)(k >> 1) & 1u, broken, timeouts);
-        if (threadIdx.x == 0 && !broken && c + gridDim.x < p.nchunks &&
-            chunk_by_bulk(p, c + gridDim.x))
-            issue_chunk<VARMASS>(p, c + gridDim.x, pbuf + (buf ^ 1) * 3 * p.chunk,
-                                 mbuf + (buf ^ 1) * p.chunk, &bar[buf ^ 1]);
+        if (k > 0)
+            feed.next = sh_next[buf ^ 1];
+        if (threadIdx.x == 0) {
+            if (!broken && feed.next < p.nchunks && chunk_by_bulk(p, feed.next))
+                issue_chunk<VARMASS>(p, feed.next, pbuf + (buf ^ 1) * 3 * p.chunk,
+                                     mbuf + (buf ^ 1) * p.chunk, &bar[buf ^ 1]);
+            feed_ahead(feed, &sh_next[buf], st);
+        }
 
+        f2sum alt = {0.f, 0.f};
         // Same trip count for every lane: the merge shuffles need full warps.
         for (int j0 = 0; j0 < cnt; j0 += blockDim.x) {
             const int j = j0 + threadIdx.x;
@@ -636,46 +724,24 @@ __global__ void __launch_bounds__(kWinThreads, 1)
                 if (VARMASS)
                     m = M[j];
             }
-            // The products split_q28 forms first.  Particles at 1 <= |x N/L| <
-            // 2^22 cells on every axis (all but those within a cell of the
-            // origin, far outside the box, or invalid) take the split without
-            // its near-origin step and clamp; the others the general split.
-            const float xh = __fmul_rn(x, p.uh), yh = __fmul_rn(y, p.uh), zh = __fmul_rn(z, p.uh);
-            bool fast = j < cnt && fabsf(xh) >= 1.f && fabsf(xh) < kFastSplitMax &&
-                        fabsf(yh) >= 1.f && fabsf(yh) < kFastSplitMax && fabsf(zh) >= 1.f &&
-                        fabsf(zh) < kFastSplitMax;
+            AxisQ a[3];
+            bool valid = split3_fast<CORNER>(x, y, z, p.uh, p.ul, p.dims, a) && j < cnt;
             if (VARMASS)
-                fast = fast && fabsf(m) <= 3.4028235e38f;
-            bool valid = fast;
-            AxisQ ax, ay, az;
-            if (fast) {
-                ax = split_q28_unwrapped(x, xh, p.uh, p.ul);
-                ay = split_q28_unwrapped(y, yh, p.uh, p.ul);
-                az = split_q28_unwrapped(z, zh, p.uh, p.ul);
-                // as unsigned values, so that a negative cell reads as out of range
-                if (max((unsigned)ax.cell, max((unsigned)ay.cell, (unsigned)az.cell)) >=
-                    (unsigned)p.dims) {
-                    ax.cell = wrap_cell(ax.cell, p.dims);
-                    ay.cell = wrap_cell(ay.cell, p.dims);
-                    az.cell = wrap_cell(az.cell, p.dims);
-                }
-            } else {
-                valid = j < cnt;
+                valid = valid && fabsf(m) <= 3.4028235e38f;
+            if (!valid && j < cnt) {  // outside the box, a carry, or invalid
+                valid = fabsf(x * p.uh) <= kPosLimit && fabsf(y * p.uh) <= kPosLimit &&
+                        fabsf(z * p.uh) <= kPosLimit;
+                if (VARMASS)
+                    valid = valid && fabsf(m) <= 3.4028235e38f;
                 if (valid) {
-                    bool ok = fabsf(xh) <= kPosLimit && fabsf(yh) <= kPosLimit &&
-                              fabsf(zh) <= kPosLimit;
-                    if (VARMASS)
-                        ok = ok && fabsf(m) <= 3.4028235e38f;
-                    if (!ok) {
-                        bad++;
-                        valid = false;
-                        x = y = z = 0.f;
-                    }
+                    a[0] = split_q28(x, p.uh, p.ul, p.dims);
+                    a[1] = split_q28(y, p.uh, p.ul, p.dims);
+                    a[2] = split_q28(z, p.uh, p.ul, p.dims);
+                } else {
+                    bad++;
                 }
-                ax = split_q28(x, p.uh, p.ul, p.dims);
-                ay = split_q28(y, p.uh, p.ul, p.dims);
-                az = split_q28(z, p.uh, p.ul, p.dims);
             }
+            const AxisQ &ax = a[0], &ay = a[1], &az = a[2];
             unsigned mant = umant;
             int ef = uef;
             bool neg = uneg;
@@ -762,8 +828,11 @@ __global__ void __launch_bounds__(kWinThreads, 1)
                 }
             }
         }
+        if (CORNER)
+            corner_add_chunk(corner, alt);
+        feed.cur = feed.next;
     }
-    report_block<VARMASS, CORNER>(p, st, alt, bad, timeouts, mscale);
+    report_stream_block<CORNER>(st, corner, bad, timeouts);
 }
 
 // Per-CTA FP64 mass partials (Kahan in FP32 first) and the max |mass|.
@@ -889,13 +958,21 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-__global__ void k_window_finish(DeviceStatus *st, double *field_corner, bool clean)
+// The corner sum in mass units joins the grid's (a stream pass's limbs are in
+// units of a uniform mass umass, or, with umass 0, of 2^(28 - fx_shift)); what a
+// pass counts up is zero again for the next.
+__global__ void k_window_finish(DeviceStatus *st, double *field_corner, double umass, bool clean)
 {
     wait_previous();
     st = fresh(st);
+    const double unit = umass != 0.0 ? umass : ldexp(1.0, 28 - st->fx_shift);
     *field_corner = (clean ? 0.0 : *field_corner) +
-                    ldexp((double)st->alt_sum, -(st->fx_shift + 4));
-    st->alt_sum = 0;  // zero for the next pass
+                    ldexp((double)st->alt_sum, -(st->fx_shift + 4)) +
+                    (ldexp((double)st->alt_hi, -18) + ldexp((double)st->alt_lo, -40)) * unit;
+    st->alt_sum = 0;
+    st->alt_hi = 0;
+    st->alt_lo = 0;
+    st->next_chunk = 0u;
 }
 
 // Probe: for up to `samples` evenly spread chunks, the window volume in cells
@@ -1131,7 +1208,8 @@ cudaError_t deposit_window_pass(const DepositGeom &g, const DepositArgs &a, int 
         mark("win_convert");
     }
     (*launches)++;
-    return launch_after(k_window_finish, 1, 1, 0, stream, dstat, a.field_corner, a.clean);
+    return launch_after(k_window_finish, 1, 1, 0, stream, dstat, a.field_corner,
+                        a.masses ? 0.0 : (double)a.mass, a.clean);
 }
 
 

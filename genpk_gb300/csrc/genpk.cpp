@@ -37,14 +37,15 @@ constexpr int kMaxStages = 64;
 constexpr int64_t kWindowMinParticles = (int64_t)1 << 20;
 constexpr int64_t kZeroCopyMinParticles = (int64_t)1 << 20;
 constexpr double kWindowMaxCellsPerParticle = 64.0;
-// Coherent passes whose consecutive particles mostly advance one z cell along
-// one (x, y) cell column (a lattice at about one particle per cell) take the
-// stream mode: its neighbour merge then halves the reductions, and windows
-// would merge few adds.  Measured at 512^3 particles (Zel'dovich lattice):
-// merge rate 0.93 on a 512^3 grid (stream 1.41 ms, window 1.75 ms); 0.65 on
-// 384^3 / 512^3, 0.49 on 512^3 / 256^3 and 0.02 on 256^3 / 512^3, where the
-// window mode is 2-17 % faster.
-constexpr double kStreamMergeRate = 0.8;
+// Coherent passes more than half of whose consecutive particles advance one z
+// cell along one (x, y) cell column (a lattice at about one particle per cell)
+// take the stream mode: its neighbour merge then halves the reductions, and
+// windows would merge few adds.  Measured (Zel'dovich lattices, merge rate:
+// stream and window ms): 512^3 on 512^3 0.94: 1.10 and 1.81; 384^3 0.65: 0.85 and
+// 0.93; 352^3 0.53: 0.77 and 0.92; 180^3 on 256^3 0.55: 0.13 and 0.19; 256^3 on
+// 512^3 0.02: 0.57 and 0.50.  Below one half the windows merge as much as the
+// lanes (512^3 particles along a Morton curve: 2.32 and 2.22).
+constexpr double kStreamMergeRate = 0.52;
 
 struct Pending {
     bool active = false;

@@ -83,6 +83,8 @@ struct DeviceStatus {
     int fx_shift;                      // weights are accumulated as round(w * 2^fx_shift)
     unsigned max_mass_bits;            // max |mass| of the pass, as float bits
     unsigned long long pass_bad;       // particles the current binned pass has skipped
+    long long alt_hi, alt_lo;          // stream passes: the same in two limbs
+    unsigned next_chunk;               // stream passes: chunks handed out
 };
 
 struct DepositArgs {
