@@ -33,6 +33,11 @@
 //     reductions, merged between neighbouring lanes of one z cell column.
 //     Chosen by the merge rate k_stream_probe measures.
 //
+//   k_direct_deposit  for particles in no order that are too few for a sort to
+//     pay: one particle per thread, its weights straight to the accumulator,
+//     lane pairs sharing the sectors; k_direct_convert then writes the FP32
+//     grid and clears the accumulator behind itself.
+//
 // Sums are exact: the window cells (32-bit, overflows moved on as 2^32 units)
 // and the pass accumulator (64-bit) are integers of 2^-s mass units (the
 // sorted engine's weights, common.cuh pair_w / z_mass / corner_w);
@@ -835,6 +840,232 @@ __global__ void __launch_bounds__(kWinThreads, 1)
     report_stream_block<CORNER>(st, corner, bad, timeouts);
 }
 
+// ---- direct passes -----------------------------------------------------------
+//
+// Particles in no order, few enough that a sort's kernels cost more than the
+// scattered reductions: one particle per thread, eight 64-bit reductions each.
+// Every reduction goes to the L2 as a 32-byte sector of its own, at about 200 G
+// a second, which bounds the pass; so lanes 2i and 2i + 1 swap weights (one
+// shuffle per (x, y) corner) and both add the lower- and upper-z weight of one
+// particle, then of the other: the two lie in one sector three times out of
+// four.  1 M particles on 128^3: 68 -> 47 us (the stream kernel without its
+// merges); 40 k on 64^3, where the pass is latency: 5 us against 24 for the
+// binned sort's three kernels.
+constexpr int kDirectThreads = 256;
+
+template <bool VARMASS, bool CORNER, bool WIDE>
+__global__ void __launch_bounds__(kDirectThreads)
+    k_direct_deposit(WinParams p, DeviceStatus *st, acc_t *acc)
+{
+    typedef typename CellIndex<WIDE>::T I;
+    wait_previous();
+    st = fresh(st);
+    const int lane = threadIdx.x & 31;
+    const bool odd = (lane & 1) != 0;
+    const int fxs = VARMASS ? st->fx_shift : p.fx_shift;
+    const int emax = 154 - fxs;
+    const unsigned ubits = __float_as_uint(p.umass);
+    const float mscale = ldexpf(1.f, fxs - 28);  // the largest mass scales below 1
+    f2sum alt = {0.f, 0.f};
+    unsigned bad = 0;
+    // (whole warps go round together: the pairs' shuffles need them)
+    for (int64_t i = (int64_t)blockIdx.x * kDirectThreads + threadIdx.x; i - lane < p.n;
+         i += (int64_t)gridDim.x * kDirectThreads) {
+        float x = 0.f, y = 0.f, z = 0.f, m = p.umass;
+        if (i < p.n) {
+            x = __ldg(p.pos + 3 * i);
+            y = __ldg(p.pos + 3 * i + 1);
+            z = __ldg(p.pos + 3 * i + 2);
+            if (VARMASS)
+                m = __ldg(p.masses + i);
+        }
+        AxisQ a[3];
+        bool valid = split3_fast<CORNER>(x, y, z, p.uh, p.ul, p.dims, a) && i < p.n;
+        if (VARMASS)
+            valid = valid && fabsf(m) <= 3.4028235e38f;
+        if (!valid && i < p.n) {  // outside the box, a carry, or invalid
+            valid = fabsf(x * p.uh) <= kPosLimit && fabsf(y * p.uh) <= kPosLimit &&
+                    fabsf(z * p.uh) <= kPosLimit;
+            if (VARMASS)
+                valid = valid && fabsf(m) <= 3.4028235e38f;
+            if (valid) {
+                a[0] = split_q28(x, p.uh, p.ul, p.dims);
+                a[1] = split_q28(y, p.uh, p.ul, p.dims);
+                a[2] = split_q28(z, p.uh, p.ul, p.dims);
+            } else {
+                bad++;
+            }
+        }
+        const unsigned mb = VARMASS ? __float_as_uint(m) : ubits;
+        const int ef = (int)((mb >> 23) & 0xffu);
+        const unsigned mant = (mb & 0x7fffffu) | 0x800000u;
+        const bool neg = (mb >> 31) != 0u;
+        valid = valid && ef != 0;  // zero or subnormal mass deposits nothing
+        const int dsh = VARMASS ? max(emax - ef, 0) : 0;
+        if (CORNER && valid) {
+            f2sum v = corner_factor_q(a[0], a[1], a[2]);
+            if (VARMASS) {
+                const float mm = m * mscale;
+                const float h = __fmul_rn(v.hi, mm);
+                v = f2sum{h, fmaf(v.hi, mm, -h) + v.lo * mm};
+            }
+            f2_accumulate(alt, f2_signed(v, a[0].cell ^ a[1].cell ^ a[2].cell));
+        }
+        const uint32_t qx = a[0].q, qy = a[1].q, qz = a[2].q;
+        const uint32_t rx = kFracOne - qx, ry = kFracOne - qy, rz = kFracOne - qz;
+        const uint32_t pw[4] = {pair_w(rx, ry), pair_w(qx, ry), pair_w(rx, qy), pair_w(qx, qy)};
+        const uint32_t zl = z_mass(rz, mant, dsh), zu = z_mass(qz, mant, dsh);
+
+        // This particle's and the pair's other particle's cells and wraps.
+        const I own = (I)a[0].cell * (I)p.plane + (I)(a[1].cell * p.row + a[2].cell);
+        const int wrap = (a[0].cell + 1 == p.dims ? 1 : 0) | (a[1].cell + 1 == p.dims ? 2 : 0) |
+                         (a[2].cell + 1 == p.dims ? 4 : 0) | (valid ? 8 : 0) | (neg ? 16 : 0);
+        const I other = __shfl_xor_sync(0xffffffffu, own, 1);
+        const int wrap_o = __shfl_xor_sync(0xffffffffu, wrap, 1);
+        // first the even lane's particle, then the odd lane's; the even lane
+        // adds lower-z weights, the odd lane upper-z ones
+        const I at[2] = {odd ? other : own, odd ? own : other};
+        const int wr[2] = {odd ? wrap_o : wrap, odd ? wrap : wrap_o};
+        I base[2], dx[2], dy[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            dx[k] = (wr[k] & 1) ? -(I)(p.dims - 1) * (I)p.plane : (I)p.plane;
+            dy[k] = (I)((wr[k] & 2) ? -(p.dims - 1) * p.row : p.row);
+            base[k] = at[k] + (odd ? (I)((wr[k] & 4) ? -(p.dims - 1) : 1) : (I)0);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint32_t wl = corner_w(pw[q], zl), wu = corner_w(pw[q], zu);
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? wl : wu, 1);
+            const uint32_t w[2] = {odd ? got : wl, odd ? wu : got};
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const I cell = base[k] + ((q & 1) ? dx[k] : (I)0) + ((q & 2) ? dy[k] : (I)0);
+                if (wr[k] & 8)
+                    atomicAdd(acc + cell, (acc_t)((wr[k] & 16) ? -(long long)w[k] : (long long)w[k]));
+            }
+        }
+    }
+    CornerSum c = {0, 0};
+    if (CORNER) {
+        alt = two_sum(alt.hi, alt.lo);
+        c.hi = __float2ll_rn(alt.hi * 262144.f);
+        const float r = fmaf(-__ll2float_rn(c.hi), 1.f / 262144.f, alt.hi);  // exact
+        c.lo = __float2ll_rn(__fadd_rn(r, alt.lo) * 1099511627776.f);
+    }
+    const unsigned skipped = __reduce_add_sync(0xffffffffu, bad);
+    if (lane == 0 && skipped)
+        atomicAdd(&st->pass_bad, (unsigned long long)skipped);
+    report_stream_block<CORNER>(st, c, bad, 0u);
+}
+
+// What ends a direct pass.  A uniform mass's constants come from the host for
+// all n particles; where some were skipped (st->pass_bad), they are formed again
+// from the rest.  Others' were set before the pass (k_window_prep).
+struct DirectEnd {
+    int var;
+    double umass;
+    long long n;
+    PassConsts host;
+    double inv_cells;
+    int clean;
+    double *field_mass, *field_sub, *field_corner;
+};
+
+__device__ __forceinline__ PassConsts direct_consts(const DirectEnd &e, const DeviceStatus *st)
+{
+    if (e.var)
+        return {st->pass_mass, st->fx_shift, st->mean_fixed};
+    const unsigned long long bad = st->pass_bad;
+    if (bad == 0)
+        return e.host;
+    return pass_consts((double)(e.n - (long long)bad) * e.umass, (float)fabs(e.umass),
+                       e.inv_cells);
+}
+
+__device__ __forceinline__ void end_direct(const DirectEnd &e, const PassConsts &k,
+                                           DeviceStatus *st)
+{
+    if (!e.var) {
+        st->pass_mass = k.mass;
+        st->fx_shift = k.fx_shift;
+        st->mean_fixed = k.mean_fixed;
+        add_pass_sums(k, e.clean != 0, e.field_mass, e.field_sub);
+    }
+    const double unit = e.var ? ldexp(1.0, 28 - k.fx_shift) : e.umass;
+    *e.field_corner = (e.clean ? 0.0 : *e.field_corner) +
+                      (ldexp((double)st->alt_hi, -18) + ldexp((double)st->alt_lo, -40)) * unit;
+    st->alt_hi = 0;
+    st->alt_lo = 0;
+    st->pass_bad = 0;
+}
+
+// The end of a direct pass whose sums stay in the accumulator (one thread).
+__global__ void k_direct_end(const __grid_constant__ DirectEnd e, DeviceStatus *st)
+{
+    wait_previous();
+    st = fresh(st);
+    end_direct(e, direct_consts(e, st), st);
+}
+
+// k_window_convert that leaves the accumulator zero behind it (the next pass
+// needs no clear) and ends the pass: the last block to have read the constants
+// does that.  Two cells per thread and round, four rounds' loads ahead of their
+// stores: with each pair cleared right after its load, loads waited 5 us for
+// the stores beside them (256^3 grid: 340 us, 54 so; 128^3 26 and 13).
+__global__ void __launch_bounds__(256)
+    k_direct_convert(acc_t *acc, float *__restrict__ grid, int dims, int row, unsigned npairs,
+                     const __grid_constant__ DirectEnd e, DeviceStatus *st)
+{
+    __shared__ long long sh_mean;
+    __shared__ float sh_scale;
+    wait_previous();
+    acc = fresh(acc);
+    st = fresh(st);
+    if (threadIdx.x == 0) {
+        const PassConsts k = direct_consts(e, st);
+        sh_mean = k.mean_fixed;
+        sh_scale = ldexpf(1.f, -k.fx_shift);
+        __threadfence();
+        if (atomicAdd(&st->ticket, 1u) == gridDim.x - 1) {
+            end_direct(e, k, st);
+            st->ticket = 0u;
+        }
+    }
+    __syncthreads();
+    const long long mean = sh_mean;
+    const float inv_scale = sh_scale;
+    const unsigned half_row = (unsigned)row >> 1;
+    const unsigned last = (unsigned)(dims - 1) >> 1;  // the pair holding z = dims - 1
+    const unsigned stride = gridDim.x * 256;
+    for (unsigned k0 = blockIdx.x * 256 + threadIdx.x; k0 < npairs; k0 += 4 * stride) {
+        longlong2 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (k0 + u * stride < npairs)
+                v[u] = __ldcs(reinterpret_cast<longlong2 *>(acc) + k0 + u * stride);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const unsigned k = k0 + u * stride;
+            const unsigned z = k % half_row;
+            if (k >= npairs || z > last)
+                continue;
+            float2 f = make_float2(i64_to_f32_rn(v[u].x - mean) * inv_scale,
+                                   i64_to_f32_rn(v[u].y - mean) * inv_scale);
+            float2 *dst = reinterpret_cast<float2 *>(grid) + k;
+            if (!e.clean) {
+                const float2 o = *dst;
+                f = make_float2(o.x + f.x, o.y + f.y);
+            }
+            if (z < last || !(dims & 1))
+                *dst = f;
+            else
+                grid[2 * (size_t)k] = f.x;
+            __stcs(reinterpret_cast<longlong2 *>(acc) + k, make_longlong2(0, 0));
+        }
+    }
+}
+
 // Per-CTA FP64 mass partials (Kahan in FP32 first) and the max |mass|.
 __global__ void __launch_bounds__(256)
     k_mass_reduce(const float *__restrict__ masses, int64_t n, double *__restrict__ mass_part,
@@ -1082,6 +1313,19 @@ WinParams make_win_params(const DepositGeom &g, const DepositArgs &a, int chunk)
     return p;
 }
 
+// 32-bit element indices (false) where every index and both of the stream
+// mode's sentinels fit.  The environment variable GENPK_WIDE_INDEX=1 forces the
+// 64-bit variants on any grid (a test hook: they otherwise run only from
+// N = 1626 up).
+bool wide_index(const GridGeom &g)
+{
+    static const bool force_wide = [] {
+        const char *e = std::getenv("GENPK_WIDE_INDEX");
+        return e && e[0] == '1';
+    }();
+    return force_wide || g.nfloat >= ((int64_t)1 << 32) - 2;
+}
+
 }  // namespace
 
 int window_cap_cells(int chunk, bool variable_masses)
@@ -1176,14 +1420,7 @@ cudaError_t deposit_window_pass(const DepositGeom &g, const DepositArgs &a, int 
         const int smem = stream_mode ? p.win_off : p.win_off + 4 * p.cap;
         auto kern = a.masses ? (p.corner ? k_window_deposit<true, true> : k_window_deposit<true, false>)
                              : (p.corner ? k_window_deposit<false, true> : k_window_deposit<false, false>);
-        // 32-bit element indices where every index and both sentinels fit.  The
-        // environment variable GENPK_WIDE_INDEX=1 forces the 64-bit variant on any grid
-        // (a test hook: that variant otherwise runs only from N = 1626 up).
-        static const bool force_wide = [] {
-            const char *e = std::getenv("GENPK_WIDE_INDEX");
-            return e && e[0] == '1';
-        }();
-        if (stream_mode && !force_wide && g.grid.nfloat < ((int64_t)1 << 32) - 2)
+        if (stream_mode && !wide_index(g.grid))
             kern = a.masses ? (p.corner ? k_stream_deposit<true, true, false>
                                         : k_stream_deposit<true, false, false>)
                             : (p.corner ? k_stream_deposit<false, true, false>
@@ -1212,5 +1449,73 @@ cudaError_t deposit_window_pass(const DepositGeom &g, const DepositArgs &a, int 
                         a.masses ? 0.0 : (double)a.mass, a.clean);
 }
 
+cudaError_t deposit_direct_pass(const DepositGeom &g, const DepositArgs &a, double *mass_part,
+                                int mass_ctas, unsigned long long *acc, size_t clear_bytes,
+                                bool defer_convert, int num_sms, DeviceStatus *dstat,
+                                cudaStream_t stream, int64_t *launches, StageHook hook,
+                                void *hook_user)
+{
+    auto mark = [&](const char *name) {
+        (*launches)++;
+        if (hook)
+            hook(hook_user, name);
+    };
+    cudaError_t err;
+    WinParams p = make_win_params(g, a, kStreamChunk);
+    DirectEnd e;
+    e.var = a.masses ? 1 : 0;
+    e.umass = (double)a.mass;
+    e.n = (long long)a.n;
+    e.inv_cells = 1.0 / ((double)g.grid.dims * g.grid.dims * g.grid.dims);
+    e.host = pass_consts((double)a.n * e.umass, (float)fabs(e.umass), e.inv_cells);
+    e.clean = a.clean ? 1 : 0;
+    e.field_mass = a.field_mass;
+    e.field_sub = a.field_sub;
+    e.field_corner = a.field_corner;
+    p.fx_shift = e.host.fx_shift;
+    if (a.masses) {
+        if ((err = launch_after(k_mass_reduce, mass_ctas, 256, 0, stream, a.masses, a.n, mass_part,
+                                dstat)) != cudaSuccess)
+            return err;
+        mark("win_mass");
+        if ((err = launch_after(k_window_prep, 1, 1, 0, stream, mass_part, mass_ctas,
+                                (double)a.mass, a.n, e.inv_cells, a.clean, a.field_mass,
+                                a.field_sub, dstat)) != cudaSuccess)
+            return err;
+        mark("win_prep");
+    }
+    if (clear_bytes) {
+        clear_bytes = std::min(clear_bytes, sizeof(acc_t) * (size_t)g.grid.nfloat);
+        if ((err = cudaMemsetAsync(acc, 0, clear_bytes, stream)) != cudaSuccess)
+            return err;
+        mark("win_clear");
+    }
+    const bool wide = wide_index(g.grid);
+    auto kern = a.masses ? (p.corner ? (wide ? k_direct_deposit<true, true, true>
+                                             : k_direct_deposit<true, true, false>)
+                                     : (wide ? k_direct_deposit<true, false, true>
+                                             : k_direct_deposit<true, false, false>))
+                         : (p.corner ? (wide ? k_direct_deposit<false, true, true>
+                                             : k_direct_deposit<false, true, false>)
+                                     : (wide ? k_direct_deposit<false, false, true>
+                                             : k_direct_deposit<false, false, false>));
+    const unsigned ctas = (unsigned)std::max<int64_t>(
+        1, std::min<int64_t>((a.n + kDirectThreads - 1) / kDirectThreads, (int64_t)num_sms * 16));
+    if ((err = launch_after(kern, ctas, kDirectThreads, 0, stream, p, dstat, acc)) != cudaSuccess)
+        return err;
+    mark("direct_deposit");
+    if (defer_convert) {
+        (*launches)++;
+        return launch_after(k_direct_end, 1, 1, 0, stream, e, dstat);
+    }
+    const unsigned pairs = (unsigned)(g.grid.nfloat / 2);
+    const unsigned cctas =
+        (unsigned)std::min<int64_t>(((int64_t)pairs + 511) / 512, (int64_t)num_sms * 8);
+    if ((err = launch_after(k_direct_convert, cctas, 256, 0, stream, acc, a.grid, g.grid.dims,
+                            g.grid.row, pairs, e, dstat)) != cudaSuccess)
+        return err;
+    mark("direct_convert");
+    return cudaSuccess;
+}
 
 }  // namespace genpk

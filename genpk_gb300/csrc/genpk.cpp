@@ -248,6 +248,19 @@ size_t acc_bytes(const genpk_ctx *ctx)
     return sizeof(unsigned long long) * (size_t)ctx->gg.nfloat;
 }
 
+// How much of the accumulator a pass has to clear before it adds to it.  The
+// accumulator counts as unknown from here on (a pass that fails part-way must
+// not leave it marked clear).
+size_t acc_clear_bytes(genpk_ctx *ctx)
+{
+    const size_t clear = ctx->acc_zero ? 0 : ctx->acc_dirty_bytes ? ctx->acc_dirty_bytes
+                                                                   : acc_bytes(ctx);
+    ctx->acc_zero = false;
+    ctx->acc_dirty_bytes = 0;
+    ctx->acc_spent = false;
+    return clear;
+}
+
 // The accumulator's first `bytes` bytes were overwritten (used as a float
 // buffer): only they need clearing if the rest was zero.
 void acc_overwritten(genpk_ctx *ctx, size_t bytes)
@@ -478,6 +491,11 @@ int density_band(const genpk_ctx *ctx, int64_t n)
 }
 
 constexpr int64_t kTuneMinParticles = (int64_t)1 << 16;
+// The largest accumulator of a direct pass below that count (N = 264).  A direct
+// pass reads, converts and clears it whole; us of the deposit, direct and binned
+// sort, 40 k particles: 20 and 29 on 64^3, 25 and 41 on 128^3, 42 and 60 on
+// 200^3, 76 and 97 on 256^3.
+constexpr size_t kDirectMaxBytes = (size_t)150 << 20;
 // Timed runs per candidate (the fastest counts): single runs of a small pass
 // varied by 10-20 %, enough to flip close choices from run to run.
 constexpr int kTuneReps = 2;
@@ -533,23 +551,28 @@ int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, boo
         GENPK_TRY(grow(ctx, &ctx->dscr.mass_part, &mp, (size_t)mass_ctas));
         ctx->dscr.mass_part_cap = (int)mp;
         float ms = 1e30f;
+        const bool zero0 = ctx->acc_zero, spent0 = ctx->acc_spent;
+        const size_t dirty0 = ctx->acc_dirty_bytes;
         for (int rep = 0; rep < kTuneReps; rep++) {
+            const size_t clear = acc_clear_bytes(ctx);
             GENPK_CUDA(cudaEventRecord(e0, ctx->stream));
-            GENPK_CUDA(deposit_window_pass(g, a,
-                                           stream_chunk(a.n, a.masses != nullptr, ctx->num_sms),
-                                           true, ctx->dscr.mass_part, mass_ctas,
-                                           ctx->dscr.win_acc, acc_bytes(ctx), false, ctx->num_sms,
+            GENPK_CUDA(deposit_direct_pass(g, a, ctx->dscr.mass_part, mass_ctas,
+                                           ctx->dscr.win_acc, clear, false, ctx->num_sms,
                                            ctx->d_status, ctx->stream, &ctx->launches, nullptr,
                                            nullptr));
+            ctx->acc_zero = true;
             GENPK_CUDA(cudaEventRecord(e1, ctx->stream));
             GENPK_CUDA(cudaEventSynchronize(e1));
             float t = 0.f;
             GENPK_CUDA(cudaEventElapsedTime(&t, e0, e1));
             ms = std::min(ms, t);
         }
-        ctx->acc_zero = false;  // it holds the trial's sums
-        ctx->acc_dirty_bytes = 0;
-        ctx->acc_spent = true;
+        // The trials leave the accumulator zero; it is recorded as it was before
+        // them, so that a call that tunes ends in the state of one that does not
+        // (the graphs compare them).
+        ctx->acc_zero = zero0;
+        ctx->acc_spent = spent0;
+        ctx->acc_dirty_bytes = dirty0;
         ctx->trial_tile[0] = TileShape{0, 0, 0};
         ctx->trial_ctas[0] = 0;
         ctx->trial_ms[0] = ms;
@@ -741,6 +764,20 @@ int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const f
         }
         stage_event(ctx, "probe");
     }
+    // Particles in no order: the tuner's stream candidate is the direct pass, and
+    // so is an automatic pass too small to tune, of a uniform mass, where the
+    // accumulator stays in the L2 (it counts as the sorted engine's).
+    bool direct = engine == GENPK_ENGINE_STREAM && no_order;
+    const bool small = auto_sorted && engine == GENPK_ENGINE_SORTED && n < kTuneMinParticles &&
+                       !masses && acc_bytes(ctx) <= kDirectMaxBytes;
+    if (small && !s.win_acc) {
+        GENPK_CUDA(cudaStreamSynchronize(ctx->stream));
+        if (cudaMalloc(&s.win_acc, acc_bytes(ctx)) != cudaSuccess) {
+            cudaGetLastError();
+            s.win_acc = nullptr;
+        }
+    }
+    direct = direct || (small && s.win_acc);
     if ((engine == GENPK_ENGINE_WINDOW || engine == GENPK_ENGINE_STREAM) && !s.win_acc) {
         // The window engine's accumulator (8 bytes per grid element) is allocated on first
         // use; where it does not fit (the largest grids) an automatic pass takes the sorted
@@ -754,9 +791,11 @@ int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const f
                 return fail(ctx, GENPK_ERR_NOMEM,
                             "window engine: the 64-bit accumulator does not fit in device memory");
             engine = GENPK_ENGINE_SORTED;
+            direct = false;
         }
     }
-    const bool chunked = engine == GENPK_ENGINE_WINDOW || engine == GENPK_ENGINE_STREAM;
+    const bool chunked = !direct &&
+                         (engine == GENPK_ENGINE_WINDOW || engine == GENPK_ENGINE_STREAM);
     if (engine == GENPK_ENGINE_STREAM)
         chunk = stream_chunk(n, masses != nullptr, ctx->num_sms);
     if (chunked && ctx->inject_chunk >= 0) {
@@ -764,7 +803,7 @@ int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const f
         a.skip_wait = ctx->inject_clocks;
         ctx->inject_chunk = -1;
     }
-    if (host_mapped && !chunked) {
+    if (host_mapped && !chunked && !direct) {
         // The sorted engine reads positions twice: copy them over once instead.
         GENPK_TRY(ensure_stage(ctx, n));
         GENPK_CUDA(cudaMemcpyAsync(ctx->stage_pos, pos, sizeof(float) * 3 * (size_t)n,
@@ -785,21 +824,24 @@ int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const f
     bool own = a.clean && chunked && (use_xfft(ctx) || use_kz(ctx));
     if (no_order && use_xfft(ctx))
         own = a.clean && n >= kTuneMinParticles && n < own_transform_limit(ctx->dims);
-    if (chunked) {
+    if (chunked || direct) {
         const int mass_ctas = ctx->num_sms * 4;
         size_t mp = (size_t)s.mass_part_cap;
         GENPK_TRY(grow(ctx, &s.mass_part, &mp, (size_t)mass_ctas));
         s.mass_part_cap = (int)mp;
         const bool defer = own;
-        // (a pass that fails part-way must not leave the accumulator marked clear)
-        const size_t clear = ctx->acc_zero ? 0 : ctx->acc_dirty_bytes ? ctx->acc_dirty_bytes
-                                                                       : acc_bytes(ctx);
-        ctx->acc_zero = false;
-        ctx->acc_dirty_bytes = 0;
-        GENPK_CUDA(deposit_window_pass(g, a, chunk, engine == GENPK_ENGINE_STREAM, s.mass_part,
+        const size_t clear = acc_clear_bytes(ctx);
+        if (direct) {
+            GENPK_CUDA(deposit_direct_pass(g, a, s.mass_part, mass_ctas, s.win_acc, clear, defer,
+                                           ctx->num_sms, ctx->d_status, ctx->stream,
+                                           &ctx->launches, hook, ctx));
+            ctx->acc_zero = !defer;  // cleared behind the conversion
+        } else {
+            GENPK_CUDA(deposit_window_pass(g, a, chunk, engine == GENPK_ENGINE_STREAM, s.mass_part,
                                        mass_ctas, s.win_acc, clear, defer, ctx->num_sms,
                                        ctx->d_status, ctx->stream, &ctx->launches, hook, ctx));
-        ctx->acc_spent = !defer;  // converted in the pass
+            ctx->acc_spent = !defer;  // converted in the pass
+        }
         if (defer)
             ctx->acc_pending = f;
     } else {

@@ -85,6 +85,7 @@ struct DeviceStatus {
     unsigned long long pass_bad;       // particles the current binned pass has skipped
     long long alt_hi, alt_lo;          // stream passes: the same in two limbs
     unsigned next_chunk;               // stream passes: chunks handed out
+    unsigned ticket;                   // direct passes: blocks that have read the constants
 };
 
 struct DepositArgs {
@@ -213,6 +214,15 @@ cudaError_t deposit_window_pass(const DepositGeom &g, const DepositArgs &a, int 
                                 int num_sms,
                                 DeviceStatus *dstat, cudaStream_t stream, int64_t *launches,
                                 StageHook hook, void *hook_user);
+// A pass over particles in no order without a sort: as deposit_window_pass,
+// with scattered reductions (k_direct_deposit).  Unless the conversion is
+// deferred, the accumulator is zero again after the pass.  Grids of fewer than
+// 2^33 elements.
+cudaError_t deposit_direct_pass(const DepositGeom &g, const DepositArgs &a, double *mass_part,
+                                int mass_ctas, unsigned long long *acc, size_t clear_bytes,
+                                bool defer_convert, int num_sms, DeviceStatus *dstat,
+                                cudaStream_t stream, int64_t *launches, StageHook hook,
+                                void *hook_user);
 // The accumulator of the last window pass minus its mean, rounded once to FP32,
 // into `grid` (clean: stored, else added).
 cudaError_t window_convert(const GridGeom &g, const unsigned long long *acc, float *grid,

@@ -227,7 +227,10 @@ int genpk_set_deposit_tile(genpk_ctx *ctx, int tile_x, int tile_y, int tile_z);
  *  STREAM: the window engine's chunk pipeline without windows: reductions
  *          straight to the accumulator, merged between neighbouring particles
  *          of one z cell column; for coherent order at about one particle per
- *          cell, where windows merge few adds.
+ *          cell, where windows merge few adds.  (Chosen automatically for
+ *          particles in no order, it takes its form without the merges; passes
+ *          of fewer than 65536 such particles take that too where the
+ *          accumulator is small, and count as SORTED.)
  *  AUTO (default): from a sample of particle chunks, STREAM or WINDOW when the
  *          order is coherent (by window cells per particle), else SORTED. */
 #define GENPK_ENGINE_AUTO 0

@@ -1,0 +1,103 @@
+"""Direct passes (particles in no order, too few for a sort to pay) at the edges
+of their range: the automatic engine's grid against the sorted engine's bit for
+bit, and P(k) against the oracle, 1e-5 per bin (the last bin is the corner mode).
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gp(native_lib):
+    import torch
+    assert torch.cuda.is_available(), "GPU tests need a CUDA device"
+    import genpk_gb300
+    return genpk_gb300
+
+
+@pytest.mark.parametrize("dims,n,mass", [
+    (3, 1, 1.0),            # odd grid, one lane of one pair
+    (5, 31, -2.0),          # a warp short of one lane
+    (64, 257, 1.0),         # one particle past a block
+    (75, 4001, 0.25),       # odd grid: half-padded rows
+    (264, 65535, 3.0),      # the largest grid and count of an untuned direct pass
+    (265, 5000, 1.0),       # one past that grid: the sort
+    (128, 0, 1.0),
+])
+def test_small_unordered_passes(gp, dims, n, mass):
+    box = 1000.0
+    rng = np.random.default_rng(dims)
+    pos = (rng.random((n, 3)) * box).astype(np.float32)
+    if n > 100:
+        pos[::7] += np.float32(box)       # periodic images
+        pos[1::9, 2] = np.float32(box * (1 - 0.3 / dims))  # the wrapped upper z cell
+        pos[2::11] = 0.0
+    norm = abs(mass) * n + 1.0
+    with gp.Context(dims, 8) as ctx:
+        got = []
+        for _ in range(3):  # the accumulator is clear again after each
+            ctx.zero(0)
+            ctx.deposit(0, box, pos, None, mass)
+            got.append((ctx.read_field(0), ctx.power(0, 0, norm, norm)[0]))
+        assert all(np.array_equal(g[0], got[0][0]) and np.array_equal(g[1], got[0][1]) for g in got)
+        # two passes onto one grid: each adds its own, each minus its own mean
+        ctx.zero(0)
+        ctx.deposit(0, box, pos, None, mass)
+        ctx.sync()
+        ctx.deposit(0, box, pos, None, mass)
+        twice = ctx.read_field(0)
+        ctx.set_engine(gp.api.ENGINE_SORTED)
+        ctx.zero(0)
+        ctx.deposit(0, box, pos, None, mass)
+        assert np.array_equal(ctx.read_field(0), got[0][0])
+        ctx.sync()
+        ctx.deposit(0, box, pos, None, mass)
+        assert np.array_equal(ctx.read_field(0), twice)
+    if n >= 1000:
+        pr, cr, _ = O.pk(pos, box, dims, 8, None, mass, m_norm=norm)
+        ok = cr > 0
+        assert (np.abs(got[0][1][ok] - pr[ok]) / pr[ok]).max() <= 1e-5
+
+
+def test_skipped_particles_in_a_direct_pass(gp):
+    box, n, dims = 1000.0, 3000, 64
+    pos = (np.random.default_rng(1).random((n, 3)) * box).astype(np.float32)
+    bad = pos.copy()
+    bad[[0, 33, n - 1], [0, 1, 2]] = [np.nan, np.inf, -1e30]
+    keep = np.ones(n, bool)
+    keep[[0, 33, n - 1]] = False
+    with gp.Context(dims, 8) as ctx:
+        ctx.deposit(0, box, pos[keep], None, 1.0)
+        want = ctx.read_field(0)
+        for _ in range(2):
+            ctx.zero(0)
+            ctx.deposit(0, box, bad, None, 1.0)
+            with pytest.raises(gp.GenPKError) as e:
+                ctx.read_field(0)
+            assert "3 particle(s)" in str(e.value)
+            assert np.array_equal(ctx.read_field(0), want)
+
+
+@pytest.mark.parametrize("mass", ["one", "signed"])
+@pytest.mark.parametrize("dims", [75, 128])
+def test_tuned_unordered_passes(gp, dims, mass):
+    """Counts that the tuner times: whichever of the direct pass and the sort it
+    keeps, the grid is the sorted engine's."""
+    box, n = 1000.0, 70_001
+    rng = np.random.default_rng(dims)
+    pos = (rng.random((n, 3)) * box).astype(np.float32)
+    m = None
+    if mass == "signed":
+        m = (rng.lognormal(0.0, 1.0, n) * np.where(rng.random(n) < 0.3, -1, 1)).astype(np.float32)
+        m[::50] = 0.0
+    with gp.Context(dims, 8) as ctx:
+        ctx.deposit(0, box, pos, m, 1.0)
+        auto = ctx.read_field(0)
+        assert ((0, 0, 0), 0) in [(t, c) for t, c, _ in ctx.deposit_trials()]
+        ctx.set_engine(gp.api.ENGINE_SORTED)
+        ctx.zero(0)
+        ctx.deposit(0, box, pos, m, 1.0)
+        assert np.array_equal(ctx.read_field(0), auto)
