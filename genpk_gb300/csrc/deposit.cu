@@ -942,7 +942,6 @@ struct TileParams {
     int64_t plane;
     int row;
     int ntx, nty, ntz;
-    float mass;  // uniform mass when the particles carry none
 };
 
 constexpr int kTileThreads = 512;
@@ -1022,7 +1021,8 @@ struct ChunkRecords {
 // particles weigh a uniform mass, and its constants come from the host, for all
 // n[b] particles (where some were skipped, st->pass_bad of them, the mean is
 // formed again from the rest), and the box's first tile puts them in the status
-// words and the running sums.  Else the sort kernel's last CTA did.
+// words and the running sums.  Else the sort kernel's last CTA did.  umass is the
+// uniform mass either way.
 struct TileConsts {
     int host[kMaxGroupBoxes];
     int fx_shift[kMaxGroupBoxes];
@@ -1164,7 +1164,7 @@ __global__ void __launch_bounds__(kTileThreads, 4)
     // Weights in 2^-s mass units with s = 154 - emax (common.cuh pair_w / z_mass /
     // corner_w, as the window engine computes them).
     const int emax = 154 - s;
-    const unsigned ubits = __float_as_uint(p.mass);
+    const unsigned ubits = __float_as_uint((float)consts.umass[tb.box]);  // (it was a float)
     const unsigned umant = (ubits & 0x7fffffu) | 0x800000u;
     const int uef = (int)((ubits >> 23) & 0xffu);
     const bool uneg = (ubits >> 31) != 0u;
@@ -1409,8 +1409,7 @@ struct TileTarget {
     float *grid;
     int64_t grid_stride;
     int nbox;
-    float mass;  // uniform mass when !var
-    bool var;    // records carry the masses
+    bool var;    // weights from the records' masses, else from the boxes' uniform masses
     bool clean;
     TileConsts consts;
     PassEnd end;
@@ -1430,7 +1429,6 @@ cudaError_t launch_tile_kernels(const DepositGeom &g, const TileTarget &a, const
     tp.ntx = g.ntx;
     tp.nty = g.nty;
     tp.ntz = g.ntz;
-    tp.mass = a.mass;
     const size_t smem = sizeof(uint4) * ((2 * L::NACC + 3) / 4);
     const bool var = a.var;
     const dim3 tiles((unsigned)g.ntz, (unsigned)g.nty, (unsigned)(g.ntx * a.nbox));
@@ -1679,12 +1677,13 @@ cudaError_t deposit_pass(const DepositGeom &g, const DepositArgs &a, DepositScra
 {
     const OneBox src{sort_params(g, a.pos, a.masses, a.mass, a.n, g.units_hi, g.units_lo,
                                  sort_ctas)};
-    TileTarget t{a.grid, 0, 1, a.mass, a.masses != nullptr, a.clean, {}, {}};
+    TileTarget t{a.grid, 0, 1, a.masses != nullptr, a.clean, {}, {}};
     t.consts.inv_cells = 1.0 / ((double)g.grid.dims * g.grid.dims * g.grid.dims);
     t.consts.field_mass = a.field_mass;
     t.consts.field_sub = a.field_sub;
     t.end.field_corner = a.field_corner;
     t.end.clean = a.clean;
+    t.consts.umass[0] = (double)a.mass;
     if (deposit_binned(g)) {
         OneBin one = {};
         one.b.s = src.p;
@@ -1716,6 +1715,8 @@ cudaError_t deposit_pass(const DepositGeom &g, const DepositArgs &a, DepositScra
     return launch_tile_pass(g, t, RangeRecords{s.tile_start}, s, dstat, stream, launches, hook, hook_user);
 }
 
+// (At most sort_ctas of them in all, unless there are more boxes: one more than
+// the SMs hold at once would run alone after all the others.)
 GroupLayout deposit_group_layout(int nbox, const GroupBox *boxes, int sort_ctas)
 {
     GroupLayout lay = {};
@@ -1723,20 +1724,31 @@ GroupLayout deposit_group_layout(int nbox, const GroupBox *boxes, int sort_ctas)
     int64_t total = 0;
     for (int b = 0; b < nbox; b++)
         total += boxes[b].n;
+    int ctas[kMaxGroupBoxes], sum = 0;
+    for (int b = 0; b < nbox; b++) {
+        // (an empty box's one CTA sets its pass constants)
+        const double share = total > 0 ? (double)sort_ctas * (double)boxes[b].n / (double)total : 0.0;
+        ctas[b] = std::max(1, (int)share);
+        sum += ctas[b];
+    }
+    auto chunks = [&](int b) { return (boxes[b].n + kBinThreads - 1) / kBinThreads; };
+    for (; sum < sort_ctas; sum++) {  // the rest to the boxes whose CTAs have most to do
+        int most = -1;
+        for (int b = 0; b < nbox; b++)
+            if (ctas[b] < chunks(b) &&
+                (most < 0 || (double)boxes[b].n * ctas[most] > (double)boxes[most].n * ctas[b]))
+                most = b;
+        if (most < 0)
+            break;
+        ctas[most]++;
+    }
     int c = 0;
     int64_t r = 0;
     for (int b = 0; b < nbox; b++) {
-        const int64_t n = boxes[b].n;
-        int k = 1;  // (an empty box's one CTA sets its pass constants)
-        if (n > 0) {
-            const double share = (double)sort_ctas * (double)n / (double)total;
-            const int64_t chunks = (n + kBinThreads - 1) / kBinThreads;
-            k = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)std::llround(share), chunks));
-        }
         lay.cta0[b] = c;
         lay.rec0[b] = r;
-        c += k;
-        r += n;
+        c += (int)std::max<int64_t>(1, std::min<int64_t>(ctas[b], chunks(b)));
+        r += boxes[b].n;
     }
     lay.cta0[nbox] = c;
     lay.rec0[nbox] = r;
@@ -1753,8 +1765,15 @@ cudaError_t deposit_group_pass(const DepositGeom &g, const GroupLayout &lay, con
     if (nbox < 1 || nbox > kMaxGroupBoxes || !deposit_shared_hist(g) ||
         lay.rec0[nbox] > (int64_t)0xfffffffeLL)
         return cudaErrorInvalidValue;
-    // every box's records carry its mass bits, so the tile kernels read them
-    TileTarget t{grid0, grid_stride, nbox, 0.f, true, true, {}, {}};
+    // Every box's records carry its mass bits, which the tile kernel reads where
+    // some box's particles have masses of their own; else it takes the boxes'
+    // uniform masses (six boxes of 105 M particles on 256^3: 0.87 -> 0.70 ms).
+    bool var = false;
+    for (int b = 0; b < nbox; b++)
+        var = var || boxes[b].masses;
+    TileTarget t{grid0, grid_stride, nbox, var, true, {}, {}};
+    for (int b = 0; b < nbox; b++)
+        t.consts.umass[b] = (double)boxes[b].mass;
     t.consts.inv_cells = 1.0 / ((double)g.grid.dims * g.grid.dims * g.grid.dims);
     t.consts.field_mass = field_mass0;
     t.consts.field_sub = field_sub0;
