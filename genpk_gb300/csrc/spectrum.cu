@@ -38,7 +38,6 @@ struct BinParams {
     int dims, hc, half;
     int nrbins;
     float bpu_half;  // 0.5 * binsperunit as float, for the first-guess bin
-    int rp;          // modes per lane per piece (odd)
     int warps;       // warps per CTA
 };
 
@@ -115,19 +114,17 @@ __host__ __device__ inline BinLayout bin_layout(int nrbins, int hc, int np, int 
     return L;
 }
 
-constexpr int kMaxRP = 9;
-
 // One piece of a row: 32*RP consecutive modes from kz = pb, field values into
 // registers (coalesced loads; zero past the row's end).
-template <int NF>
+template <int NF, int RP>
 __device__ __forceinline__ void load_piece(const BinParams &p, int64_t r, int pb, int lane,
-                                           float2 (&v)[NF][kMaxRP])
+                                           float2 (&v)[NF][RP])
 {
     const size_t rowoff = (size_t)r * p.hc;
 #pragma unroll
-    for (int t = 0; t < kMaxRP; t++) {
+    for (int t = 0; t < RP; t++) {
         const int m = pb + t * 32 + lane;
-        const bool in = t < p.rp && m < p.hc;
+        const bool in = m < p.hc;
 #pragma unroll
         for (int f = 0; f < NF; f++)
             v[f][t] = in ? __ldg(p.f[f] + rowoff + m) : make_float2(0.f, 0.f);
@@ -137,9 +134,9 @@ __device__ __forceinline__ void load_piece(const BinParams &p, int64_t r, int pb
 // Registers -> the warp's staging buffer, with the two special modes fixed:
 // (0,0,0) is skipped (zeroed) and the exact corner value replaces the
 // transform's (N/2,N/2,N/2) mode.
-template <int NF>
+template <int NF, int RP>
 __device__ __forceinline__ void stage_piece(const BinParams &p, int64_t r, int pb, int lane,
-                                            float2 (&v)[NF][kMaxRP], float2 *buf, int piece)
+                                            float2 (&v)[NF][RP], float2 *buf, int piece)
 {
     if (r == 0 && pb == 0 && lane == 0) {
 #pragma unroll
@@ -148,7 +145,7 @@ __device__ __forceinline__ void stage_piece(const BinParams &p, int64_t r, int p
     }
     if (r == p.corner_row) {
 #pragma unroll
-        for (int t = 0; t < kMaxRP; t++) {
+        for (int t = 0; t < RP; t++) {
             if (pb + t * 32 + lane == p.half) {
 #pragma unroll
                 for (int f = 0; f < NF; f++)
@@ -159,12 +156,10 @@ __device__ __forceinline__ void stage_piece(const BinParams &p, int64_t r, int p
     }
     __syncwarp();
 #pragma unroll
-    for (int t = 0; t < kMaxRP; t++) {
-        if (t < p.rp) {
+    for (int t = 0; t < RP; t++) {
 #pragma unroll
-            for (int f = 0; f < NF; f++)
-                buf[f * piece + t * 32 + lane] = v[f][t];
-        }
+        for (int f = 0; f < NF; f++)
+            buf[f * piece + t * 32 + lane] = v[f][t];
     }
     __syncwarp();
 }
@@ -180,16 +175,25 @@ __device__ __forceinline__ void stage_piece(const BinParams &p, int64_t r, int p
 // are combined by a segmented warp scan over their (non-decreasing) bins and
 // each bin's last lane adds the total without atomics.  Every kPromoteRows
 // rows the touched FP32 bins are promoted into the warp's FP64 histogram.
-template <int NF, bool CROSS1>
-__global__ void __launch_bounds__(256)
+//
+// Bound by instruction issue and, on small grids, by its CTAs' start and end
+// (five rows a warp at N = 200): the stream of modes is 5 us of memory time
+// there.  RP is a template argument so that a lane's loads, stores and run
+// are unrolled at their true count - as a run-time value of up to 9 the
+// staging registers alone held a CTA to 3 per SM (68 registers; now 54, 4 per
+// SM and exactly two waves of the 1216 CTAs) and the row cost 509
+// instructions (now 410).  With k_bin_finalize: N = 200 40.3 -> 30.7 us,
+// N = 160 28.7 -> 22.5, N = 384 124 -> 96.
+template <int NF, bool CROSS1, int RP>
+__global__ void __launch_bounds__(256, NF == 1 ? 4 : 2)
     k_bin(BinParams p, const uint32_t *__restrict__ thr_g, const float *__restrict__ iw_g,
           double *__restrict__ partial)
 {
     constexpr int NP = PairSet<NF, CROSS1>::NP;
     extern __shared__ __align__(16) unsigned char smem[];
     const int nrb = p.nrbins;
-    const int rp = p.rp, piece = 32 * rp;
-    const BinLayout L = bin_layout(nrb, p.hc, NP, NF, rp);
+    constexpr int piece = 32 * RP;
+    const BinLayout L = bin_layout(nrb, p.hc, NP, NF, RP);
     uint32_t *thr = (uint32_t *)smem;
     float2 *izc = (float2 *)(smem + L.izc);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -222,22 +226,22 @@ __global__ void __launch_bounds__(256)
     int i = (int)(r_begin / p.dims), j = (int)(r_begin - (int64_t)i * p.dims);
     int bmin = nrb, bmax = -1;  // bins touched since the last FP64 promotion
     int rows_since = 0;
-    float2 v[NF][kMaxRP];
+    float2 v[NF][RP];
     if (r_begin < r_end)
-        load_piece<NF>(p, r_begin, 0, lane, v);
+        load_piece<NF, RP>(p, r_begin, 0, lane, v);
     for (int64_t r = r_begin; r < r_end; r++) {
         const int ki = kval_dev(i, p.dims), kj = kval_dev(j, p.dims);
         const uint32_t r2 = (uint32_t)(ki * ki + kj * kj);
         const float pxy = __ldg(iw_g + i) * __ldg(iw_g + j);
         for (int pb = 0; pb < p.hc; pb += piece) {
-            stage_piece<NF>(p, r, pb, lane, v, buf, piece);
+            stage_piece<NF, RP>(p, r, pb, lane, v, buf, piece);
             // next piece (this row's, or the next row's first) in flight
             if (pb + piece < p.hc)
-                load_piece<NF>(p, r, pb + piece, lane, v);
+                load_piece<NF, RP>(p, r, pb + piece, lane, v);
             else if (r + 1 < r_end)
-                load_piece<NF>(p, r + 1, 0, lane, v);
+                load_piece<NF, RP>(p, r + 1, 0, lane, v);
 
-            const int kz0 = pb + lane * rp;
+            const int kz0 = pb + lane * RP;
             int cb = nrb;  // key of a lane without modes: sorts after every bin
             float acc[NP];
 #pragma unroll
@@ -248,9 +252,12 @@ __global__ void __launch_bounds__(256)
                 cb = bin_lookup(kk2, thr, nrb, p.bpu_half);
                 bmin = min(bmin, cb);
                 uint32_t nx = thr[cb + 1];
-                const int lim = min(rp, p.hc - kz0);
-                const float2 *bl = buf + lane * rp;
-                for (int t = 0; t < lim; t++) {
+                const int lim = min(RP, p.hc - kz0);
+                const float2 *bl = buf + lane * RP;
+#pragma unroll
+                for (int t = 0; t < RP; t++) {
+                    if (t >= lim)
+                        break;
                     const int kz = kz0 + t;
                     if (kk2 >= nx) {
 #pragma unroll
@@ -340,6 +347,8 @@ __global__ void __launch_bounds__(256)
 // planes, 2 elsewhere; value c * p^4 |F|^2 with p = (iw_x iw_y) iw_z, the
 // float product order of k_bin; (0,0,0) skipped; the exact corner value at
 // (N/2, N/2, N/2).  One spectrum (its auto pair).
+constexpr int kKzMaxRP = 9;
+
 struct BinKzParams {
     const float2 *f;
     const double *corner;  // exact (N/2, N/2, N/2) value, or null
@@ -355,13 +364,13 @@ struct BinKzParams {
 
 // Half-row r (physical row r/2 = kz * N + x, half r & 1): piece loads.
 __device__ __forceinline__ void load_piece_kz(const BinKzParams &p, int64_t r, int pb, int lane,
-                                              float2 (&v)[kMaxRP])
+                                              float2 (&v)[kKzMaxRP])
 {
     const int h = (int)(r & 1);
     const int len = h ? p.half - 1 : p.hc;
     const float2 *row = p.f + (size_t)(r >> 1) * (size_t)p.dims;
 #pragma unroll
-    for (int t = 0; t < kMaxRP; t++) {
+    for (int t = 0; t < kKzMaxRP; t++) {
         const int m = pb + t * 32 + lane;
         const bool in = t < p.rp && m < len;
         const int y = h ? p.dims - 1 - m : m;
@@ -405,7 +414,7 @@ __global__ void __launch_bounds__(256)
     const int64_t r_begin = min(nrows, gw * per), r_end = min(nrows, r_begin + per);
     int bmin = nrb, bmax = -1;
     int rows_since = 0;
-    float2 v[kMaxRP];
+    float2 v[kKzMaxRP];
     if (r_begin < r_end)
         load_piece_kz(p, r_begin, 0, lane, v);
     for (int64_t r = r_begin; r < r_end; r++) {
@@ -430,13 +439,13 @@ __global__ void __launch_bounds__(256)
                 v[0] = make_float2(0.f, 0.f);
             if (corner) {
 #pragma unroll
-                for (int t = 0; t < kMaxRP; t++)
+                for (int t = 0; t < kKzMaxRP; t++)
                     if (pb + t * 32 + lane == p.half)
                         v[t] = make_float2((float)*p.corner, 0.f);
             }
             __syncwarp();
 #pragma unroll
-            for (int t = 0; t < kMaxRP; t++)
+            for (int t = 0; t < kKzMaxRP; t++)
                 if (t < rp)
                     buf[t * 32 + lane] = v[t];
             __syncwarp();
@@ -520,7 +529,10 @@ struct NormParams {
 };
 
 // One block per (pair, bin): strided sums over the CTA partials, then a
-// fixed-order tree, so the result does not depend on scheduling.
+// fixed-order tree, so the result does not depend on scheduling.  Bound by
+// latency: the loads of a thread are issued eight at a time and added in their
+// order, and the tree's last five levels are shuffles (1216 partials of a
+// N = 200 pass: 9.7 -> 7.6 us).
 constexpr int kFinalizeThreads = 256;
 
 __global__ void __launch_bounds__(kFinalizeThreads)
@@ -537,20 +549,36 @@ __global__ void __launch_bounds__(kFinalizeThreads)
     const int k = blockIdx.x;
     const int s = k / nrbins, b = k - s * nrbins;
     const size_t src = (size_t)mn.src[s] * nrbins + b;
+    const double cnt = count[b];
     double part = 0.0;
-    for (int c = threadIdx.x; c < ctas; c += blockDim.x)
-        part += partial[(size_t)c * mn.npc * nrbins + src];
+    constexpr int U = 8;  // loads in flight; added in the CTAs' order
+    for (int c0 = threadIdx.x; c0 < ctas; c0 += U * kFinalizeThreads) {
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int c = c0 + u * kFinalizeThreads;
+            v[u] = c < ctas ? partial[(size_t)c * mn.npc * nrbins + src] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (c0 + u * kFinalizeThreads < ctas)
+                part += v[u];
+    }
     sh[threadIdx.x] = part;
     __syncthreads();
-    for (int w = kFinalizeThreads / 2; w > 0; w >>= 1) {
+    for (int w = kFinalizeThreads / 2; w >= 32; w >>= 1) {
         if (threadIdx.x < w)
             sh[threadIdx.x] += sh[threadIdx.x + w];
         __syncthreads();
     }
+    if (threadIdx.x >= 32)
+        return;
+    double acc = sh[threadIdx.x];
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1)  // (the tree's last levels)
+        acc += __shfl_down_sync(0xffffffffu, acc, w);
     if (threadIdx.x != 0)
         return;
-    const double acc = sh[0];
-    const double cnt = count[b];
     double out = 0.0;
     if (cnt > 0.0) {
         out = acc / (mn.ma[s] * mn.mb[s]);
@@ -634,12 +662,15 @@ cudaError_t bin_spectra(const GridGeom &g, const BinTables &t, const BinDevice &
     p.half = g.half;
     p.nrbins = t.nrbins;
     p.bpu_half = (float)(0.5 * t.binsperunit);
-    p.rp = bin_rp(g.hc);
     p.warps = warps;
     cudaError_t err;
 #define GENPK_BIN_LAUNCH(NF, CROSS1)                                                          \
     do {                                                                                      \
-        auto kern = k_bin<NF, CROSS1>;                                                        \
+        const int rp = bin_rp(g.hc);                                                          \
+        auto kern = rp == 1   ? k_bin<NF, CROSS1, 1>                                          \
+                    : rp == 3 ? k_bin<NF, CROSS1, 3>                                          \
+                    : rp == 5 ? k_bin<NF, CROSS1, 5>                                          \
+                              : k_bin<NF, CROSS1, 9>;                                         \
         if ((err = ensure_dynamic_smem(kern, smem)) != cudaSuccess)                           \
             return err;                                                                       \
         err = launch_after(kern, ctas, 32 * warps, smem, stream, p, d.thr, d.iw, partial);    \
