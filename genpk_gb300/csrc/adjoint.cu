@@ -158,6 +158,8 @@ struct GatherParams {
     float mass;
     float dl_dm;
     int64_t n;
+    uint32_t plane_b, row_b;     // strides in bytes
+    uint32_t wrap_x, wrap_y, wrap_z;  // bytes from the last cell of an axis to the first
 };
 
 // The trilinear value and the three derivatives of dL/drho at one particle.
@@ -165,23 +167,11 @@ struct GatherOut {
     float gx, gy, gz, val;
 };
 
-__device__ __forceinline__ GatherOut gather_one(const GatherParams &p, const float *__restrict__ grid,
-                                                float x, float y, float z, float m)
+// The eight cell values g (bit 0: x, 1: y, 2: z) and the fractions d -> value
+// and derivatives, for a particle of mass m.
+__device__ __forceinline__ GatherOut gather_tree(const GatherParams &p, const float (&g)[8],
+                                                 const float (&d)[3], float m)
 {
-    int c[3];
-    float d[3];
-    split_cell(x, p.uh, p.ul, p.dims, c[0], d[0]);
-    split_cell(y, p.uh, p.ul, p.dims, c[1], d[1]);
-    split_cell(z, p.uh, p.ul, p.dims, c[2], d[2]);
-    int h[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-        h[a] = c[a] + 1 == p.dims ? 0 : c[a] + 1;
-    float g[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-        g[k] = __ldg(grid + cell_index(p.plane, p.row, (k & 1) ? h[0] : c[0], (k & 2) ? h[1] : c[1],
-                                       (k & 4) ? h[2] : c[2]));
     const float t0 = 1.f - d[0], t1 = 1.f - d[1];
     // Interpolate along z first, then y, then x; derivatives from the same tree.
     const float g00 = fmaf(d[2], g[4] - g[0], g[0]);  // (x0,y0)
@@ -200,6 +190,112 @@ __device__ __forceinline__ GatherOut gather_one(const GatherParams &p, const flo
     const float dgz = t0 * (t1 * e00 + d[1] * e01) + d[0] * (t1 * e10 + d[1] * e11);
     const float s = m * p.units;
     return {s * dgx, s * dgy, s * dgz, val};
+}
+
+// split_cell of an axis whose floor(xh) lies in [0, dims) and whose fraction
+// does not carry: the same cell and fraction without a conversion.  xh + 1.5 *
+// 2^23 rounded down holds floor(xh) in its low bits for 0 <= xh < 2^22; every
+// other xh (negative, larger, infinite, NaN) leaves a cell outside [0, dims).
+__device__ __forceinline__ void split_cell_fast(float x, float uh, float ul, uint32_t &cell,
+                                                float &frac)
+{
+    const float xh = __fmul_rn(x, uh);
+    const float xe = fmaf(x, uh, -xh);
+    const float xl = fmaf(x, ul, xe);
+    const float r = __fadd_rd(xh, 12582912.f);
+    frac = __fadd_rn(__fsub_rn(xh, __fsub_rn(r, 12582912.f)), xl);
+    cell = (uint32_t)(__float_as_int(r) - kMagicBits);
+}
+
+// How the four-particle kernel reads a particle's eight cells (gather_cells).
+enum Loads {
+    kGeneral,  // split_cell and 64-bit indices: a grid of 4 GB or more
+    kCells,    // eight 4-byte loads
+    kPairs,    // 8-byte loads of z pairs
+};
+
+// The cells and fractions of a particle; false for a non-finite one (whose
+// cells are 0).
+__device__ __forceinline__ bool split3_cell(const GatherParams &p, float x, float y, float z,
+                                            uint32_t (&c)[3], float (&d)[3])
+{
+    split_cell_fast(x, p.uh, p.ul, c[0], d[0]);
+    split_cell_fast(y, p.uh, p.ul, c[1], d[1]);
+    split_cell_fast(z, p.uh, p.ul, c[2], d[2]);
+    if (max(c[0], max(c[1], c[2])) < (uint32_t)p.dims &&
+        max(__float_as_uint(d[0]), max(__float_as_uint(d[1]), __float_as_uint(d[2]))) <
+            __float_as_uint(1.f))
+        return true;
+    const float v[3] = {x, y, z};
+    const bool finite = finite3(x, y, z);
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        int cell = 0;
+        d[a] = 0.f;
+        if (finite)
+            split_cell(v[a], p.uh, p.ul, p.dims, cell, d[a]);
+        c[a] = (uint32_t)cell;
+    }
+    return finite;
+}
+
+// The gather of a particle inside a grid below 4 GB, by 32-bit byte offsets.
+// PAIRS (even N): a z pair whose lower cell is even is one 8-byte load; an odd
+// lower cell's own pair holds only itself, the upper one is loaded alone.
+template <bool PAIRS>
+__device__ __forceinline__ GatherOut gather_cells(const GatherParams &p, const float *__restrict__ grid,
+                                                  const uint32_t (&c)[3], const float (&d)[3], float m)
+{
+    const uint32_t last = (uint32_t)p.dims - 1u;
+    const uint32_t sx = c[0] == last ? p.wrap_x : p.plane_b;
+    const uint32_t sy = c[1] == last ? p.wrap_y : p.row_b;
+    const char *base = reinterpret_cast<const char *>(grid);
+    const uint32_t row = c[0] * p.plane_b + c[1] * p.row_b;
+    float g[8];
+    if (PAIRS) {
+        const bool odd = c[2] & 1u;
+        const uint32_t o = row + (c[2] & ~1u) * 4u;
+        const uint32_t oz = c[2] == last ? p.wrap_z + 4u : 8u;  // (last is odd)
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t s = o + ((k & 1) ? sx : 0u) + ((k & 2) ? sy : 0u);
+            const float2 v = __ldg(reinterpret_cast<const float2 *>(base + s));
+            float up = v.y;
+            if (odd)
+                up = __ldg(reinterpret_cast<const float *>(base + (uint32_t)(s + oz)));
+            g[k] = odd ? v.y : v.x;
+            g[k + 4] = up;
+        }
+    } else {
+        const uint32_t o = row + c[2] * 4u;
+        const uint32_t sz = c[2] == last ? p.wrap_z : 4u;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            g[k] = __ldg(reinterpret_cast<const float *>(
+                base +
+                (uint32_t)(o + ((k & 4) ? sz : 0u) + ((k & 1) ? sx : 0u) + ((k & 2) ? sy : 0u))));
+    }
+    return gather_tree(p, g, d, m);
+}
+
+__device__ __forceinline__ GatherOut gather_one(const GatherParams &p, const float *__restrict__ grid,
+                                                float x, float y, float z, float m)
+{
+    int c[3];
+    float d[3];
+    split_cell(x, p.uh, p.ul, p.dims, c[0], d[0]);
+    split_cell(y, p.uh, p.ul, p.dims, c[1], d[1]);
+    split_cell(z, p.uh, p.ul, p.dims, c[2], d[2]);
+    int h[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+        h[a] = c[a] + 1 == p.dims ? 0 : c[a] + 1;
+    float g[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        g[k] = __ldg(grid + cell_index(p.plane, p.row, (k & 1) ? h[0] : c[0], (k & 2) ? h[1] : c[1],
+                                       (k & 4) ? h[2] : c[2]));
+    return gather_tree(p, g, d, m);
 }
 
 // One particle per thread, grid-stride.  (Tiles of 1024 particles staged
@@ -233,11 +329,15 @@ __global__ void __launch_bounds__(256)
 }
 
 // Four consecutive particles per thread: three 16-byte loads of positions
-// (and one of masses), the 32 grid loads of the four particles issued
-// together, three 16-byte stores of gradients.  The one-particle kernel's
-// thread waits out a position load and then the grid loads for every
-// particle; here each wait covers four.  Needs pos, gpos (and masses, gmass)
-// on 16-byte boundaries; the last n % 4 particles go one per thread.
+// (and one of masses), three 16-byte stores of gradients.  Needs pos, gpos (and
+// masses, gmass) on 16-byte boundaries; the last n % 4 particles go one per
+// thread.  Bound by instruction issue and the L1 data path (the 32 lanes' loads
+// of one of the eight cells lie in several lines): 172 instructions a particle
+// with split_cell and 64-bit indices, about 100 with the cell split without
+// conversions and 32-bit byte offsets.  512^3 lattice 0.80 -> 0.70 ms (0.57 ms
+// of memory time), 8 M particles in no order on 256^3 229 -> 162 us.  The 128
+// particles of a warp transposed through shared memory, so that its lanes hold
+// neighbours, took 0.78 ms.
 __device__ __forceinline__ GatherOut gather_or_zero(const GatherParams &p, const float *__restrict__ grid,
                                                     float x, float y, float z, float m)
 {
@@ -246,7 +346,22 @@ __device__ __forceinline__ GatherOut gather_or_zero(const GatherParams &p, const
     return gather_one(p, grid, x, y, z, m);
 }
 
-template <bool VARMASS>
+template <int LOADS>
+__device__ __forceinline__ GatherOut gather_any(const GatherParams &p, const float *__restrict__ grid,
+                                                float x, float y, float z, float m)
+{
+    if (LOADS == kGeneral)
+        return gather_or_zero(p, grid, x, y, z, m);
+    uint32_t c[3];
+    float d[3];
+    const bool finite = split3_cell(p, x, y, z, c, d);
+    const GatherOut o = gather_cells<LOADS == kPairs>(p, grid, c, d, m);
+    if (!finite)
+        return {0.f, 0.f, 0.f, -p.dl_dm};
+    return o;
+}
+
+template <bool VARMASS, int LOADS>
 __global__ void __launch_bounds__(256)
     k_gather4(GatherParams p, const float *__restrict__ grid, const float *__restrict__ pos,
               const float *__restrict__ masses, float *__restrict__ gpos, float *__restrict__ gmass)
@@ -261,10 +376,10 @@ __global__ void __launch_bounds__(256)
         float4 m = make_float4(p.mass, p.mass, p.mass, p.mass);
         if (VARMASS)
             m = __ldg(reinterpret_cast<const float4 *>(masses) + q);
-        const GatherOut o0 = gather_or_zero(p, grid, a.x, a.y, a.z, m.x);
-        const GatherOut o1 = gather_or_zero(p, grid, a.w, b.x, b.y, m.y);
-        const GatherOut o2 = gather_or_zero(p, grid, b.z, b.w, c.x, m.z);
-        const GatherOut o3 = gather_or_zero(p, grid, c.y, c.z, c.w, m.w);
+        const GatherOut o0 = gather_any<LOADS>(p, grid, a.x, a.y, a.z, m.x);
+        const GatherOut o1 = gather_any<LOADS>(p, grid, a.w, b.x, b.y, m.y);
+        const GatherOut o2 = gather_any<LOADS>(p, grid, b.z, b.w, c.x, m.z);
+        const GatherOut o3 = gather_any<LOADS>(p, grid, c.y, c.z, c.w, m.w);
         float4 *d = reinterpret_cast<float4 *>(gpos) + 3 * q;
         d[0] = make_float4(o0.gx, o0.gy, o0.gz, o1.gx);
         d[1] = make_float4(o1.gy, o1.gz, o2.gx, o2.gy);
@@ -330,7 +445,7 @@ cudaError_t adjoint_mode_gradient_coef(const GridGeom &g, const BinTables &t, co
 
 cudaError_t adjoint_gather(const GridGeom &g, float units_hi, float units_lo, const float *grid,
                            const float *pos, const float *masses, float mass, int64_t n,
-                           float *grad_pos, float *grad_mass, float dl_dmass_norm,
+                           float *grad_pos, float *grad_mass, float dl_dmass_norm, bool coherent,
                            cudaStream_t stream, int64_t *launches)
 {
     if (n <= 0)
@@ -345,6 +460,11 @@ cudaError_t adjoint_gather(const GridGeom &g, float units_hi, float units_lo, co
     p.mass = mass;
     p.dl_dm = dl_dmass_norm;
     p.n = n;
+    p.plane_b = (uint32_t)(4 * g.plane);
+    p.row_b = 4u * (uint32_t)g.row;
+    p.wrap_x = 0u - (uint32_t)(g.dims - 1) * p.plane_b;
+    p.wrap_y = 0u - (uint32_t)(g.dims - 1) * p.row_b;
+    p.wrap_z = 0u - (uint32_t)(g.dims - 1) * 4u;
     // Four CTAs per resident slot (8 per SM at 32-36 registers).  Sizing the
     // grid to the resident CTAs, so that the stride sweeps the particles in
     // order, cut the DRAM reads at 512^3 from 2.85 to 2.56 GB (2.15 GB of
@@ -353,9 +473,20 @@ cudaError_t adjoint_gather(const GridGeom &g, float units_hi, float units_lo, co
                      (!masses || (aligned16(masses) && aligned16(grad_mass)));
     if (vec) {
         const int blocks4 = (int)std::min<int64_t>(std::max<int64_t>((n / 4 + 255) / 256, 1), 152 * 32);
+        // Neighbouring lanes of a pass in grid order read neighbouring cells:
+        // a load is a few lines however wide it is, and the pairs' selections
+        // only cost (lattice 512^3: 0.70 ms, pairs 0.74).  Otherwise every lane
+        // reads its own sectors, and a pair is half as many (Morton order at
+        // 512^3 1.01 ms, cells 1.09; 8 M in no order on 256^3 162 us, cells 222;
+        // 2 M clustered on 160^3 43 us, cells 57).
+        const int loads = sizeof(float) * (uint64_t)g.nfloat > 0xffffffffull ? kGeneral
+                          : coherent || (g.dims & 1)                         ? kCells
+                                                                             : kPairs;
+        auto kern = loads == kGeneral ? (masses ? k_gather4<true, kGeneral> : k_gather4<false, kGeneral>)
+                    : loads == kCells ? (masses ? k_gather4<true, kCells> : k_gather4<false, kCells>)
+                                      : (masses ? k_gather4<true, kPairs> : k_gather4<false, kPairs>);
         (*launches)++;
-        return launch_after(masses ? k_gather4<true> : k_gather4<false>, blocks4, 256, 0, stream, p,
-                            grid, pos, masses, grad_pos, grad_mass);
+        return launch_after(kern, blocks4, 256, 0, stream, p, grid, pos, masses, grad_pos, grad_mass);
     }
     const int blocks = (int)std::min<int64_t>((n + 255) / 256, 152 * 32);
     (*launches)++;

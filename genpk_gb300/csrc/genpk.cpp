@@ -2293,7 +2293,8 @@ int genpk_adjoint(genpk_ctx *ctx, int field, double boxsize, const float *pos, c
         stage_event(ctx, "adj_c2r");
     const DepositGeom dg = deposit_geom(ctx, boxsize);
     GENPK_CUDA(adjoint_gather(ctx->gg, dg.units_hi, dg.units_lo, g, dpos, dmass, (float)mass, n,
-                              dgpos, dgmass, (float)dldm, ctx->stream, &ctx->launches));
+                              dgpos, dgmass, (float)dldm, ctx->last_engine == GENPK_ENGINE_STREAM,
+                              ctx->stream, &ctx->launches));
     stage_event(ctx, "adj_gather");
     if (!dev) {
         GENPK_CUDA(cudaMemcpyAsync(grad_pos, dgpos, sizeof(float) * 3 * (size_t)n,

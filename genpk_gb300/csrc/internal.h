@@ -421,7 +421,7 @@ cudaError_t zifft_kz_pass(const GridGeom &g, const float *kz_major, float *out, 
 // CIC gather of the real gradient grid: grad_pos[n][3], grad_mass[n] (optional).
 cudaError_t adjoint_gather(const GridGeom &g, float units_hi, float units_lo, const float *grid,
                            const float *pos, const float *masses, float mass, int64_t n,
-                           float *grad_pos, float *grad_mass, float dl_dmass_norm,
+                           float *grad_pos, float *grad_mass, float dl_dmass_norm, bool coherent,
                            cudaStream_t stream, int64_t *launches);
 
 int device_sm_count();
