@@ -749,10 +749,22 @@ struct ZPair<float> {
     static __device__ __forceinline__ float2 value(const V &a, long long, float) { return a; }
 };
 
+// Place of Z[i] in a warp's row (M = 32 R values): padded so that a half-warp's
+// 8-byte writes at the end of the transform fall into different banks (the 4
+// lanes of a group at R = 8 are 64 values apart, the 2 at R = 16 256), while
+// consecutive values stay in order.
+template <int R>
 __device__ __forceinline__ int zpad(int i)
 {
-    return i + (i >> 5);
+    return R == 16 ? i + 8 * (i >> 8) : R == 8 ? i + 4 * (i >> 6) : i + (i >> 5);
 }
+
+// The exchange before it: value (k1, l) at k1 * kZStep + l, so that a
+// half-warp's reads (4 k1 of 4 values at R = 8, 8 k1 of 2 at R = 16) do too.
+template <int R>
+constexpr int kZStep = R == 16 ? 34 : 36;
+template <int R>
+constexpr int kZRow = R >= 8 ? R * kZStep<R> : 33 * R;
 
 // Radix-2 decimation-in-frequency step across lanes xor s (upper lanes take
 // (a - b) W, lower lanes a + b).
@@ -771,11 +783,26 @@ __global__ void __launch_bounds__(kZThreads)
     typedef typename ZPair<T>::V V;
     constexpr int M = N / 2;
     constexpr int R = M / 32;
-    __shared__ float2 tw[N];
-    __shared__ float2 zs_all[kZThreads / 32][M + M / 32];  // Z[k] (or exchange) at zpad(k)
+    __shared__ float2 tw[M + 1];                   // W_N^k
+    __shared__ float2 tw1[R > 1 ? (R - 1) * 32 : 1];  // W_M^{lane k1} at [k1 - 1][lane]
+    __shared__ float2 tw2[R == 8 ? 7 * 4 : 32];  // R = 8: W_32^{q ki} at [ki - 1][q];
+                                                 // else W_{2s}^j at s + j, j < s
+    __shared__ float2 zs_all[kZThreads / 32][kZRow<R>];   // Z[k] at zpad(k), or exchange
     extern __shared__ __align__(16) unsigned char zdyn[];  // [warps][M] V
-    for (int i = threadIdx.x; i < N; i += blockDim.x)
+    for (int i = threadIdx.x; i <= M; i += blockDim.x)
         tw[i] = tw_g[i];
+    for (int i = threadIdx.x; i < (R - 1) * 32; i += blockDim.x)
+        tw1[i] = tw_g[(2 * (i & 31) * ((i >> 5) + 1)) & (N - 1)];
+    if (threadIdx.x < 32) {
+        const int i = threadIdx.x;
+        if (R == 8) {
+            if (i < 28)
+                tw2[i] = tw_g[((i & 3) * ((i >> 2) + 1) * (N / 32)) & (N - 1)];
+        } else if (i > 0) {
+            const int s = 1 << (31 - __clz(i));
+            tw2[i] = tw_g[(i - s) * (N / (2 * s))];
+        }
+    }
     wait_previous();
     in = fresh(in);
     st = fresh(st);
@@ -813,21 +840,21 @@ __global__ void __launch_bounds__(kZThreads)
             dft<R>(v);
 #pragma unroll
         for (int k1 = 1; k1 < R; k1++)
-            v[k1] = cmul(v[k1], tw[(2 * lane * k1) & (N - 1)]);
+            v[k1] = cmul(v[k1], tw1[(k1 - 1) * 32 + lane]);
         if constexpr (R == 8) {
             // exchange: y_l[k1] at (k1, l) -> lane 4 k1 + q takes l = q + 4 i
 #pragma unroll
             for (int k1 = 0; k1 < 8; k1++)
-                zs[zpad(k1 * 32 + lane)] = v[k1];
+                zs[k1 * kZStep<R> + lane] = v[k1];
             __syncwarp();
 #pragma unroll
             for (int i = 0; i < 8; i++)
-                v[i] = zs[zpad(k1g * 32 + qg + 4 * i)];
+                v[i] = zs[k1g * kZStep<R> + qg + 4 * i];
             __syncwarp();
             dft8(v);
 #pragma unroll
             for (int ki = 1; ki < 8; ki++)
-                v[ki] = cmul(v[ki], tw[(qg * ki * (N / 32)) & (N - 1)]);  // W_32^{q ki}
+                v[ki] = cmul(v[ki], tw2[(ki - 1) * 4 + qg]);  // W_32^{q ki}
             // 4-point DFT over q across the lanes of the group (xor 2, then xor 1)
             const float2 w2 = tw[(qg & 1) * (N / 4)];  // W_4^{q mod 2}
 #pragma unroll
@@ -838,12 +865,12 @@ __global__ void __launch_bounds__(kZThreads)
             // lane holds Z[k1 + 8 (ki + 8 bitrev2(q))]
 #pragma unroll
             for (int ki = 0; ki < 8; ki++)
-                zs[zpad(k1g + 8 * (ki + 8 * qrev))] = v[ki];
+                zs[zpad<R>(k1g + 8 * (ki + 8 * qrev))] = v[ki];
         } else {
 #pragma unroll
             for (int s = 16; s >= 1; s >>= 1) {
                 const bool upper = (lane & s) != 0;
-                const float2 w = tw[(lane & (s - 1)) * (N / (2 * s))];  // W_{2s}^{lane mod s}
+                const float2 w = tw2[s + (lane & (s - 1))];  // W_{2s}^{lane mod s}
 #pragma unroll
                 for (int k1 = 0; k1 < R; k1++)
                     v[k1] = dif_shfl(v[k1], s, upper, w);
@@ -851,7 +878,7 @@ __global__ void __launch_bounds__(kZThreads)
             // lane holds Z[k1 + R bitrev5(lane)]
 #pragma unroll
             for (int k1 = 0; k1 < R; k1++)
-                zs[zpad(k1 + R * br)] = v[k1];
+                zs[zpad<R>(k1 + R * br)] = v[k1];
         }
         __syncwarp();
         float2 *out = reinterpret_cast<float2 *>(grid + base);
@@ -861,7 +888,7 @@ __global__ void __launch_bounds__(kZThreads)
             if (k <= M) {
                 const int ka = k == M ? 0 : k;      // Z[N/2] = Z[0]
                 const int kb = k == 0 ? 0 : M - k;  // Z[(N/2 - k) mod N/2]
-                const float2 a = zs[zpad(ka)], b = zs[zpad(kb)];
+                const float2 a = zs[zpad<R>(ka)], b = zs[zpad<R>(kb)];
                 const float2 e = make_float2(a.x + b.x, a.y - b.y);
                 const float2 o = make_float2(a.x - b.x, a.y + b.y);
                 const float2 wo = cmul(tw[k], o);
@@ -925,8 +952,8 @@ __global__ void __launch_bounds__(kTThreads)
 {
     constexpr int N = 1024, M = N / 2, R = M / 32, HC = N / 2 + 1;
     extern __shared__ __align__(16) unsigned char ts[];
-    float2 *zx = reinterpret_cast<float2 *>(ts) + (threadIdx.x >> 5) * (M + M / 32);
-    float2 *tb = reinterpret_cast<float2 *>(ts) + kTRows * (M + M / 32);  // [HC][kTRows + 1]
+    float2 *zx = reinterpret_cast<float2 *>(ts) + (threadIdx.x >> 5) * kZRow<R>;
+    float2 *tb = reinterpret_cast<float2 *>(ts) + kTRows * kZRow<R>;  // [HC][kTRows + 1]
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t row0 = (int64_t)blockIdx.x * kTRows;
     const int x = (int)(row0 / N), y0 = (int)(row0 - (int64_t)x * N);
@@ -951,15 +978,15 @@ __global__ void __launch_bounds__(kTThreads)
     dft16(v);
 #pragma unroll
     for (int k1 = 1; k1 < R; k1++)
-        v[k1] = cmul(v[k1], __ldg(tw + ((2 * lane * k1) & (N - 1))));  // W_M^{l k1}
+        v[k1] = cmul(v[k1], __ldg(tw + N + (k1 - 1) * 32 + lane));  // W_M^{l k1}
 #pragma unroll
     for (int k1 = 0; k1 < R; k1++)
-        zx[zpad(k1 * 32 + lane)] = v[k1];
+        zx[k1 * kZStep<R> + lane] = v[k1];
     __syncwarp();
     const int k1g = lane >> 1, q = lane & 1;
 #pragma unroll
     for (int i = 0; i < R; i++)
-        v[i] = zx[zpad(k1g * 32 + q + 2 * i)];
+        v[i] = zx[k1g * kZStep<R> + q + 2 * i];
     __syncwarp();
     dft16(v);
     if (q) {
@@ -972,7 +999,7 @@ __global__ void __launch_bounds__(kTThreads)
         v[ki] = dif_shfl(v[ki], 1, q != 0, make_float2(1.f, 0.f));
 #pragma unroll
     for (int ki = 0; ki < R; ki++)
-        zx[zpad(k1g + 16 * (ki + 16 * q))] = v[ki];
+        zx[zpad<R>(k1g + 16 * (ki + 16 * q))] = v[ki];
     __syncwarp();
 #pragma unroll
     for (int j = 0; j <= R; j++) {
@@ -980,7 +1007,7 @@ __global__ void __launch_bounds__(kTThreads)
         if (k <= M) {
             const int ka = k == M ? 0 : k;      // Z[N/2] = Z[0]
             const int kb = k == 0 ? 0 : M - k;  // Z[(N/2 - k) mod N/2]
-            const float2 za = zx[zpad(ka)], zb = zx[zpad(kb)];
+            const float2 za = zx[zpad<R>(ka)], zb = zx[zpad<R>(kb)];
             const float2 e = make_float2(za.x + zb.x, za.y - zb.y);
             const float2 o = make_float2(za.x - zb.x, za.y + zb.y);
             const float2 wo = cmul(__ldg(tw + k), o);
@@ -1011,8 +1038,8 @@ __global__ void __launch_bounds__(kTThreads)
 {
     constexpr int N = 1024, M = N / 2, R = M / 32, HC = N / 2 + 1;
     extern __shared__ __align__(16) unsigned char ts[];
-    float2 *zx = reinterpret_cast<float2 *>(ts) + (threadIdx.x >> 5) * (M + M / 32);
-    float2 *tb = reinterpret_cast<float2 *>(ts) + kTRows * (M + M / 32);  // [HC][kTRows + 1]
+    float2 *zx = reinterpret_cast<float2 *>(ts) + (threadIdx.x >> 5) * kZRow<R>;
+    float2 *tb = reinterpret_cast<float2 *>(ts) + kTRows * kZRow<R>;  // [HC][kTRows + 1]
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t row0 = (int64_t)blockIdx.x * kTRows;
     const int x = (int)(row0 / N), y0 = (int)(row0 - (int64_t)x * N);
@@ -1058,15 +1085,15 @@ __global__ void __launch_bounds__(kTThreads)
     dft16(v);
 #pragma unroll
     for (int k1 = 1; k1 < R; k1++)
-        v[k1] = cmul(v[k1], __ldg(tw + ((2 * lane * k1) & (N - 1))));
+        v[k1] = cmul(v[k1], __ldg(tw + N + (k1 - 1) * 32 + lane));
 #pragma unroll
     for (int k1 = 0; k1 < R; k1++)
-        zx[zpad(k1 * 32 + lane)] = v[k1];
+        zx[k1 * kZStep<R> + lane] = v[k1];
     __syncwarp();
     const int k1g = lane >> 1, q = lane & 1;
 #pragma unroll
     for (int i = 0; i < R; i++)
-        v[i] = zx[zpad(k1g * 32 + q + 2 * i)];
+        v[i] = zx[k1g * kZStep<R> + q + 2 * i];
     __syncwarp();
     dft16(v);
     if (q) {
@@ -1079,13 +1106,13 @@ __global__ void __launch_bounds__(kTThreads)
         v[ki] = dif_shfl(v[ki], 1, q != 0, make_float2(1.f, 0.f));
 #pragma unroll
     for (int ki = 0; ki < R; ki++)
-        zx[zpad(k1g + 16 * (ki + 16 * q))] = make_float2(v[ki].x, -v[ki].y);  // conj: z[n]
+        zx[zpad<R>(k1g + 16 * (ki + 16 * q))] = make_float2(v[ki].x, -v[ki].y);  // conj: z[n]
     __syncwarp();
     float2 *orow = reinterpret_cast<float2 *>(out + (size_t)(row0 + wid) * (size_t)row_floats);
 #pragma unroll
     for (int j = 0; j < R; j++) {
         const int nn = lane + 32 * j;
-        orow[nn] = zx[zpad(nn)];
+        orow[nn] = zx[zpad<R>(nn)];
     }
 }
 
@@ -1258,6 +1285,16 @@ void xfft_twiddles(int dims, std::vector<float> *out)
         (*out)[2 * (size_t)m] = (float)std::cos(a);
         (*out)[2 * (size_t)m + 1] = (float)std::sin(a);
     }
+    if (dims != 1024)
+        return;
+    // W_512^{l k1} at [N + 32 (k1 - 1) + l], as the lanes of the kz-major z
+    // passes read them: in the table itself they are up to 32 lines apart.
+    for (int k1 = 1; k1 < 16; k1++)
+        for (int l = 0; l < 32; l++) {
+            const size_t m = (size_t)(2 * l * k1) % 1024;
+            out->push_back((*out)[2 * m]);
+            out->push_back((*out)[2 * m + 1]);
+        }
 }
 
 namespace {
@@ -1411,7 +1448,7 @@ cudaError_t zfft_kz_pass(const GridGeom &g, float *grid, const unsigned long lon
     if (g.dims != 1024)
         return cudaErrorNotSupported;
     constexpr int M = 512, HC = 513;
-    const size_t smem = sizeof(float2) * ((size_t)kTRows * (M + M / 32) + (size_t)HC * (kTRows + 1));
+    const size_t smem = sizeof(float2) * ((size_t)kTRows * kZRow<M / 32> + (size_t)HC * (kTRows + 1));
     cudaError_t err;
     if ((err = ensure_dynamic_smem(k_zfft_t1024, smem)) != cudaSuccess)
         return err;
@@ -1427,7 +1464,7 @@ cudaError_t zifft_kz_pass(const GridGeom &g, const float *kz_major, float *out, 
     if (g.dims != 1024)
         return cudaErrorNotSupported;
     constexpr int M = 512, HC = 513;
-    const size_t smem = sizeof(float2) * ((size_t)kTRows * (M + M / 32) + (size_t)HC * (kTRows + 1));
+    const size_t smem = sizeof(float2) * ((size_t)kTRows * kZRow<M / 32> + (size_t)HC * (kTRows + 1));
     cudaError_t err;
     if ((err = ensure_dynamic_smem(k_zifft_t1024, smem)) != cudaSuccess)
         return err;
