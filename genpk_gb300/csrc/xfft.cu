@@ -5,7 +5,7 @@
 //
 //   k_zfft    the r2c along z of one freshly deposited field, read straight
 //             from the deposit's 64-bit accumulator (one warp per row);
-//   k_yfft    the complex pass along y (cp.async tiles, Stockham stages);
+//   k_yfft    the complex pass along y (Stockham stages);
 //   k_xfft    the complex pass along x for every (j, kz) column, in place (the
 //             layout cuFFT's 3-D R2C produces).  It runs after k_zfft + k_yfft
 //             or after a batched 2-D cuFFT R2C over the x-planes (fields that
@@ -258,12 +258,36 @@ __device__ __forceinline__ void dft(float2 *v)
     }
 }
 
+// Place of (row, c) in a tile between the stages of span 1 and 8.  With rows of
+// 64 bytes (N = 512) the first stage's writes of a half-warp are two rows, 8
+// apart: their 64-byte halves of a line trade places by row bit 3 (k_xfft<512>
+// with this and the twiddles below: binning pass 0.330 -> 0.312 ms, mode
+// gradient 0.298 -> 0.279).
+template <int N>
+__device__ __forceinline__ int mid_place(int row, int c)
+{
+    constexpr int TZ = kXTileBytes / 8 / N;
+    const int e = row * TZ + c;
+    return TZ == 8 ? e ^ (row & 8) : e;
+}
+
+// The twiddles of the stage of span 8: tw[k TSTEP], tw[2 k TSTEP], tw[4 k TSTEP]
+// at k, 8 + k, 16 + k (in the table itself they lie 64 bytes and more apart).
+template <int N>
+__device__ __forceinline__ void span8_twiddles(float2 *tw8, const float2 *__restrict__ tw_g)
+{
+    if (threadIdx.x < 24) {
+        const int i = threadIdx.x;
+        tw8[i] = tw_g[(i & 7) * (N / 64) << (i >> 3)];
+    }
+}
+
 // Reads of one Stockham stage (radix R, current span NS, length N): 8 values
 // per thread (8/R butterflies), twiddled and transformed, kept in registers.
 // All strides are compile-time constants.
 template <int N, int NS, int R>
-__device__ __forceinline__ void stage_read(const float2 *tile, const float2 *tw, int c, int g,
-                                           float2 (&v)[8])
+__device__ __forceinline__ void stage_read(const float2 *tile, const float2 *tw, const float2 *tw8,
+                                           int c, int g, float2 (&v)[8])
 {
     constexpr int TZ = kXTileBytes / 8 / N;
     constexpr int PER = 8 / R;
@@ -277,7 +301,9 @@ __device__ __forceinline__ void stage_read(const float2 *tile, const float2 *tw,
         if (NS > 1) {
             if (R == 8) {
                 // three table reads, the other four by products (a few ulp)
-                const float2 w1 = tw[k * TSTEP], w2 = tw[2 * k * TSTEP], w4 = tw[4 * k * TSTEP];
+                const float2 w1 = NS == 8 ? tw8[k] : tw[k * TSTEP];
+                const float2 w2 = NS == 8 ? tw8[8 + k] : tw[2 * k * TSTEP];
+                const float2 w4 = NS == 8 ? tw8[16 + k] : tw[4 * k * TSTEP];
                 const float2 w3 = cmul(w1, w2);
                 w[1] = w1;
                 w[2] = w2;
@@ -294,7 +320,8 @@ __device__ __forceinline__ void stage_read(const float2 *tile, const float2 *tw,
         }
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            float2 x = tile[(j + r * NB) * TZ + c];
+            const int row = j + r * NB;
+            float2 x = tile[NS == 8 ? mid_place<N>(row, c) : row * TZ + c];
             if (NS > 1 && r > 0)
                 x = cmul(x, w[r]);
             v[m * R + r] = x;
@@ -320,14 +347,17 @@ __device__ __forceinline__ void stage_write(float2 *tile, int c, int g, const fl
 #pragma unroll
     for (int m = 0; m < PER; m++)
 #pragma unroll
-        for (int r = 0; r < R; r++)
-            tile[stage_out_row<N, NS, R>(g, m, r) * TZ + c] = v[m * R + r];
+        for (int r = 0; r < R; r++) {
+            const int row = stage_out_row<N, NS, R>(g, m, r);
+            tile[NS == 1 ? mid_place<N>(row, c) : row * TZ + c] = v[m * R + r];
+        }
 }
 
 template <int N, int NS>
-__device__ __forceinline__ void stage(float2 *tile, const float2 *tw, int c, int g, float2 (&v)[8])
+__device__ __forceinline__ void stage(float2 *tile, const float2 *tw, const float2 *tw8, int c, int g,
+                                      float2 (&v)[8])
 {
-    stage_read<N, NS, 8>(tile, tw, c, g, v);
+    stage_read<N, NS, 8>(tile, tw, tw8, c, g, v);
     __syncthreads();
     stage_write<N, NS, 8>(tile, c, g, v);
     __syncthreads();
@@ -343,24 +373,24 @@ struct FftPlan {
 
 // Every stage but the last written back; the last stage's values left in v.
 template <int N>
-__device__ __forceinline__ void fft_to_last(float2 *tile, const float2 *tw, int c, int g,
-                                            float2 (&v)[8])
+__device__ __forceinline__ void fft_to_last(float2 *tile, const float2 *tw, const float2 *tw8, int c,
+                                            int g, float2 (&v)[8])
 {
     using P = FftPlan<N>;
     if constexpr (P::N8 >= 1)
-        stage<N, 1>(tile, tw, c, g, v);
+        stage<N, 1>(tile, tw, tw8, c, g, v);
     if constexpr (P::N8 >= 2)
-        stage<N, 8>(tile, tw, c, g, v);
+        stage<N, 8>(tile, tw, tw8, c, g, v);
     if constexpr (P::N8 >= 3)
-        stage<N, 64>(tile, tw, c, g, v);
-    stage_read<N, P::NSL, P::RL>(tile, tw, c, g, v);
+        stage<N, 64>(tile, tw, tw8, c, g, v);
+    stage_read<N, P::NSL, P::RL>(tile, tw, tw8, c, g, v);
 }
 
 // fft_to_last with every input value passed through f(row, value) as the
 // first stage (radix 8, span 1, no twiddles) reads it.
 template <int N, typename F>
-__device__ __forceinline__ void fft_to_last_in(float2 *tile, const float2 *tw, int c, int g,
-                                               float2 (&v)[8], F f)
+__device__ __forceinline__ void fft_to_last_in(float2 *tile, const float2 *tw, const float2 *tw8,
+                                               int c, int g, float2 (&v)[8], F f)
 {
     using P = FftPlan<N>;
     static_assert(P::N8 >= 1, "the first stage is radix 8");
@@ -375,10 +405,10 @@ __device__ __forceinline__ void fft_to_last_in(float2 *tile, const float2 *tw, i
     stage_write<N, 1, 8>(tile, c, g, v);
     __syncthreads();
     if constexpr (P::N8 >= 2)
-        stage<N, 8>(tile, tw, c, g, v);
+        stage<N, 8>(tile, tw, tw8, c, g, v);
     if constexpr (P::N8 >= 3)
-        stage<N, 64>(tile, tw, c, g, v);
-    stage_read<N, P::NSL, P::RL>(tile, tw, c, g, v);
+        stage<N, 64>(tile, tw, tw8, c, g, v);
+    stage_read<N, P::NSL, P::RL>(tile, tw, tw8, c, g, v);
 }
 
 __device__ __forceinline__ int kval_x(int i, int n)
@@ -453,6 +483,7 @@ __global__ void __launch_bounds__(kXThreads, kXCtasPerSm)
     q += (BIN || GRAD) ? sizeof(uint32_t) * (p.nrbins + 1) : 0;
     float *gco = reinterpret_cast<float *>(q);                   // [nrbins] (GRAD)
     __shared__ __align__(8) unsigned long long bar[2];
+    __shared__ float2 tw8[24];
 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int c = tid % TZ, g = tid / TZ;  // FFT: column and butterfly group
@@ -460,6 +491,7 @@ __global__ void __launch_bounds__(kXThreads, kXCtasPerSm)
         tw_s[i] = p.tw[i];
         iw_s[i] = (BIN || GRAD) ? p.iw[i] : 0.f;
     }
+    span8_twiddles<N>(tw8, p.tw);
     if (BIN) {
         for (int i = tid; i < (kXThreads / 32) * p.nrbins; i += kXThreads)
             whist[i] = 0.f;
@@ -569,12 +601,12 @@ __global__ void __launch_bounds__(kXThreads, kXCtasPerSm)
                 const float s = gco[bb] * (p2 * p2);
                 return make_float2(s * x.x, -(s * x.y));
             };
-            fft_to_last_in<N>(tile, tw_s, c, g, v, scale);
+            fft_to_last_in<N>(tile, tw_s, tw8, c, g, v, scale);
 #pragma unroll
             for (int r = 0; r < 8; r++)
                 v[r].y = -v[r].y;
         } else {
-            fft_to_last<N>(tile, tw_s, c, g, v);
+            fft_to_last<N>(tile, tw_s, tw8, c, g, v);
         }
         __syncthreads();
         const ColInfo *cols = cols2 + (k & 1) * TZ;
@@ -1141,70 +1173,84 @@ __global__ void __launch_bounds__(256)
 
 // k_yfft: the length-N complex transform along y of every (x-plane, kz)
 // column, in place in the in-place r2c layout.  Tiles of N rows x TZ columns
-// (consecutive kz of one x-plane) are copied into shared memory by 8-byte
-// asynchronous copies (cp.async; the rows are (N/2+1)*8 bytes apart, which
-// tensor copies cannot address), double-buffered so the next tile streams in
-// while this one is transformed by the x pass's Stockham stages; the last
-// stage writes straight back.  Columns past kz = N/2 are zero-filled.  (A third
-// buffer for the stages to alternate between, halving the barriers, made the
-// pass slower: 100 KB of shared memory per CTA leaves the 8-byte copies, which
-// go through L1, too little of it.)
+// (consecutive kz of one x-plane; the rows are (N/2+1)*8 bytes apart, which
+// tensor copies cannot address).  A thread loads the 8 values of its first
+// radix-8 butterfly straight into registers, the next tile's while this one is
+// transformed; the stages in between alternate between two shared-memory
+// tiles, so that each ends in one barrier; the last stage writes straight back.
+// Columns past kz = N/2 are zeros.  The loads go to L2 but not into L1, and not
+// first out of L2 (__ldcs): a tile's rows are 64 bytes at N = 512, their ends
+// share sectors with the next tile's (0.39 ms).  Bound by those partial sectors
+// and by latency, two CTAs of 16 warps per SM: N = 512 0.24 ms (0.30 with
+// 8-byte asynchronous copies into a double-buffered tile and two barriers a
+// stage; 0.16 of memory time), N = 256 37 -> 33 us.
 template <int N>
 __global__ void __launch_bounds__(kXThreads, kXCtasPerSm)
     k_yfft(float2 *spec, int hc, int tiles_per_plane, int64_t ntiles,
            const float2 *__restrict__ tw_g)
 {
     constexpr int TZ = kXTileBytes / 8 / N;
+    constexpr int kTile = kXTileBytes / (int)sizeof(float2);
     using P = FftPlan<N>;
+    static_assert(P::N8 == 1 || P::N8 == 2, "one or two stages before the last");
     extern __shared__ __align__(16) unsigned char ys[];
-    float2 *tiles = reinterpret_cast<float2 *>(ys);                   // [2][N][TZ]
-    float2 *tw_s = reinterpret_cast<float2 *>(ys + 2 * kXTileBytes);  // [N]
+    float2 *tile_a = reinterpret_cast<float2 *>(ys);  // [N][TZ]
+    float2 *tile_b = tile_a + kTile;                  // [N][TZ]
+    float2 *tw_s = tile_b + kTile;                    // [N]
+    __shared__ float2 tw8[24];
     const int tid = threadIdx.x;
     const int c = tid % TZ, g = tid / TZ;
     for (int i = tid; i < N; i += kXThreads)
         tw_s[i] = tw_g[i];
+    span8_twiddles<N>(tw8, tw_g);
     wait_previous();
     spec = fresh(spec);
-    auto fetch = [&](int64_t t, float2 *dst) {
+    auto column = [&](int64_t t, bool &in) -> float2 * {
         const int64_t plane = t / tiles_per_plane;
-        const int kz0 = (int)(t - plane * tiles_per_plane) * TZ;
-        const float2 *pl = spec + (size_t)plane * (size_t)N * (size_t)hc;
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            const int e = tid + kXThreads * q;
-            const int row = e / TZ, col = e - row * TZ;
-            const int kz = kz0 + col;
-            const bool in = kz < hc;
-            cp_async8(dst + row * TZ + col, pl + (size_t)row * hc + (in ? kz : 0), in ? 8u : 0u);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        const int kz = (int)(t - plane * tiles_per_plane) * TZ + c;
+        in = kz < hc;
+        return spec + (size_t)plane * (size_t)N * (size_t)hc + kz;
     };
-    int k = 0;
+    float2 next[8];
+    auto fetch = [&](int64_t t) {
+        bool in;
+        const float2 *col = column(t, in);
+#pragma unroll
+        for (int r = 0; r < 8; r++)
+            next[r] = in ? __ldcg(col + (size_t)(g + r * (N / 8)) * hc) : make_float2(0.f, 0.f);
+    };
     if ((int64_t)blockIdx.x < ntiles)
-        fetch(blockIdx.x, tiles);
-    for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x, k++) {
-        float2 *tile = tiles + (k & 1) * (kXTileBytes / (int)sizeof(float2));
-        __syncthreads();  // every thread is done with the other buffer
-        const bool next = t + gridDim.x < ntiles;
-        if (next)
-            fetch(t + gridDim.x, tiles + ((k + 1) & 1) * (kXTileBytes / (int)sizeof(float2)));
-        if (next)
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        else
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();  // this tile's copies, from every thread, have landed
-        const int64_t plane = t / tiles_per_plane;
-        const int kz0 = (int)(t - plane * tiles_per_plane) * TZ;
-        float2 *pl = spec + (size_t)plane * (size_t)N * (size_t)hc;
+        fetch(blockIdx.x);
+    for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
         float2 v[8];
-        fft_to_last<N>(tile, tw_s, c, g, v);
-        const int kz = kz0 + c;
-        if (kz < hc) {
+#pragma unroll
+        for (int r = 0; r < 8; r++)
+            v[r] = next[r];
+        dft<8>(v);
+        // The first tile is free: its readers passed the barrier below (N8 = 2),
+        // or read it before the end of the previous tile (N8 = 1).
+        if (P::N8 == 1)
+            __syncthreads();
+        stage_write<N, 1, 8>(tile_a, c, g, v);
+        __syncthreads();
+        if (t + gridDim.x < ntiles)
+            fetch(t + gridDim.x);
+        if constexpr (P::N8 == 2) {
+            stage_read<N, 8, 8>(tile_a, tw_s, tw8, c, g, v);
+            stage_write<N, 8, 8>(tile_b, c, g, v);
+            __syncthreads();
+            stage_read<N, P::NSL, P::RL>(tile_b, tw_s, tw8, c, g, v);
+        } else {
+            stage_read<N, P::NSL, P::RL>(tile_a, tw_s, tw8, c, g, v);
+        }
+        bool in;
+        float2 *col = column(t, in);
+        if (in) {
 #pragma unroll
             for (int m = 0; m < 8 / P::RL; m++)
 #pragma unroll
                 for (int r = 0; r < P::RL; r++)
-                    pl[(size_t)stage_out_row<N, P::NSL, P::RL>(g, m, r) * hc + kz] =
+                    col[(size_t)stage_out_row<N, P::NSL, P::RL>(g, m, r) * hc] =
                         v[m * P::RL + r];
         }
     }
