@@ -131,6 +131,12 @@ struct WinBox {
     bool use;    // the box fits the window
 };
 
+// Division of i < 2^16 by d, 1 < d < 2^16: __umulhi(i, small_div(d)).
+__device__ __forceinline__ uint32_t small_div(uint32_t d)
+{
+    return 0xffffffffu / d + 1u;
+}
+
 // Block-wide periodic bounding box from the per-thread float offset ranges
 // [fmn, fmx] (offsets from ref; empty when fmn > fmx).  Two barriers.
 __device__ __forceinline__ WinBox window_box(const float fmn[3], const float fmx[3],
@@ -177,8 +183,12 @@ __device__ __forceinline__ WinBox window_box(const float fmn[3], const float fmx
             }
             vol *= ext;
         }
-        if (lane == 0)
+        if (lane == 0) {
             sh_box[6] = vol <= p.cap ? 1 : 0;
+            const uint32_t dy = (uint32_t)sh_box[5], dx = (uint32_t)sh_box[4] * dy;
+            sh_box[7] = (int)small_div(dx);
+            sh_box[8] = (int)small_div(dy);
+        }
     }
     __syncthreads();
     WinBox b;
@@ -425,6 +435,14 @@ __device__ __forceinline__ void feed_ahead(ChunkFeed &f, int *slot, DeviceStatus
     f.after = 2 * (int)gridDim.x + (int)atomicAdd(&st->next_chunk, 1u);
 }
 
+// The shortest z extent of a window whose rows are flushed one to a warp; below,
+// a row's 45 instructions of addressing are for a few lanes' cells (27 M
+// particles along a Morton curve on 512^3, windows about 10 cells deep: 880
+// instructions per 32 particles, 0.91 ms; over all cells in order 0.66 ms).  A
+// lattice's windows are as deep as the grid: in order over all cells they take
+// 0.75 ms for 0.65.  64 and 128 measure the same.
+constexpr int kFlushRows = 64;
+
 template <bool VARMASS, bool CORNER>
 __global__ void __launch_bounds__(kWinThreads, 1)
     k_window_deposit(WinParams p, DeviceStatus *st, acc_t *__restrict__ acc)
@@ -435,7 +453,7 @@ __global__ void __launch_bounds__(kWinThreads, 1)
     int *win = reinterpret_cast<int *>(win_smem + p.win_off);       // [cap]
     __shared__ __align__(8) unsigned long long bar[2];
     __shared__ int sh_mm[6][32];
-    __shared__ int sh_box[8];
+    __shared__ int sh_box[9];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nwarps = blockDim.x >> 5;
 
@@ -611,10 +629,10 @@ __global__ void __launch_bounds__(kWinThreads, 1)
         }
         __syncthreads();
 
-        // Flush and clear: one warp per window row, lanes along z (each
-        // reduction instruction then covers consecutive cells); every non-zero
-        // cell is added exactly to the pass accumulator.
-        if (box.use) {
+        // Flush and clear: every non-zero cell is added exactly to the pass
+        // accumulator.  Long z rows go one to a warp, lanes along z; the cells
+        // of short ones in order over all lanes, their place by two divisions.
+        if (box.use && box.ext[2] >= kFlushRows) {
             const int nrows = box.ext[0] * box.ext[1];
             for (int r = wid; r < nrows; r += nwarps) {
                 const int wx = r / box.ext[1];
@@ -632,6 +650,23 @@ __global__ void __launch_bounds__(kWinThreads, 1)
                         atomicAdd(arow + gz, (acc_t)(long long)v);
                     }
                 }
+            }
+        } else if (box.use) {
+            const int cells = box.ext[0] * DX;
+            const uint32_t mx = (uint32_t)sh_box[7], my = (uint32_t)sh_box[8];
+            for (int i = threadIdx.x; i < cells; i += blockDim.x) {
+                const int v = win[i];
+                if (v == 0)
+                    continue;
+                win[i] = 0;
+                const int wx = (int)__umulhi((uint32_t)i, mx);
+                const int yz = i - wx * DX;
+                const int wy = (int)__umulhi((uint32_t)yz, my);
+                const int gx = wrap_once(box.org[0] + wx, p.dims);
+                const int gy = wrap_once(box.org[1] + wy, p.dims);
+                const int gz = wrap_once(box.org[2] + (yz - wy * DY), p.dims);
+                atomicAdd(acc + (size_t)gx * (size_t)p.plane + (size_t)(gy * p.row + gz),
+                          (acc_t)(long long)v);
             }
         }
         // The next chunk's window writes come after the two barriers of its
@@ -1113,20 +1148,38 @@ __global__ void __launch_bounds__(256)
 // maps into [2^27, 2^28) units of 2^-s) and the pass mean in fixed point,
 // rounded to 24 significant bits (an empty cell then reads back exactly 0).
 // nparts = 0: uniform mass umass; else the sum of nparts partial sums.
-__global__ void k_window_prep(const double *__restrict__ mass_part, int nparts, double umass,
-                              int64_t n, double inv_cells, bool clean, double *field_mass,
-                              double *field_sub, DeviceStatus *st)
+constexpr int kPrepThreads = 256;
+
+__global__ void __launch_bounds__(kPrepThreads)
+    k_window_prep(const double *__restrict__ mass_part, int nparts, double umass, int64_t n,
+                  double inv_cells, bool clean, double *field_mass, double *field_sub,
+                  DeviceStatus *st)
 {
     wait_previous();
     mass_part = fresh(mass_part);
+    // The partial sums are added one after the other, as the sorted engine adds
+    // them; all threads fetch them (608 parts: 41 us when one thread also
+    // waited for memory).
+    __shared__ double part[1024];
     double m = 0.0;
+    for (int c0 = 0; c0 < nparts; c0 += 1024) {
+        const int cnt = min(1024, nparts - c0);
+        __syncthreads();
+        for (int c = threadIdx.x; c < cnt; c += kPrepThreads)
+            part[c] = mass_part[c0 + c];
+        __syncthreads();
+        if (threadIdx.x == 0)
+#pragma unroll 8
+            for (int c = 0; c < cnt; c++)
+                m += part[c];
+    }
+    if (threadIdx.x != 0)
+        return;
     float mref;
     if (nparts == 0) {
         m = (double)n * umass;
         mref = (float)fabs(umass);
     } else {
-        for (int c = 0; c < nparts; c++)
-            m += mass_part[c];
         mref = __uint_as_float(st->max_mass_bits);
         st->max_mass_bits = 0u;  // read: zero again for the next pass
     }
@@ -1212,7 +1265,7 @@ __global__ void __launch_bounds__(256)
     k_window_probe(WinParams p, int samples, long long *__restrict__ vol_out)
 {
     __shared__ int sh_mm[6][32];
-    __shared__ int sh_box[8];
+    __shared__ int sh_box[9];
     const int64_t c = (int64_t)blockIdx.x * p.nchunks / samples;
     const float *P = p.pos + 3 * chunk_first(p, c);
     const int cnt = (int)min((int64_t)p.chunk, p.n - chunk_first(p, c));
@@ -1391,7 +1444,7 @@ cudaError_t deposit_window_pass(const DepositGeom &g, const DepositArgs &a, int 
         mark("win_mass");
     }
     if (a.masses || p.nchunks == 0) {
-        if ((err = launch_after(k_window_prep, 1, 1, 0, stream, mass_part,
+        if ((err = launch_after(k_window_prep, 1, kPrepThreads, 0, stream, mass_part,
                                 a.masses ? mass_ctas : 0, (double)a.mass, a.n, 1.0 / n3, a.clean,
                                 a.field_mass, a.field_sub, dstat)) != cudaSuccess)
             return err;
@@ -1478,7 +1531,7 @@ cudaError_t deposit_direct_pass(const DepositGeom &g, const DepositArgs &a, doub
                                 dstat)) != cudaSuccess)
             return err;
         mark("win_mass");
-        if ((err = launch_after(k_window_prep, 1, 1, 0, stream, mass_part, mass_ctas,
+        if ((err = launch_after(k_window_prep, 1, kPrepThreads, 0, stream, mass_part, mass_ctas,
                                 (double)a.mass, a.n, e.inv_cells, a.clean, a.field_mass,
                                 a.field_sub, dstat)) != cudaSuccess)
             return err;

@@ -43,8 +43,8 @@ constexpr double kWindowMaxCellsPerParticle = 64.0;
 // windows would merge few adds.  Measured (Zel'dovich lattices, merge rate:
 // stream and window ms): 512^3 on 512^3 0.94: 1.10 and 1.81; 384^3 0.65: 0.85 and
 // 0.93; 352^3 0.53: 0.77 and 0.92; 180^3 on 256^3 0.55: 0.13 and 0.19; 256^3 on
-// 512^3 0.02: 0.57 and 0.50.  Below one half the windows merge as much as the
-// lanes (512^3 particles along a Morton curve: 2.32 and 2.22).
+// 512^3 0.02: 0.57 and 0.50.  Below one half the windows merge more than the
+// lanes (512^3 particles along a Morton curve: 2.32 and 1.67).
 constexpr double kStreamMergeRate = 0.52;
 
 struct Pending {
