@@ -149,7 +149,23 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// The coefficients by value, as a kernel parameter, into device memory: a copy
+// of a few hundred bytes from pageable memory takes the host longer than the
+// launch, and the stream waits for it.
+struct CoefParam {
+    float g[kMaxCoefParam];
+};
+
+__global__ void k_set_coef(const __grid_constant__ CoefParam c, int n, float *gcoef)
+{
+    wait_previous();  // (an earlier call's kernels may still read the last ones)
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        gcoef[i] = c.g[i];
+}
+
 struct GatherParams {
+    const DeviceStatus *st_in;  // the call's status words, which the gather's
+    DeviceStatus *st_out;       // first thread puts into mapped host memory
     int dims;
     int64_t plane;
     int row;
@@ -298,6 +314,12 @@ __device__ __forceinline__ GatherOut gather_one(const GatherParams &p, const flo
     return gather_tree(p, g, d, m);
 }
 
+__device__ __forceinline__ void put_status(const GatherParams &p)
+{
+    if (p.st_out && blockIdx.x == 0 && threadIdx.x == 0)
+        *p.st_out = *fresh(p.st_in);
+}
+
 // One particle per thread, grid-stride.  (Tiles of 1024 particles staged
 // through shared memory with 16-byte loads and stores, four particles per
 // thread, ran slower: 1.20 ms against 0.93 at 512^3, with fewer warps resident
@@ -309,6 +331,7 @@ __global__ void __launch_bounds__(256)
 {
     wait_previous();
     grid = fresh(grid);
+    put_status(p);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const float x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
@@ -368,6 +391,7 @@ __global__ void __launch_bounds__(256)
 {
     wait_previous();
     grid = fresh(grid);
+    put_status(p);
     const int64_t groups = p.n >> 2;
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (int64_t q = tid; q < groups; q += (int64_t)gridDim.x * blockDim.x) {
@@ -406,6 +430,18 @@ bool aligned16(const void *ptr)
 }
 
 }  // namespace
+
+cudaError_t adjoint_set_coef(const float *coef, int n, float *gcoef_dev, cudaStream_t stream,
+                             int64_t *launches)
+{
+    if (n > kMaxCoefParam)
+        return cudaMemcpyAsync(gcoef_dev, coef, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice,
+                               stream);
+    CoefParam c{};
+    std::copy(coef, coef + n, c.g);
+    (*launches)++;
+    return launch_after(k_set_coef, 1, 256, 0, stream, c, n, gcoef_dev);
+}
 
 cudaError_t adjoint_mode_gradient_kz(const GridGeom &g, const BinTables &t, const BinDevice &d,
                                      float2 *spec, const float *gcoef_dev, int num_sms,
@@ -446,11 +482,14 @@ cudaError_t adjoint_mode_gradient_coef(const GridGeom &g, const BinTables &t, co
 cudaError_t adjoint_gather(const GridGeom &g, float units_hi, float units_lo, const float *grid,
                            const float *pos, const float *masses, float mass, int64_t n,
                            float *grad_pos, float *grad_mass, float dl_dmass_norm, bool coherent,
-                           cudaStream_t stream, int64_t *launches)
+                           const DeviceStatus *st_in, DeviceStatus *st_out, cudaStream_t stream,
+                           int64_t *launches)
 {
     if (n <= 0)
         return cudaSuccess;
     GatherParams p;
+    p.st_in = st_in;
+    p.st_out = st_out;
     p.dims = g.dims;
     p.plane = g.plane;
     p.row = g.row;

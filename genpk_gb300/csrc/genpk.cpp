@@ -2243,8 +2243,7 @@ int genpk_adjoint(genpk_ctx *ctx, int field, double boxsize, const float *pos, c
     }
     if (dl_dmass_norm)
         *dl_dmass_norm = dldm;
-    GENPK_CUDA(cudaMemcpyAsync(ctx->d_gcoef, gcoef.data(), sizeof(float) * nrb,
-                               cudaMemcpyHostToDevice, ctx->stream));
+    GENPK_CUDA(adjoint_set_coef(gcoef.data(), nrb, ctx->d_gcoef, ctx->stream, &ctx->launches));
     float *g = grid_of(ctx, field);
     if (kz) {
         // mode gradient in place, the inverse (x, y) transform per kz plane,
@@ -2292,9 +2291,16 @@ int genpk_adjoint(genpk_ctx *ctx, int field, double boxsize, const float *pos, c
     if (!kz)
         stage_event(ctx, "adj_c2r");
     const DepositGeom dg = deposit_geom(ctx, boxsize);
+    // The gather's status words come back in the results' mapped host memory (a
+    // batch request's results may still be in there).
+    DeviceStatus *st_out = nullptr;
+    if (n > 0 && !ctx->deferred.active) {
+        GENPK_TRY(grow_res(ctx, kStatusDoubles));
+        st_out = reinterpret_cast<DeviceStatus *>(ctx->res_dev);
+    }
     GENPK_CUDA(adjoint_gather(ctx->gg, dg.units_hi, dg.units_lo, g, dpos, dmass, (float)mass, n,
                               dgpos, dgmass, (float)dldm, ctx->last_engine == GENPK_ENGINE_STREAM,
-                              ctx->stream, &ctx->launches));
+                              ctx->d_status, st_out, ctx->stream, &ctx->launches));
     stage_event(ctx, "adj_gather");
     if (!dev) {
         GENPK_CUDA(cudaMemcpyAsync(grad_pos, dgpos, sizeof(float) * 3 * (size_t)n,
@@ -2303,8 +2309,10 @@ int genpk_adjoint(genpk_ctx *ctx, int field, double boxsize, const float *pos, c
             GENPK_CUDA(cudaMemcpyAsync(grad_mass, dgmass, sizeof(float) * (size_t)n,
                                        cudaMemcpyDeviceToHost, ctx->stream));
     }
+    if (!st_out)
+        return collect_status(ctx);
     GENPK_CUDA(cudaStreamSynchronize(ctx->stream));
-    return collect_status(ctx);
+    return report_status(ctx, *reinterpret_cast<const DeviceStatus *>(ctx->res_host));
 }
 
 int genpk_timing_reset(genpk_ctx *ctx)

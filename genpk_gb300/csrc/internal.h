@@ -400,6 +400,12 @@ cudaError_t bin_spectra(const GridGeom &g, const BinTables &t, const BinDevice &
 // ---------------------------------------------------------------------------
 // Adjoint
 // ---------------------------------------------------------------------------
+// The per-bin coefficients into device memory (up to kMaxCoefParam as a kernel
+// parameter, more by a copy).
+constexpr int kMaxCoefParam = 512;
+cudaError_t adjoint_set_coef(const float *coef, int n, float *gcoef_dev, cudaStream_t stream,
+                             int64_t *launches);
+
 // Replace the spectrum F in `spec` (in place) by the c2r input H of the
 // density gradient for the auto spectrum: H_m = G_b V_m (c_m / mult_m) F_m with
 // gcoef_dev[b] = G_b = 2 g_b / (M^2 C_b) (device, nrbins floats).
@@ -422,7 +428,8 @@ cudaError_t zifft_kz_pass(const GridGeom &g, const float *kz_major, float *out, 
 cudaError_t adjoint_gather(const GridGeom &g, float units_hi, float units_lo, const float *grid,
                            const float *pos, const float *masses, float mass, int64_t n,
                            float *grad_pos, float *grad_mass, float dl_dmass_norm, bool coherent,
-                           cudaStream_t stream, int64_t *launches);
+                           const DeviceStatus *st_in, DeviceStatus *st_out, cudaStream_t stream,
+                           int64_t *launches);
 
 int device_sm_count();
 

@@ -72,3 +72,22 @@ def test_gather_kernels_agree(dims, order, masses):
     assert (ga[~np.isfinite(pos).all(axis=1)] == 0).all()
     if masses:
         np.testing.assert_array_equal(ma.view(np.uint32), mb.view(np.uint32))
+
+
+@pytest.mark.parametrize("nrbins", [1, 512, 513])
+def test_coefficients_by_value_and_by_copy(nrbins):
+    """Up to 512 per-bin coefficients go up as a kernel parameter, more by a
+    copy; both give the oracle's gradient within the adjoint tests' 1e-4."""
+    from genpk_gb300 import api, synth
+    from oracle import oracle as O
+
+    dims, box = 36, 1000.0
+    pos = synth.zeldovich(dims, box, seed=21)
+    m = O.total_mass(len(pos), None, 1.0)
+    with api.Context(dims, nrbins) as ctx:
+        ctx.deposit(0, box, pos, None, 1.0)
+        p, c, _ = ctx.power(0, 0, m, m)
+        g = np.where(c > 0, 1.0 + np.cos(np.arange(nrbins)), 0.0)
+        gpos, _, _ = ctx.adjoint(0, box, pos, g, m, mass=1.0)
+    ref, _, _ = O.reference_gradient(pos, box, dims, nrbins, g, None, 1.0, m_norm=m)
+    assert np.abs(gpos - ref).max() <= 1e-4 * np.abs(ref).max()
