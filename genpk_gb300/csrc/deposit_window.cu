@@ -377,14 +377,41 @@ __device__ __forceinline__ void corner_add_chunk(CornerSum &c, f2sum v)
     c.lo += __float_as_int(fmaf(__fadd_rn(r, v.lo), 1099511627776.f, 12582912.f)) - kMagicBits;
 }
 
-// Block epilogue of the stream mode: the warps' corner sums and the
-// invalid-particle and wait-timeout counts.
+// Block epilogue of the stream mode and the direct passes: the corner sum and
+// the invalid-particle and wait-timeout counts, one atomic each per block.  (One
+// each per warp, all to the same words, took longer than the adds: a direct pass
+// of 1.2 M particles on 512^3 0.35 ms, 0.29 with masses.)  Returns the block's
+// invalid particles to thread 0.
 template <bool CORNER>
-__device__ __forceinline__ void report_stream_block(DeviceStatus *st, CornerSum c, unsigned bad,
-                                             unsigned timeouts)
+__device__ __forceinline__ unsigned report_stream_block(DeviceStatus *st, CornerSum c, unsigned bad,
+                                                        unsigned timeouts)
 {
-    const int lane = threadIdx.x & 31;
+    __shared__ CornerSum part[32];
+    __shared__ unsigned counts[2];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (threadIdx.x < 2)
+        counts[threadIdx.x] = 0u;
+    __syncthreads();
     if (CORNER) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            c.hi += __shfl_xor_sync(0xffffffffu, c.hi, o);
+            c.lo += __shfl_xor_sync(0xffffffffu, c.lo, o);
+        }
+        if (lane == 0)
+            part[wid] = c;
+    }
+    bad = __reduce_add_sync(0xffffffffu, bad);
+    timeouts = __reduce_add_sync(0xffffffffu, timeouts);
+    if (lane == 0 && bad)
+        atomicAdd(&counts[0], bad);
+    if (lane == 0 && timeouts)
+        atomicAdd(&counts[1], timeouts);
+    __syncthreads();
+    if (wid != 0)
+        return 0u;
+    if (CORNER) {
+        c = lane < nw ? part[lane] : CornerSum{0, 0};
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             c.hi += __shfl_xor_sync(0xffffffffu, c.hi, o);
@@ -395,12 +422,11 @@ __device__ __forceinline__ void report_stream_block(DeviceStatus *st, CornerSum 
             atomicAdd((unsigned long long *)&st->alt_lo, (unsigned long long)c.lo);
         }
     }
-    bad = __reduce_add_sync(0xffffffffu, bad);
-    timeouts = __reduce_add_sync(0xffffffffu, timeouts);
-    if (lane == 0 && bad)
-        atomicAdd(&st->bad_particles, (unsigned long long)bad);
-    if (lane == 0 && timeouts)
-        atomicAdd(&st->timeouts, (unsigned long long)timeouts);
+    if (lane == 0 && counts[0])
+        atomicAdd(&st->bad_particles, (unsigned long long)counts[0]);
+    if (lane == 0 && counts[1])
+        atomicAdd(&st->timeouts, (unsigned long long)counts[1]);
+    return lane == 0 ? counts[0] : 0u;
 }
 
 // The stream mode hands out its chunks in order: a CTA's first two are fixed, the others come
@@ -884,8 +910,11 @@ __global__ void __launch_bounds__(kWinThreads, 1)
 // shuffle per (x, y) corner) and both add the lower- and upper-z weight of one
 // particle, then of the other: the two lie in one sector three times out of
 // four.  1 M particles on 128^3: 68 -> 47 us (the stream kernel without its
-// merges); 40 k on 64^3, where the pass is latency: 5 us against 24 for the
-// binned sort's three kernels.
+// merges), 33 since a block reports its sums once; 40 k on 64^3, where the pass
+// is latency: 5 us against 24 for the binned sort's three kernels.  On grids past
+// the L2 DRAM bounds it, at a line read and written per sector: 2 M on 512^3
+// 0.33 ms.  Eight CTAs per SM: 4 and 16 take 0.35 and 0.34 there, 67 and 82 us for
+// 600 k on 256^3 (8: 72).
 constexpr int kDirectThreads = 256;
 
 template <bool VARMASS, bool CORNER, bool WIDE>
@@ -988,10 +1017,9 @@ __global__ void __launch_bounds__(kDirectThreads)
         const float r = fmaf(-__ll2float_rn(c.hi), 1.f / 262144.f, alt.hi);  // exact
         c.lo = __float2ll_rn(__fadd_rn(r, alt.lo) * 1099511627776.f);
     }
-    const unsigned skipped = __reduce_add_sync(0xffffffffu, bad);
-    if (lane == 0 && skipped)
+    const unsigned skipped = report_stream_block<CORNER>(st, c, bad, 0u);
+    if (skipped)
         atomicAdd(&st->pass_bad, (unsigned long long)skipped);
-    report_stream_block<CORNER>(st, c, bad, 0u);
 }
 
 // What ends a direct pass.  A uniform mass's constants come from the host for
@@ -1553,7 +1581,7 @@ cudaError_t deposit_direct_pass(const DepositGeom &g, const DepositArgs &a, doub
                                      : (wide ? k_direct_deposit<false, false, true>
                                              : k_direct_deposit<false, false, false>));
     const unsigned ctas = (unsigned)std::max<int64_t>(
-        1, std::min<int64_t>((a.n + kDirectThreads - 1) / kDirectThreads, (int64_t)num_sms * 16));
+        1, std::min<int64_t>((a.n + kDirectThreads - 1) / kDirectThreads, (int64_t)num_sms * 8));
     if ((err = launch_after(kern, ctas, kDirectThreads, 0, stream, p, dstat, acc)) != cudaSuccess)
         return err;
     mark("direct_deposit");

@@ -101,6 +101,7 @@ struct genpk_ctx {
         int band = 0;
         bool var = false;
         bool with_stream = false;         // the stream engine was among the trials
+        bool own = false;                 // the pass was headed for the own transform passes
         int engine = GENPK_ENGINE_SORTED;  // the faster: SORTED (with this tile) or STREAM
         TileShape tile{16, 16, 16};
     };
@@ -513,7 +514,7 @@ constexpr int kTuneReps = 2;
 // counters are put back before the next.  The chosen candidate then runs as
 // the real pass.
 int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, bool with_stream,
-                const genpk_ctx::Tuned **out)
+                bool own, const genpk_ctx::Tuned **out)
 {
     static const TileShape tiles[] = {{8, 8, 8}, {16, 16, 8}, {16, 16, 16}};
     const size_t stash = 0;  // the error counters are kept in the probe buffer meanwhile
@@ -534,6 +535,7 @@ int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, boo
     best.band = density_band(ctx, a.n);
     best.var = a.masses != nullptr;
     best.with_stream = with_stream;
+    best.own = own;
     float best_ms = 1e30f;
     ctx->ntrials = 0;
     if (with_stream && !ctx->dscr.win_acc) {
@@ -553,11 +555,16 @@ int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, boo
         float ms = 1e30f;
         const bool zero0 = ctx->acc_zero, spent0 = ctx->acc_spent;
         const size_t dirty0 = ctx->acc_dirty_bytes;
+        // Headed for the own transform passes a direct pass leaves its conversion
+        // to the z pass; a clear of the whole accumulator stands for what the
+        // transform then does more (it reads 8 bytes a cell for 4 and clears
+        // them).  With the conversion counted, 1.2 to 4 M particles on 512^3 took
+        // the sorted engine, 1.50 ms a spectrum and more, for 1.09 to 1.24.
         for (int rep = 0; rep < kTuneReps; rep++) {
-            const size_t clear = acc_clear_bytes(ctx);
+            const size_t clear = own ? acc_bytes(ctx) : acc_clear_bytes(ctx);
             GENPK_CUDA(cudaEventRecord(e0, ctx->stream));
             GENPK_CUDA(deposit_direct_pass(g, a, ctx->dscr.mass_part, mass_ctas,
-                                           ctx->dscr.win_acc, clear, false, ctx->num_sms,
+                                           ctx->dscr.win_acc, clear, own, ctx->num_sms,
                                            ctx->d_status, ctx->stream, &ctx->launches, nullptr,
                                            nullptr));
             ctx->acc_zero = true;
@@ -567,6 +574,8 @@ int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, boo
             GENPK_CUDA(cudaEventElapsedTime(&t, e0, e1));
             ms = std::min(ms, t);
         }
+        if (own)
+            GENPK_CUDA(cudaMemsetAsync(ctx->dscr.win_acc, 0, acc_bytes(ctx), ctx->stream));
         // The trials leave the accumulator zero; it is recorded as it was before
         // them, so that a call that tunes ends in the state of one that does not
         // (the graphs compare them).
@@ -618,13 +627,14 @@ int tune_sorted(genpk_ctx *ctx, int f, double boxsize, const DepositArgs &a, boo
     return GENPK_OK;
 }
 
-const genpk_ctx::Tuned *find_tuned(const genpk_ctx *ctx, int64_t n, bool var, bool with_stream)
+const genpk_ctx::Tuned *find_tuned(const genpk_ctx *ctx, int64_t n, bool var, bool with_stream,
+                                   bool own)
 {
     const int band = density_band(ctx, n);
     const int have = std::min(ctx->ntuned, genpk_ctx::kTuned);
     for (int i = 0; i < have; i++)
         if (ctx->tuned[i].band == band && ctx->tuned[i].var == var &&
-            ctx->tuned[i].with_stream == with_stream)
+            ctx->tuned[i].with_stream == with_stream && ctx->tuned[i].own == own)
             return &ctx->tuned[i];
     return nullptr;
 }
@@ -639,15 +649,30 @@ const genpk_ctx::Tuned *find_tuned(const genpk_ctx *ctx, int64_t n, bool var, bo
 // 0.069 and 0.079 at 2^20 particles on 128^3, 0.111 and 0.097 at 2^21; 0.131 and
 // 0.141 at 2^19 on 256^3, 0.175 and 0.155 at 2^20; 0.67 and 0.83 at 2^20 on
 // 512^3, 0.88 and 0.86 at 2^21.
-int64_t own_transform_limit(int64_t dims)
+// Particles with masses on 512^3 are stars in the order of a snapshot's cells:
+// direct adds find neighbours in the L2 and are the faster up to where windows
+// hold them (with the own passes 1.09 ms at 1.2 M and 1.24 at 4 M, sorted with
+// cuFFT 1.53 and 1.64; from 5 M on they are windows).
+int64_t own_transform_limit(int64_t dims, bool masses)
 {
-    return dims <= 128 ? (int64_t)3 << 19 : dims <= 256 ? (int64_t)3 << 18 : (int64_t)1 << 21;
+    return dims <= 128   ? (int64_t)3 << 19
+           : dims <= 256 ? (int64_t)3 << 18
+           : masses      ? (int64_t)3 << 21
+                         : (int64_t)1 << 21;
+}
+
+bool use_xfft(const genpk_ctx *ctx);
+
+// A clean pass without order is headed for the own transform passes.
+bool unordered_own(const genpk_ctx *ctx, const DepositArgs &a)
+{
+    return use_xfft(ctx) && a.clean && a.n >= kTuneMinParticles &&
+           a.n < own_transform_limit(ctx->dims, a.masses != nullptr);
 }
 
 // One deposit pass from device particle arrays, or (host_mapped) from pinned
 // host arrays read in place by the window engine.
 int flush_acc(genpk_ctx *ctx);
-bool use_xfft(const genpk_ctx *ctx);
 bool use_kz(const genpk_ctx *ctx);
 
 int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const float *masses,
@@ -742,9 +767,10 @@ int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const f
                              !ctx->tile_fixed && !host_mapped;
     const bool no_order = auto_sorted || (reuse && hit->no_order);
     if (auto_sorted || (engine == GENPK_ENGINE_SORTED && !ctx->tile_fixed && !host_mapped)) {
-        tuned = find_tuned(ctx, n, masses != nullptr, auto_sorted);
+        const bool own = no_order && unordered_own(ctx, a);
+        tuned = find_tuned(ctx, n, masses != nullptr, auto_sorted, own);
         if (!tuned && a.clean && n >= kTuneMinParticles) {
-            GENPK_TRY(tune_sorted(ctx, f, boxsize, a, auto_sorted, &tuned));
+            GENPK_TRY(tune_sorted(ctx, f, boxsize, a, auto_sorted, own, &tuned));
             stage_event(ctx, "tune");
         }
         if (tuned && tuned->engine == GENPK_ENGINE_STREAM)
@@ -823,7 +849,7 @@ int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const f
     // pass in the accumulator: the z pass converts it on the fly.
     bool own = a.clean && chunked && (use_xfft(ctx) || use_kz(ctx));
     if (no_order && use_xfft(ctx))
-        own = a.clean && n >= kTuneMinParticles && n < own_transform_limit(ctx->dims);
+        own = unordered_own(ctx, a);
     if (chunked || direct) {
         const int mass_ctas = ctx->num_sms * 4;
         size_t mp = (size_t)s.mass_part_cap;
