@@ -170,8 +170,12 @@ __device__ __forceinline__ void stage_piece(const BinParams &p, int64_t r, int p
 // piece (RP odd: conflict-free strided shared reads) with a running FP32 sum
 // per spectrum pair.  Along a run |k|^2 grows, so the bin only moves up: the
 // next threshold is kept in a register and a completed bin inside a run is
-// added to the warp's FP32 histogram with a shared atomic (rare: only where
-// bins are narrower than a run).  At the end of a piece the lanes' open sums
+// added to the warp's FP32 histogram.  Two lanes never complete the same bin at
+// the same place of their runs (by then the upper lane has been past it for
+// RP - 1 >= 2 modes), so with the lanes in step the adds are plain ones; an FP32
+// shared atomic is a loop, and six pairs' loops at nearly every mode of a row
+// were half of its instructions (three fields, six pairs on 512^3: 0.52 -> 0.42
+// ms).  One pair's single atomic costs less than keeping the lanes in step.  At the end of a piece the lanes' open sums
 // are combined by a segmented warp scan over their (non-decreasing) bins and
 // each bin's last lane adds the total without atomics.  Every kPromoteRows
 // rows the touched FP32 bins are promoted into the warp's FP64 histogram.
@@ -193,6 +197,7 @@ __global__ void __launch_bounds__(256, NF == 1 ? 4 : 2)
     extern __shared__ __align__(16) unsigned char smem[];
     const int nrb = p.nrbins;
     constexpr int piece = 32 * RP;
+    constexpr bool kPlain = NP > 1;
     const BinLayout L = bin_layout(nrb, p.hc, NP, NF, RP);
     uint32_t *thr = (uint32_t *)smem;
     float2 *izc = (float2 *)(smem + L.izc);
@@ -247,42 +252,60 @@ __global__ void __launch_bounds__(256, NF == 1 ? 4 : 2)
 #pragma unroll
             for (int s = 0; s < NP; s++)
                 acc[s] = 0.f;
-            if (kz0 < p.hc) {
-                uint32_t kk2 = r2 + (uint32_t)(kz0 * kz0);
+            uint32_t kk2 = r2 + (uint32_t)(kz0 * kz0), nx = 0;
+            const int lim = min(RP, p.hc - kz0);  // <= 0: none
+            const float2 *bl = buf + lane * RP;
+            auto bin_mode = [&](int t) {
+                if (kk2 >= nx) {
+#pragma unroll
+                    for (int s = 0; s < NP; s++) {
+                        if (kPlain)
+                            rhist[s * nrb + cb] += acc[s];
+                        else
+                            atomicAdd(&rhist[s * nrb + cb], acc[s]);
+                        acc[s] = 0.f;
+                    }
+                    do {
+                        cb++;
+                        nx = thr[cb + 1];
+                    } while (kk2 >= nx);
+                }
+                const int kz = kz0 + t;
+                const float2 ic = izc[kz];
+                const float pz = pxy * ic.x;
+                const float p2 = pz * pz;
+                const float w = ic.y * (p2 * p2);
+                float2 fv[NF];
+#pragma unroll
+                for (int f = 0; f < NF; f++)
+                    fv[f] = bl[f * piece + t];
+                add_pairs<NF, CROSS1>(fv, w, acc);
+                kk2 += (uint32_t)(2 * kz + 1);
+            };
+            if (lim > 0) {
                 cb = bin_lookup(kk2, thr, nrb, p.bpu_half);
                 bmin = min(bmin, cb);
-                uint32_t nx = thr[cb + 1];
-                const int lim = min(RP, p.hc - kz0);
-                const float2 *bl = buf + lane * RP;
+                nx = thr[cb + 1];
+                if (!kPlain) {
+#pragma unroll
+                    for (int t = 0; t < RP; t++) {
+                        if (t >= lim)
+                            break;
+                        bin_mode(t);
+                    }
+                }
+            }
+            if (kPlain) {
 #pragma unroll
                 for (int t = 0; t < RP; t++) {
-                    if (t >= lim)
-                        break;
-                    const int kz = kz0 + t;
-                    if (kk2 >= nx) {
-#pragma unroll
-                        for (int s = 0; s < NP; s++) {
-                            atomicAdd(&rhist[s * nrb + cb], acc[s]);
-                            acc[s] = 0.f;
-                        }
-                        do {
-                            cb++;
-                            nx = thr[cb + 1];
-                        } while (kk2 >= nx);
-                    }
-                    const float2 ic = izc[kz];
-                    const float pz = pxy * ic.x;
-                    const float p2 = pz * pz;
-                    const float w = ic.y * (p2 * p2);
-                    float2 fv[NF];
-#pragma unroll
-                    for (int f = 0; f < NF; f++)
-                        fv[f] = bl[f * piece + t];
-                    add_pairs<NF, CROSS1>(fv, w, acc);
-                    kk2 += (uint32_t)(2 * kz + 1);
+                    if (t < lim)
+                        bin_mode(t);
+                    if (t > 0)
+                        __syncwarp();
                 }
-                bmax = max(bmax, cb);
             }
+            if (lim > 0)
+                bmax = max(bmax, cb);
             // Segmented inclusive scan over lanes with equal open bin.
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
