@@ -947,10 +947,15 @@ __global__ void __launch_bounds__(kZThreads)
 //      gives lanes 2 k1 and 2 k1 + 1 the values l = q + 2 i (i < 16), a
 //      16-point DFT over i, twiddles W_32^{q ki}, then a 2-point DFT across
 //      the lane pair, so that lane (k1, q) holds Z[k1 + 16 (ki + 16 q)];
-//   4. X[k] = E[k] + W_N^k O[k], k = 0..M, into a [kz][row] shared buffer;
+//   4. X[k] = E[k] + W_N^k O[k], k = 0..M, into a [kz][row] shared buffer (over
+//      the exchanges, when every warp is done with its own);
 //   5. the CTA's rows leave as runs of kTRows consecutive y per kz.
+// Each CTA loads, computes and stores in turn, so two have to share an SM: 70 KB
+// of shared memory (139 with a buffer of its own) and 64 registers (a row is
+// loaded in two halves).  1024^3: 3.39 ms with one CTA per SM, 2.17 now, 1.94 of
+// memory time.
 // The accumulator is left as it is: the kz-major binning pass clears it.
-constexpr int kTRows = 16;  // rows per CTA: 128-byte runs per kz plane (8: 3.54 -> 3.41 ms)
+constexpr int kTRows = 16;  // rows per CTA: 128-byte runs per kz plane (8 rows: 2.24 ms)
 constexpr int kTThreads = kTRows * 32;
 
 // Forward 16-point DFT in registers (two 8-point DFTs and W_16 twiddles).
@@ -978,14 +983,14 @@ __device__ __forceinline__ void dft16(float2 *v)
     }
 }
 
-__global__ void __launch_bounds__(kTThreads)
+__global__ void __launch_bounds__(kTThreads, 2)
     k_zfft_t1024(const unsigned long long *__restrict__ acc, float2 *__restrict__ spec, int row_floats,
                  const float2 *__restrict__ tw, const DeviceStatus *__restrict__ st)
 {
     constexpr int N = 1024, M = N / 2, R = M / 32, HC = N / 2 + 1;
     extern __shared__ __align__(16) unsigned char ts[];
     float2 *zx = reinterpret_cast<float2 *>(ts) + (threadIdx.x >> 5) * kZRow<R>;
-    float2 *tb = reinterpret_cast<float2 *>(ts) + kTRows * kZRow<R>;  // [HC][kTRows + 1]
+    float2 *tb = reinterpret_cast<float2 *>(ts);  // [HC][kTRows + 1], over the rows' exchanges
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t row0 = (int64_t)blockIdx.x * kTRows;
     const int x = (int)(row0 / N), y0 = (int)(row0 - (int64_t)x * N);
@@ -997,15 +1002,18 @@ __global__ void __launch_bounds__(kTThreads)
 
     const longlong2 *src =
         reinterpret_cast<const longlong2 *>(acc + (size_t)(row0 + wid) * (size_t)row_floats);
-    longlong2 a[R];
-#pragma unroll
-    for (int m = 0; m < R; m++)
-        a[m] = src[lane + 32 * m];
     float2 v[R];
 #pragma unroll
-    for (int m = 0; m < R; m++)
-        v[m] = make_float2(i64_to_f32_rn(a[m].x - mean) * inv_scale,
-                           i64_to_f32_rn(a[m].y - mean) * inv_scale);
+    for (int h = 0; h < 2; h++) {  // (in halves: a row is 64 registers)
+        longlong2 a[R / 2];
+#pragma unroll
+        for (int m = 0; m < R / 2; m++)
+            a[m] = src[lane + 32 * (m + h * (R / 2))];
+#pragma unroll
+        for (int m = 0; m < R / 2; m++)
+            v[m + h * (R / 2)] = make_float2(i64_to_f32_rn(a[m].x - mean) * inv_scale,
+                                             i64_to_f32_rn(a[m].y - mean) * inv_scale);
+    }
 
     dft16(v);
 #pragma unroll
@@ -1033,6 +1041,7 @@ __global__ void __launch_bounds__(kTThreads)
     for (int ki = 0; ki < R; ki++)
         zx[zpad<R>(k1g + 16 * (ki + 16 * q))] = v[ki];
     __syncwarp();
+    float2 out[R + 1];
 #pragma unroll
     for (int j = 0; j <= R; j++) {
         const int k = lane + 32 * j;
@@ -1043,8 +1052,15 @@ __global__ void __launch_bounds__(kTThreads)
             const float2 e = make_float2(za.x + zb.x, za.y - zb.y);
             const float2 o = make_float2(za.x - zb.x, za.y + zb.y);
             const float2 wo = cmul(__ldg(tw + k), o);
-            tb[k * (kTRows + 1) + wid] = make_float2(0.5f * (e.x + wo.y), 0.5f * (e.y - wo.x));
+            out[j] = make_float2(0.5f * (e.x + wo.y), 0.5f * (e.y - wo.x));
         }
+    }
+    __syncthreads();  // the exchanges are done with
+#pragma unroll
+    for (int j = 0; j <= R; j++) {
+        const int k = lane + 32 * j;
+        if (k <= M)
+            tb[k * (kTRows + 1) + wid] = out[j];
     }
     __syncthreads();
     for (int e = threadIdx.x; e < HC * kTRows; e += kTThreads) {
@@ -1064,14 +1080,14 @@ __global__ void __launch_bounds__(kTThreads)
 // unnormalised inverse M-point DFT of Z, as conj(DFT(conj Z)) with the
 // forward pass's structure, gives x[2n] + i x[2n+1] = z[n]: the real row,
 // written to `out` in the padded row layout (row_floats floats per row).
-__global__ void __launch_bounds__(kTThreads)
+__global__ void __launch_bounds__(kTThreads, 2)
     k_zifft_t1024(const float2 *__restrict__ spec, float *__restrict__ out, int row_floats,
                   const float2 *__restrict__ tw)
 {
     constexpr int N = 1024, M = N / 2, R = M / 32, HC = N / 2 + 1;
     extern __shared__ __align__(16) unsigned char ts[];
     float2 *zx = reinterpret_cast<float2 *>(ts) + (threadIdx.x >> 5) * kZRow<R>;
-    float2 *tb = reinterpret_cast<float2 *>(ts) + kTRows * kZRow<R>;  // [HC][kTRows + 1]
+    float2 *tb = reinterpret_cast<float2 *>(ts);  // [HC][kTRows + 1], under the rows' exchanges
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t row0 = (int64_t)blockIdx.x * kTRows;
     const int x = (int)(row0 / N), y0 = (int)(row0 - (int64_t)x * N);
@@ -1114,6 +1130,7 @@ __global__ void __launch_bounds__(kTThreads)
         const float2 wd = cmul(make_float2(w.x, -w.y), d);   // W_N^{-k} d
         v[m] = make_float2(s.x - wd.y, -(s.y + wd.x));       // conj(s + i wd)
     }
+    __syncthreads();  // tb has been read
     dft16(v);
 #pragma unroll
     for (int k1 = 1; k1 < R; k1++)
@@ -1494,7 +1511,8 @@ cudaError_t zfft_kz_pass(const GridGeom &g, float *grid, const unsigned long lon
     if (g.dims != 1024)
         return cudaErrorNotSupported;
     constexpr int M = 512, HC = 513;
-    const size_t smem = sizeof(float2) * ((size_t)kTRows * kZRow<M / 32> + (size_t)HC * (kTRows + 1));
+    const size_t smem =
+        sizeof(float2) * std::max((size_t)kTRows * kZRow<M / 32>, (size_t)HC * (kTRows + 1));
     cudaError_t err;
     if ((err = ensure_dynamic_smem(k_zfft_t1024, smem)) != cudaSuccess)
         return err;
@@ -1510,7 +1528,8 @@ cudaError_t zifft_kz_pass(const GridGeom &g, const float *kz_major, float *out, 
     if (g.dims != 1024)
         return cudaErrorNotSupported;
     constexpr int M = 512, HC = 513;
-    const size_t smem = sizeof(float2) * ((size_t)kTRows * kZRow<M / 32> + (size_t)HC * (kTRows + 1));
+    const size_t smem =
+        sizeof(float2) * std::max((size_t)kTRows * kZRow<M / 32>, (size_t)HC * (kTRows + 1));
     cudaError_t err;
     if ((err = ensure_dynamic_smem(k_zifft_t1024, smem)) != cudaSuccess)
         return err;
