@@ -49,9 +49,9 @@ PEAKS_FALLBACK = {"hbm_gbs": 6800.0}
 # keyed by (kernel, particles per side, grid): the positions and the 64-bit
 # accumulator's lines read, the accumulator written.  Reported only for those
 # workloads.
-NCU_TRAFFIC = {("k_stream_deposit", 512, 512): 2.691e9 + 1.036e9,
+NCU_TRAFFIC = {("k_stream_deposit", 512, 512): 2.691e9 + 1.032e9,
                ("k_window_deposit", 512, 512): 2.692e9 + 1.052e9,
-               ("k_stream_deposit", 256, 256): 337.3e6 + 92.7e6}
+               ("k_stream_deposit", 256, 256): 337.3e6 + 88.0e6}
 
 
 def parse():
@@ -683,19 +683,22 @@ def main():
     peak = float(pk_["hbm_gbs"])
     b_dep, b_bin = algorithmic_bytes(npart, n)
     engine = {1: "sorted", 2: "window", 3: "stream"}.get(ctx.last_engine, "?")
-    t_pass = sum(v for k, v in stages.items() if k.startswith(("dep_", "win_", "stream_"))) * 1e-3
+    t_pass = sum(v for k, v in stages.items() if k.startswith(("dep_", "win_", "stream_", "direct_"))) * 1e-3
     # binning time: the fused x-axis FFT + binning kernel when it ran (it also
     # does the last FFT pass, so this overstates the binning time), else k_bin
     t_bin = (stages.get("xfft_bin", 0.0) + stages.get("bin_kz", 0.0) + stages.get("bin", 0.0)) * 1e-3
     if engine in ("window", "stream"):
-        stage = "win_deposit" if engine == "window" else "stream_deposit"
-        t_k = stages.get(stage, 0.0) * 1e-3
-        kname = "k_window_deposit" if engine == "window" else "k_stream_deposit"
+        # (the stream mode's pass over particles in no order is the direct one)
+        kind = ("window" if engine == "window" else
+                "direct" if "direct_deposit" in stages else "stream")
+        t_k = stages.get({"window": "win_deposit"}.get(kind, kind + "_deposit"), 0.0) * 1e-3
+        kname = f"k_{kind}_deposit"
         lattice = args.workload == "zeldovich" and args.order == "lattice"
         traffic = NCU_TRAFFIC.get((kname, nside, n)) if lattice else None
     else:
         t_k = t_pass
-        kname = "deposit pass (sorted engine: all its kernels)"
+        kname = ("k_direct_deposit and its conversion" if "direct_deposit" in stages else
+                 "deposit pass (sorted engine: all its kernels)")
         traffic = None
     ach = b_dep / t_k / 1e9
     ach_bin = b_bin / t_bin / 1e9 if t_bin > 0 else None

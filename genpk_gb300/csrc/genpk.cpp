@@ -648,7 +648,8 @@ const genpk_ctx::Tuned *find_tuned(const genpk_ctx *ctx, int64_t n, bool var, bo
 // with cuFFT took equal time (uniform random particles, ms of the deposit):
 // 0.069 and 0.079 at 2^20 particles on 128^3, 0.111 and 0.097 at 2^21; 0.131 and
 // 0.141 at 2^19 on 256^3, 0.175 and 0.155 at 2^20; 0.67 and 0.83 at 2^20 on
-// 512^3, 0.88 and 0.86 at 2^21.
+// 512^3, 0.88 and 0.86 at 2^21.  (Both sides have become faster since; the line
+// stays, for a spectrum's last bits follow it.)
 // Particles with masses on 512^3 are stars in the order of a snapshot's cells:
 // direct adds find neighbours in the L2 and are the faster up to where windows
 // hold them (with the own passes 1.09 ms at 1.2 M and 1.24 at 4 M, sorted with
