@@ -35,7 +35,11 @@ struct ModeGradParams {
 // One warp per (x, y) row of the half-complex spectrum: kx, ky, iw(kx) iw(ky)
 // and kx^2 + ky^2 once per row (no 64-bit division per mode), lanes over kz,
 // U modes per lane loaded before any is used.  Along a lane's kz the modulus
-// only grows, so after one log-guided lookup its bin only steps up.
+// only grows, so after one log-guided lookup its bin only steps up; its upper
+// threshold and coefficient stay in registers between steps.  Bound by issue:
+// a threshold and a coefficient read and a division per mode had cost 27 us at
+// N = 160 (20 now), 111 at 384 (92) and 432 at 640 (347).  The next row's loads
+// ahead of this row's work brought nothing.
 __global__ void __launch_bounds__(256)
     k_mode_gradient(ModeGradParams p, float2 *__restrict__ spec, const uint32_t *__restrict__ thr_g,
                     const float *__restrict__ iw, const float *__restrict__ gcoef)
@@ -60,6 +64,8 @@ __global__ void __launch_bounds__(256)
         const float wij = __ldg(iw + i) * __ldg(iw + j);
         float2 *rp = spec + (size_t)row * (size_t)p.hc;
         int b = -1;
+        uint32_t nx = 0;  // the open bin's upper threshold (thr[nrbins]: none)
+        float gb = 0.f;   // its coefficient
         for (int kz0 = 0; kz0 < p.hc; kz0 += 32 * U) {
             float2 f[U];
 #pragma unroll
@@ -75,21 +81,24 @@ __global__ void __launch_bounds__(256)
                 const uint32_t kk2 = r2 + (uint32_t)(kz * kz);
                 float2 h = make_float2(0.f, 0.f);
                 if (kk2 != 0) {
-                    if (b < 0) {
-                        b = (int)(p.bpu_half * __logf((float)kk2));
-                        b = max(0, min(p.nrbins - 1, b));
-                        while (b > 0 && kk2 < thr[b])
-                            b--;
+                    if (kk2 >= nx) {
+                        if (b < 0) {
+                            b = (int)(p.bpu_half * __logf((float)kk2));
+                            b = max(0, min(p.nrbins - 1, b));
+                            while (b > 0 && kk2 < thr[b])
+                                b--;
+                            nx = thr[b + 1];
+                        }
+                        while (kk2 >= nx)
+                            nx = thr[++b + 1];
+                        gb = __ldg(gcoef + b);
                     }
-                    while (b + 1 < p.nrbins && kk2 >= thr[b + 1])
-                        b++;
                     const float pz = wij * __ldg(iw + kz);
                     const float p2 = pz * pz;
-                    const bool edge = (kz == 0 || kz == p.half);               // reference weight 1
-                    const bool selfconj = (kz == 0) || (even && kz == p.half);  // c2r counts once
-                    const float cm = edge ? 1.f : 2.f;
-                    const float mult = selfconj ? 1.f : 2.f;
-                    const float sc = __ldg(gcoef + b) * (p2 * p2) * (cm / mult);
+                    // c_m / mult_m: the reference weighs kz = 0 and kz = N/2 by 1, others
+                    // by 2; the c2r counts the same, but kz = N/2 of odd N twice
+                    const float cm = !even && kz == p.half && kz != 0 ? 0.5f : 1.f;
+                    const float sc = gb * (p2 * p2) * cm;
                     h = make_float2(sc * f[u].x, sc * f[u].y);
                 }
                 rp[kz] = h;
@@ -472,8 +481,9 @@ cudaError_t adjoint_mode_gradient_coef(const GridGeom &g, const BinTables &t, co
     p.half = g.half;
     p.nrbins = t.nrbins;
     p.bpu_half = (float)(0.5 * t.binsperunit);
-    // one warp per row of kz modes; 4 CTAs of 8 warps per SM (46 registers)
-    const int blocks = (int)std::min<int64_t>(((int64_t)g.dims * g.dims + 7) / 8, 152 * 4);
+    // one warp per row of kz modes; 5 CTAs of 8 warps per SM (47 registers; 4: 388
+    // us at N = 640)
+    const int blocks = (int)std::min<int64_t>(((int64_t)g.dims * g.dims + 7) / 8, 152 * 5);
     (*launches)++;
     return launch_after(k_mode_gradient, blocks, 256, sizeof(uint32_t) * (t.nrbins + 1), stream, p,
                         spec, d.thr, d.iw, gcoef_dev);
