@@ -101,3 +101,27 @@ def test_tuned_unordered_passes(gp, dims, mass):
         ctx.zero(0)
         ctx.deposit(0, box, pos, m, 1.0)
         assert np.array_equal(ctx.read_field(0), auto)
+
+
+@pytest.mark.parametrize("masses,count,own", [(True, 2_200_001, True), (False, 2_200_001, False),
+                                              (False, 2_000_003, True)])
+def test_transform_of_unordered_particles_follows_their_count(gp, masses, count, own):
+    """On 512^3 the own z, y and x passes take fewer than 2^21 particles without
+    order, or 3 * 2^21 with masses; the spectrum is the other transform's to FP32
+    rounding (the FP32 transforms' 1e-5 against FP64)."""
+    import torch
+    from genpk_gb300 import api, synth
+
+    pos = synth.uniform(count, 1.0, seed=5, device="cuda")
+    m = torch.rand(count, device="cuda") + 0.5 if masses else None
+    total = float(m.double().sum()) if masses else float(count)
+    with api.Context(512, 32, timing=True) as ctx:
+        ctx.deposit(0, 1.0, pos, m, 1.0)
+        p, c, _ = ctx.power(0, 0, total, total)
+        assert ("zfft" in ctx.stage_times()) == own
+    with api.Context(512, 32) as ctx:
+        ctx.set_fft_mode(1)  # cuFFT's 3-D transform
+        ctx.deposit(0, 1.0, pos, m, 1.0)
+        q, d, _ = ctx.power(0, 0, total, total)
+    np.testing.assert_array_equal(c, d)
+    np.testing.assert_allclose(p[c > 0], q[c > 0], rtol=1e-5)
