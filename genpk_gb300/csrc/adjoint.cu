@@ -17,6 +17,7 @@
 #include "launch.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace genpk {
 namespace {
@@ -183,8 +184,9 @@ struct GatherParams {
     float mass;
     float dl_dm;
     int64_t n;
-    uint32_t plane_b, row_b;     // strides in bytes
-    uint32_t wrap_x, wrap_y, wrap_z;  // bytes from the last cell of an axis to the first
+    // in bytes (kWide: elements): the strides, and from the last cell of an
+    // axis to the first
+    uint32_t plane_o, row_o, wrap_x, wrap_y, wrap_z;
 };
 
 // The trilinear value and the three derivatives of dL/drho at one particle.
@@ -234,9 +236,10 @@ __device__ __forceinline__ void split_cell_fast(float x, float uh, float ul, uin
 
 // How the four-particle kernel reads a particle's eight cells (gather_cells).
 enum Loads {
-    kGeneral,  // split_cell and 64-bit indices: a grid of 4 GB or more
-    kCells,    // eight 4-byte loads
-    kPairs,    // 8-byte loads of z pairs
+    kGeneral,  // split_cell and 64-bit indices: a grid of 2^32 elements or more
+    kWide,     // eight 4-byte loads by 32-bit element offsets: 4 GB or more
+    kCells,    // the same by 32-bit byte offsets
+    kPairs,    // 8-byte loads of z pairs by 32-bit byte offsets
 };
 
 // The cells and fractions of a particle; false for a non-finite one (whose
@@ -264,20 +267,21 @@ __device__ __forceinline__ bool split3_cell(const GatherParams &p, float x, floa
     return finite;
 }
 
-// The gather of a particle inside a grid below 4 GB, by 32-bit byte offsets.
-// PAIRS (even N): a z pair whose lower cell is even is one 8-byte load; an odd
-// lower cell's own pair holds only itself, the upper one is loaded alone.
-template <bool PAIRS>
+// The gather of a particle by 32-bit offsets.  kPairs (even N): a z pair whose
+// lower cell is even is one 8-byte load; an odd lower cell's own pair holds only
+// itself, the upper one is loaded alone.
+template <int LOADS>
 __device__ __forceinline__ GatherOut gather_cells(const GatherParams &p, const float *__restrict__ grid,
                                                   const uint32_t (&c)[3], const float (&d)[3], float m)
 {
+    constexpr uint32_t kCell = LOADS == kWide ? 1u : 4u;  // a cell, in offset units
     const uint32_t last = (uint32_t)p.dims - 1u;
-    const uint32_t sx = c[0] == last ? p.wrap_x : p.plane_b;
-    const uint32_t sy = c[1] == last ? p.wrap_y : p.row_b;
+    const uint32_t sx = c[0] == last ? p.wrap_x : p.plane_o;
+    const uint32_t sy = c[1] == last ? p.wrap_y : p.row_o;
     const char *base = reinterpret_cast<const char *>(grid);
-    const uint32_t row = c[0] * p.plane_b + c[1] * p.row_b;
+    const uint32_t row = c[0] * p.plane_o + c[1] * p.row_o;
     float g[8];
-    if (PAIRS) {
+    if (LOADS == kPairs) {
         const bool odd = c[2] & 1u;
         const uint32_t o = row + (c[2] & ~1u) * 4u;
         const uint32_t oz = c[2] == last ? p.wrap_z + 4u : 8u;  // (last is odd)
@@ -292,13 +296,14 @@ __device__ __forceinline__ GatherOut gather_cells(const GatherParams &p, const f
             g[k + 4] = up;
         }
     } else {
-        const uint32_t o = row + c[2] * 4u;
-        const uint32_t sz = c[2] == last ? p.wrap_z : 4u;
+        const uint32_t o = row + c[2] * kCell;
+        const uint32_t sz = c[2] == last ? p.wrap_z : kCell;
 #pragma unroll
-        for (int k = 0; k < 8; k++)
-            g[k] = __ldg(reinterpret_cast<const float *>(
-                base +
-                (uint32_t)(o + ((k & 4) ? sz : 0u) + ((k & 1) ? sx : 0u) + ((k & 2) ? sy : 0u))));
+        for (int k = 0; k < 8; k++) {
+            const uint32_t s = o + ((k & 4) ? sz : 0u) + ((k & 1) ? sx : 0u) + ((k & 2) ? sy : 0u);
+            g[k] = LOADS == kWide ? __ldg(grid + s)
+                                  : __ldg(reinterpret_cast<const float *>(base + s));
+        }
     }
     return gather_tree(p, g, d, m);
 }
@@ -369,7 +374,7 @@ __global__ void __launch_bounds__(256)
 // conversions and 32-bit byte offsets.  512^3 lattice 0.80 -> 0.70 ms (0.57 ms
 // of memory time), 8 M particles in no order on 256^3 229 -> 162 us.  The 128
 // particles of a warp transposed through shared memory, so that its lanes hold
-// neighbours, took 0.78 ms.
+// neighbours, took 0.78 ms.  1024^3, by element offsets: 6.61 -> 6.03 ms.
 __device__ __forceinline__ GatherOut gather_or_zero(const GatherParams &p, const float *__restrict__ grid,
                                                     float x, float y, float z, float m)
 {
@@ -387,7 +392,7 @@ __device__ __forceinline__ GatherOut gather_any(const GatherParams &p, const flo
     uint32_t c[3];
     float d[3];
     const bool finite = split3_cell(p, x, y, z, c, d);
-    const GatherOut o = gather_cells<LOADS == kPairs>(p, grid, c, d, m);
+    const GatherOut o = gather_cells<LOADS>(p, grid, c, d, m);
     if (!finite)
         return {0.f, 0.f, 0.f, -p.dl_dm};
     return o;
@@ -509,11 +514,6 @@ cudaError_t adjoint_gather(const GridGeom &g, float units_hi, float units_lo, co
     p.mass = mass;
     p.dl_dm = dl_dmass_norm;
     p.n = n;
-    p.plane_b = (uint32_t)(4 * g.plane);
-    p.row_b = 4u * (uint32_t)g.row;
-    p.wrap_x = 0u - (uint32_t)(g.dims - 1) * p.plane_b;
-    p.wrap_y = 0u - (uint32_t)(g.dims - 1) * p.row_b;
-    p.wrap_z = 0u - (uint32_t)(g.dims - 1) * 4u;
     // Four CTAs per resident slot (8 per SM at 32-36 registers).  Sizing the
     // grid to the resident CTAs, so that the stride sweeps the particles in
     // order, cut the DRAM reads at 512^3 from 2.85 to 2.56 GB (2.15 GB of
@@ -528,12 +528,25 @@ cudaError_t adjoint_gather(const GridGeom &g, float units_hi, float units_lo, co
         // reads its own sectors, and a pair is half as many (Morton order at
         // 512^3 1.01 ms, cells 1.09; 8 M in no order on 256^3 162 us, cells 222;
         // 2 M clustered on 160^3 43 us, cells 57).
-        const int loads = sizeof(float) * (uint64_t)g.nfloat > 0xffffffffull ? kGeneral
-                          : coherent || (g.dims & 1)                         ? kCells
-                                                                             : kPairs;
-        auto kern = loads == kGeneral ? (masses ? k_gather4<true, kGeneral> : k_gather4<false, kGeneral>)
-                    : loads == kCells ? (masses ? k_gather4<true, kCells> : k_gather4<false, kCells>)
-                                      : (masses ? k_gather4<true, kPairs> : k_gather4<false, kPairs>);
+        const uint64_t cells = (uint64_t)g.nfloat;
+        const int loads = cells > 0xffffffffull                   ? kGeneral
+                          : sizeof(float) * cells > 0xffffffffull ? kWide
+                          : coherent || (g.dims & 1)              ? kCells
+                                                                  : kPairs;
+        const uint32_t cell = loads == kWide ? 1u : (uint32_t)sizeof(float);
+        p.plane_o = (uint32_t)g.plane * cell;
+        p.row_o = (uint32_t)g.row * cell;
+        p.wrap_x = 0u - (uint32_t)(g.dims - 1) * p.plane_o;
+        p.wrap_y = 0u - (uint32_t)(g.dims - 1) * p.row_o;
+        p.wrap_z = 0u - (uint32_t)(g.dims - 1) * cell;
+        auto pick = [&](auto k) {
+            constexpr int L = decltype(k)::value;
+            return masses ? k_gather4<true, L> : k_gather4<false, L>;
+        };
+        auto kern = loads == kGeneral ? pick(std::integral_constant<int, kGeneral>{})
+                    : loads == kWide  ? pick(std::integral_constant<int, kWide>{})
+                    : loads == kCells ? pick(std::integral_constant<int, kCells>{})
+                                      : pick(std::integral_constant<int, kPairs>{});
         (*launches)++;
         return launch_after(kern, blocks4, 256, 0, stream, p, grid, pos, masses, grad_pos, grad_mass);
     }

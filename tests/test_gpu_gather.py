@@ -36,7 +36,7 @@ def _positions(dims, order):
 
 @pytest.mark.parametrize("masses", [False, True])
 @pytest.mark.parametrize("order", ["random", "lattice"])
-@pytest.mark.parametrize("dims", [16, 33, 64, 100])
+@pytest.mark.parametrize("dims", [16, 33, 64, 100, 1024])
 def test_gather_kernels_agree(dims, order, masses):
     from genpk_gb300 import api
 
