@@ -1075,11 +1075,15 @@ __global__ void k_direct_end(const __grid_constant__ DirectEnd e, DeviceStatus *
 // needs no clear) and ends the pass: the last block to have read the constants
 // does that.  Two cells per thread and round, four rounds' loads ahead of their
 // stores: with each pair cleared right after its load, loads waited 5 us for
-// the stores beside them (256^3 grid: 340 us, 54 so; 128^3 26 and 13).
+// the stores beside them (256^3 grid: 340 us, 54 so; 128^3 26 and 13).  32-bit
+// pair indices where wide_index() says so of the grid's elements: twice the
+// pairs, so that the last round's steps past the end do not wrap either.
+template <bool WIDE>
 __global__ void __launch_bounds__(256)
-    k_direct_convert(acc_t *acc, float *__restrict__ grid, int dims, int row, unsigned npairs,
+    k_direct_convert(acc_t *acc, float *__restrict__ grid, int dims, int row, int64_t pairs,
                      const __grid_constant__ DirectEnd e, DeviceStatus *st)
 {
+    typedef typename CellIndex<WIDE>::T I;
     __shared__ long long sh_mean;
     __shared__ float sh_scale;
     wait_previous();
@@ -1098,10 +1102,11 @@ __global__ void __launch_bounds__(256)
     __syncthreads();
     const long long mean = sh_mean;
     const float inv_scale = sh_scale;
-    const unsigned half_row = (unsigned)row >> 1;
-    const unsigned last = (unsigned)(dims - 1) >> 1;  // the pair holding z = dims - 1
-    const unsigned stride = gridDim.x * 256;
-    for (unsigned k0 = blockIdx.x * 256 + threadIdx.x; k0 < npairs; k0 += 4 * stride) {
+    const I npairs = (I)pairs;
+    const I half_row = (I)(row >> 1);
+    const I last = (I)((dims - 1) >> 1);  // the pair holding z = dims - 1
+    const I stride = (I)(gridDim.x * 256);
+    for (I k0 = (I)(blockIdx.x * 256 + threadIdx.x); k0 < npairs; k0 += 4 * stride) {
         longlong2 v[4];
 #pragma unroll
         for (int u = 0; u < 4; u++)
@@ -1109,8 +1114,8 @@ __global__ void __launch_bounds__(256)
                 v[u] = __ldcs(reinterpret_cast<longlong2 *>(acc) + k0 + u * stride);
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const unsigned k = k0 + u * stride;
-            const unsigned z = k % half_row;
+            const I k = k0 + u * stride;
+            const I z = k % half_row;
             if (k >= npairs || z > last)
                 continue;
             float2 f = make_float2(i64_to_f32_rn(v[u].x - mean) * inv_scale,
@@ -1394,10 +1399,8 @@ WinParams make_win_params(const DepositGeom &g, const DepositArgs &a, int chunk)
     return p;
 }
 
-// 32-bit element indices (false) where every index and both of the stream
-// mode's sentinels fit.  The environment variable GENPK_WIDE_INDEX=1 forces the
-// 64-bit variants on any grid (a test hook: they otherwise run only from
-// N = 1626 up).
+}  // namespace
+
 bool wide_index(const GridGeom &g)
 {
     static const bool force_wide = [] {
@@ -1406,8 +1409,6 @@ bool wide_index(const GridGeom &g)
     }();
     return force_wide || g.nfloat >= ((int64_t)1 << 32) - 2;
 }
-
-}  // namespace
 
 int window_cap_cells(int chunk, bool variable_masses)
 {
@@ -1589,11 +1590,11 @@ cudaError_t deposit_direct_pass(const DepositGeom &g, const DepositArgs &a, doub
         (*launches)++;
         return launch_after(k_direct_end, 1, 1, 0, stream, e, dstat);
     }
-    const unsigned pairs = (unsigned)(g.grid.nfloat / 2);
-    const unsigned cctas =
-        (unsigned)std::min<int64_t>(((int64_t)pairs + 511) / 512, (int64_t)num_sms * 8);
-    if ((err = launch_after(k_direct_convert, cctas, 256, 0, stream, acc, a.grid, g.grid.dims,
-                            g.grid.row, pairs, e, dstat)) != cudaSuccess)
+    const int64_t pairs = g.grid.nfloat / 2;
+    const unsigned cctas = (unsigned)std::min<int64_t>((pairs + 511) / 512, (int64_t)num_sms * 8);
+    if ((err = launch_after(wide ? k_direct_convert<true> : k_direct_convert<false>, cctas, 256, 0,
+                            stream, acc, a.grid, g.grid.dims, g.grid.row, pairs, e, dstat)) !=
+        cudaSuccess)
         return err;
     mark("direct_convert");
     return cudaSuccess;

@@ -25,6 +25,12 @@ struct GridGeom {
 
 GridGeom make_grid_geom(int dims);
 
+// 32-bit element indices (false) where every index and both of the stream
+// mode's sentinels fit.  The environment variable GENPK_WIDE_INDEX=1 forces the
+// 64-bit variants on any grid (a test hook: they otherwise run only from
+// N = 1626 up).
+bool wide_index(const GridGeom &g);
+
 // Raise `func`'s dynamic shared-memory limit on the current device to at
 // least `bytes` (never lower it).  The limit is per kernel and device for the
 // whole process, so contexts used from several host threads would otherwise
@@ -216,8 +222,7 @@ cudaError_t deposit_window_pass(const DepositGeom &g, const DepositArgs &a, int 
                                 StageHook hook, void *hook_user);
 // A pass over particles in no order without a sort: as deposit_window_pass,
 // with scattered reductions (k_direct_deposit).  Unless the conversion is
-// deferred, the accumulator is zero again after the pass.  Grids of fewer than
-// 2^33 elements.
+// deferred, the accumulator is zero again after the pass.
 cudaError_t deposit_direct_pass(const DepositGeom &g, const DepositArgs &a, double *mass_part,
                                 int mass_ctas, unsigned long long *acc, size_t clear_bytes,
                                 bool defer_convert, int num_sms, DeviceStatus *dstat,
