@@ -54,6 +54,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <cstring>
 #include <type_traits>
 
 namespace genpk {
@@ -90,6 +91,10 @@ struct WinParams {
     // k_window_prep ran before the pass.
     int host_prep;
     int fx_shift;
+    // How far a uniform mass's exponent lies below the pass's: 0 unless the shift
+    // is held at its limit, for masses below 2^-73, which only the direct kernel
+    // takes (deposit_window_pass).
+    int udsh;
     double pass_mass;
     long long mean_fixed;
     double *field_mass, *field_sub;
@@ -965,7 +970,7 @@ __global__ void __launch_bounds__(kDirectThreads)
         const unsigned mant = (mb & 0x7fffffu) | 0x800000u;
         const bool neg = (mb >> 31) != 0u;
         valid = valid && ef != 0;  // zero or subnormal mass deposits nothing
-        const int dsh = VARMASS ? max(emax - ef, 0) : 0;
+        const int dsh = VARMASS ? max(emax - ef, 0) : p.udsh;
         if (CORNER && valid) {
             f2sum v = corner_factor_q(a[0], a[1], a[2]);
             if (VARMASS) {
@@ -1362,6 +1367,14 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+int uniform_shift(float mass, int fx_shift)
+{
+    uint32_t bits;
+    memcpy(&bits, &mass, sizeof bits);
+    const int ef = (int)((bits >> 23) & 0xffu);
+    return ef ? std::max(154 - fx_shift - ef, 0) : 0;  // (ef == 0 deposits nothing)
+}
+
 WinParams make_win_params(const DepositGeom &g, const DepositArgs &a, int chunk)
 {
     WinParams p;
@@ -1392,6 +1405,7 @@ WinParams make_win_params(const DepositGeom &g, const DepositArgs &a, int chunk)
     p.skip_wait = a.skip_wait;
     p.host_prep = 0;
     p.fx_shift = 0;
+    p.udsh = 0;
     p.pass_mass = 0.0;
     p.mean_fixed = 0;
     p.field_mass = p.field_sub = nullptr;
@@ -1483,6 +1497,11 @@ cudaError_t deposit_window_pass(const DepositGeom &g, const DepositArgs &a, int 
         // deposit kernel stores them (one launch fewer per pass)
         const double umass = (double)a.mass;
         const PassConsts k = pass_consts((double)a.n * umass, (float)fabs(umass), 1.0 / n3);
+        // A mass below 2^-73: the weights need a shift of their own.  A test for it
+        // in the loops of the window and stream kernels cost every pass 1-2 %.
+        if (uniform_shift(a.mass, k.fx_shift) > 0)
+            return deposit_direct_pass(g, a, mass_part, mass_ctas, acc, clear_bytes, defer_convert,
+                                       num_sms, dstat, stream, launches, hook, hook_user);
         p.host_prep = 1;
         p.fx_shift = k.fx_shift;
         p.pass_mass = k.mass;
@@ -1555,6 +1574,7 @@ cudaError_t deposit_direct_pass(const DepositGeom &g, const DepositArgs &a, doub
     e.field_sub = a.field_sub;
     e.field_corner = a.field_corner;
     p.fx_shift = e.host.fx_shift;
+    p.udsh = uniform_shift(a.mass, e.host.fx_shift);
     if (a.masses) {
         if ((err = launch_after(k_mass_reduce, mass_ctas, 256, 0, stream, a.masses, a.n, mass_part,
                                 dstat)) != cudaSuccess)
