@@ -125,3 +125,33 @@ def test_transform_of_unordered_particles_follows_their_count(gp, masses, count,
         q, d, _ = ctx.power(0, 0, total, total)
     np.testing.assert_array_equal(c, d)
     np.testing.assert_allclose(p[c > 0], q[c > 0], rtol=1e-5)
+
+
+@pytest.mark.parametrize("masses", [False, True])
+def test_unordered_particles_on_1024_take_the_kz_major_transform(gp, masses):
+    """The direct pass stays in the accumulator, which the kz-major z pass reads;
+    the spectrum is the library transform's to FP32 rounding (1e-5)."""
+    import torch
+    from genpk_gb300 import api, synth
+
+    n = 300_001
+    pos = synth.uniform(n, 1.0, seed=9, device="cuda")
+    m = torch.rand(n, device="cuda") + 0.5 if masses else None
+    total = float(m.double().sum()) if masses else float(n)
+    with api.Context(1024, 32, timing=True) as ctx:
+        got = []
+        for _ in range(2):  # the binning leaves the accumulator clear
+            ctx.zero(0)
+            ctx.timing_reset()
+            ctx.deposit(0, 1.0, pos, m, 1.0)
+            got.append(ctx.power(0, 0, total, total))
+            stages = ctx.stage_times()
+            assert "direct_deposit" in stages and "zfft_kz" in stages
+            assert "direct_convert" not in stages or "tune" in stages
+    with api.Context(1024, 32) as ctx:
+        ctx.set_fft_mode(1)  # cuFFT's 3-D transform
+        ctx.deposit(0, 1.0, pos, m, 1.0)
+        q, d, _ = ctx.power(0, 0, total, total)
+    for p, c, _ in got:
+        np.testing.assert_array_equal(c, d)
+        np.testing.assert_allclose(p[c > 0], q[c > 0], rtol=1e-5)
