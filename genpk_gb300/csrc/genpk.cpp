@@ -89,6 +89,9 @@ struct genpk_ctx {
     bool c2c_kz_made = false;
     // per field: its spectrum is kz-major, S[kz][x][y] (the N = 1024 transform)
     std::vector<bool> kzmajor;
+    // Fields whose latest pass was a stream one, of neighbours in order (the
+    // adjoint's gather loads their cells one by one, others' in pairs).
+    std::vector<bool> coherent;
     void *fft_work = nullptr;
     size_t fft_work_size = 0;
 
@@ -845,6 +848,9 @@ int run_deposit(genpk_ctx *ctx, int f, double boxsize, const float *pos, const f
     }
     a.host_mapped = host_mapped;
     ctx->last_engine = engine;
+    // (the tuner's direct pass counts as the stream engine's, its particles as
+    // unordered)
+    ctx->coherent[(size_t)f] = engine == GENPK_ENGINE_STREAM && !direct;
     timing_touch(ctx);
     // A clean grid headed for the own z/y/x transform or the kz-major one keeps a
     // window or stream pass, or the tuner's direct pass, in the accumulator: the z
@@ -1513,6 +1519,8 @@ uint64_t issue_digest(const genpk_ctx *ctx)
         mix(v);
     for (bool v : ctx->kzmajor)
         mix(v);
+    for (bool v : ctx->coherent)
+        mix(v);
     mix((uint64_t)ctx->acc_pending);
     mix((uint64_t)ctx->own_pending);
     mix(ctx->acc_zero);
@@ -1550,7 +1558,7 @@ uint64_t issue_digest(const genpk_ctx *ctx)
 // record taken before it is put back.
 struct IssueState {
     std::vector<int> state;
-    std::vector<bool> corner_valid, kzmajor, auto_valid;
+    std::vector<bool> corner_valid, kzmajor, coherent, auto_valid;
     std::vector<double> auto_mass;
     std::vector<std::vector<double>> auto_power;
     int acc_pending = -1, own_pending = -1;
@@ -1561,7 +1569,7 @@ struct IssueState {
 
     explicit IssueState(const genpk_ctx *c)
         : state(c->state), corner_valid(c->corner_valid), kzmajor(c->kzmajor),
-          auto_valid(c->auto_valid), auto_mass(c->auto_mass), auto_power(c->auto_power),
+          coherent(c->coherent), auto_valid(c->auto_valid), auto_mass(c->auto_mass), auto_power(c->auto_power),
           acc_pending(c->acc_pending), own_pending(c->own_pending), acc_zero(c->acc_zero), acc_spent(c->acc_spent),
           acc_dirty_bytes(c->acc_dirty_bytes), last_engine(c->last_engine), deferred(c->deferred)
     {
@@ -1571,6 +1579,7 @@ struct IssueState {
         c->state = state;
         c->corner_valid = corner_valid;
         c->kzmajor = kzmajor;
+        c->coherent = coherent;
         c->auto_valid = auto_valid;
         c->auto_mass = auto_mass;
         c->auto_power = auto_power;
@@ -1816,6 +1825,7 @@ int ctx_create(int64_t dims, int nrbins, int nfields, unsigned flags, genpk_ctx 
     ctx->auto_valid.assign((size_t)nfields, false);
     ctx->corner_valid.assign((size_t)nfields, false);
     ctx->kzmajor.assign((size_t)nfields, false);
+    ctx->coherent.assign((size_t)nfields, false);
     ctx->tile = deposit_default_tile((int)dims, 0);
     (void)rc;
     *out = ctx;
@@ -2330,7 +2340,7 @@ int genpk_adjoint(genpk_ctx *ctx, int field, double boxsize, const float *pos, c
         st_out = reinterpret_cast<DeviceStatus *>(ctx->res_dev);
     }
     GENPK_CUDA(adjoint_gather(ctx->gg, dg.units_hi, dg.units_lo, g, dpos, dmass, (float)mass, n,
-                              dgpos, dgmass, (float)dldm, ctx->last_engine == GENPK_ENGINE_STREAM,
+                              dgpos, dgmass, (float)dldm, ctx->coherent[(size_t)field],
                               ctx->d_status, st_out, ctx->stream, &ctx->launches));
     stage_event(ctx, "adj_gather");
     if (!dev) {
@@ -2737,6 +2747,7 @@ int group_issue(genpk_batch::Group &g, const double *boxsize, const float *const
         ctx->state[(size_t)f] = F_CLEAN;
         ctx->auto_valid[(size_t)f] = false;
         ctx->kzmajor[(size_t)f] = false;
+        ctx->coherent[(size_t)f] = false;
         ctx->corner_valid[(size_t)f] = false;
     }
     if (!g.tuned || g.tuned_n != counts) {

@@ -91,3 +91,56 @@ def test_coefficients_by_value_and_by_copy(nrbins):
         gpos, _, _ = ctx.adjoint(0, box, pos, g, m, mass=1.0)
     ref, _, _ = O.reference_gradient(pos, box, dims, nrbins, g, None, 1.0, m_norm=m)
     assert np.abs(gpos - ref).max() <= 1e-4 * np.abs(ref).max()
+
+
+def _gather_form(ctx, call):
+    """The last template argument of the gather kernel that `call` launches
+    (2: single cells, 3: z pairs); None where kernels cannot be traced."""
+    import re
+    from torch.profiler import ProfilerActivity, profile
+
+    kinds = [ProfilerActivity.CPU, ProfilerActivity.CUDA]
+    with profile(activities=kinds):  # (the first trace of a process may come back empty)
+        torch.ones(1, device="cuda")
+        torch.cuda.synchronize()
+    with profile(activities=kinds) as prof:
+        call()
+        torch.cuda.synchronize()
+    names = [e.key for e in prof.key_averages() if "k_gather" in e.key]
+    if not names:
+        return None
+    return int(re.search(r"k_gather4<\w+, (\d)>", names[0].replace("(int)", "")).group(1))
+
+
+def test_gather_form_follows_the_fields_order():
+    """The tuner's direct pass has particles in no order: z pairs.  With the
+    forward pass kept, the field's own latest pass counts, not the context's."""
+    from genpk_gb300 import api, synth
+
+    dims, n = 128, 400_000
+    random = synth.uniform(n, BOX, seed=3, device="cuda")
+    lattice = synth.zeldovich(128, BOX, seed=3, device="cuda")
+    slope = np.ones(16)
+    with api.Context(dims, 16, nfields=2) as ctx:
+        def grad(field, pos):
+            ctx.power(field, field, float(n), float(n))
+            return ctx.adjoint(field, BOX, pos, slope, float(n), mass=1.0, recompute=False)
+
+        def deposit(field, pos):
+            ctx.zero(field)
+            ctx.deposit(field, BOX, pos, None, 1.0)
+            ctx.sync()
+
+        deposit(0, random)
+        assert ((0, 0, 0), 0) in [(t, c) for t, c, _ in ctx.deposit_trials()]
+        form = _gather_form(ctx, lambda: grad(0, random))
+        if form is None:
+            pytest.skip("no kernel trace on this machine")
+        assert form == 3
+        deposit(0, lattice)  # found to be in order: the stream engine
+        assert ctx.last_engine == api.ENGINE_STREAM
+        deposit(1, random)
+        assert _gather_form(ctx, lambda: grad(0, lattice)) == 2
+        deposit(0, lattice)
+        deposit(1, random)
+        assert _gather_form(ctx, lambda: grad(1, random)) == 3
