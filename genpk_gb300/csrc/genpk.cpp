@@ -2117,6 +2117,12 @@ int genpk_load_spectrum(genpk_ctx *ctx, int field, const double *spectrum)
     cudaSetDevice(ctx->device);
     if (ctx->pend.active && ctx->pend.field == field)
         GENPK_TRY(flush_pending(ctx));
+    if (ctx->acc_pending == field) {
+        ctx->acc_pending = -1;  // (or its conversion would overwrite the spectrum)
+        ctx->acc_spent = true;
+    }
+    if (ctx->own_pending == field)
+        ctx->own_pending = -1;
     // The doubles go to the device as they are (through a buffer of at most 64
     // MB) and are rounded to floats there: a host loop over them took 0.8 of the
     // 1.1 ms of a 128^3 spectrum.

@@ -55,3 +55,27 @@ def test_host_spectrum_in_pieces(gp, dims):
     assert np.array_equal(c, cr)
     ok = cr > 0
     assert (np.abs(p[ok] - pr[ok]) / pr[ok]).max() <= 1e-5
+
+
+@pytest.mark.parametrize("engine", [0, 1, 2, 3])
+def test_loaded_spectrum_replaces_a_deposit(gp, engine):
+    """A deposit still in the accumulator when a spectrum is loaded in its place
+    does not come back over it."""
+    import torch
+    dims = 128
+    rng = np.random.default_rng(3)
+    shape = (dims, dims, dims // 2 + 1)
+    f = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    pos = torch.tensor(rng.random((300_000, 3)).astype(np.float32), device="cuda")
+    with gp.Context(dims, 8) as ctx:
+        ctx.load_spectrum(0, f)
+        want = ctx.power(0, 0, 2.0, 2.0)[0]
+    with gp.Context(dims, 8, nfields=2) as ctx:
+        ctx.set_engine(engine)
+        ctx.deposit(0, 1.0, pos, None, 1.0)
+        ctx.sync()
+        ctx.load_spectrum(0, f)
+        assert np.array_equal(ctx.power(0, 0, 2.0, 2.0)[0], want)
+        ctx.deposit(1, 1.0, pos, None, 1.0)  # a later pass starts from a clear accumulator
+        ctx.power(1, 1, 3e5, 3e5)
+        assert np.array_equal(ctx.power(0, 0, 2.0, 2.0)[0], want)
