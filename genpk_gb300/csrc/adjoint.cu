@@ -529,7 +529,7 @@ cudaError_t adjoint_gather(const GridGeom &g, float units_hi, float units_lo, co
         // 512^3 1.01 ms, cells 1.09; 8 M in no order on 256^3 162 us, cells 222;
         // 2 M clustered on 160^3 43 us, cells 57).
         const uint64_t cells = (uint64_t)g.nfloat;
-        const int loads = cells > 0xffffffffull                   ? kGeneral
+        const int loads = wide_index(g)                           ? kGeneral
                           : sizeof(float) * cells > 0xffffffffull ? kWide
                           : coherent || (g.dims & 1)              ? kCells
                                                                   : kPairs;

@@ -46,9 +46,50 @@ for dims, n in ((64, 5000), (75, 4001), (75, 70001), (100, 70001)):
 print("wide ok")
 """
 
-
 def test_direct_passes_64bit_indices():
     r = subprocess.run([sys.executable, "-c", _DIRECT.format(root=ROOT)],
+                       env={**os.environ, "GENPK_WIDE_INDEX": "1"}, capture_output=True,
+                       text=True, timeout=600)
+    assert r.returncode == 0 and "wide ok" in r.stdout, r.stdout + r.stderr
+
+
+# The four-particle gather with 64-bit indices against the one-particle kernel
+# (arrays off a 16-byte boundary), bit for bit.
+_GATHER = """
+import sys, numpy as np, torch
+sys.path.insert(0, {root!r})
+from genpk_gb300 import api
+rng = np.random.default_rng(2)
+n = 20003
+values = rng.random((n, 3)).astype(np.float32)
+values[::50] += 2.0
+values[7] = np.nan
+weights = rng.random(n).astype(np.float32) + 0.5
+for dims in (33, 64):
+    for masses in (False, True):
+        out = []
+        for shift in (0, 1):
+            p = torch.empty(3 * n + 1, device="cuda")[shift:shift + 3 * n].view(n, 3)
+            p.copy_(torch.tensor(values))
+            w = None
+            if masses:
+                w = torch.empty(n + 1, device="cuda")[shift:shift + n]
+                w.copy_(torch.tensor(weights))
+            with api.Context(dims, 16) as ctx:
+                ctx.deposit(0, 1.0, p[:7].contiguous(), None, 1.0)
+                ctx.power(0, 0, 7.0, 7.0)
+                gp, gm, _ = ctx.adjoint(0, 1.0, p, np.cos(np.arange(16.0)), 7.0, masses=w,
+                                        mass=1.0, recompute=False)
+                out.append((gp.cpu().numpy(), None if gm is None else gm.cpu().numpy()))
+        assert (out[0][0][:5] != 0).all() and (out[0][0][7] == 0).all()
+        for a, b in zip(*out):
+            assert a is b or np.array_equal(a.view(np.uint32), b.view(np.uint32))
+print("wide ok")
+"""
+
+
+def test_gather_64bit_indices():
+    r = subprocess.run([sys.executable, "-c", _GATHER.format(root=ROOT)],
                        env={**os.environ, "GENPK_WIDE_INDEX": "1"}, capture_output=True,
                        text=True, timeout=600)
     assert r.returncode == 0 and "wide ok" in r.stdout, r.stdout + r.stderr
