@@ -495,7 +495,7 @@ int density_band(const genpk_ctx *ctx, int64_t n)
 }
 
 constexpr int64_t kTuneMinParticles = (int64_t)1 << 16;
-// The largest accumulator of a direct pass below that count (N = 264).  A direct
+// The largest accumulator of a direct pass below that count (N = 269).  A direct
 // pass reads, converts and clears it whole; us of the deposit, direct and binned
 // sort, 40 k particles: 20 and 29 on 64^3, 25 and 41 on 128^3, 42 and 60 on
 // 200^3, 76 and 97 on 256^3.

@@ -155,3 +155,23 @@ def test_unordered_particles_on_1024_take_the_kz_major_transform(gp, masses):
     for p, c, _ in got:
         np.testing.assert_array_equal(c, d)
         np.testing.assert_allclose(p[c > 0], q[c > 0], rtol=1e-5)
+
+
+@pytest.mark.parametrize("dims,n,mass,masses,direct", [
+    (269, 65535, 1.0, False, True),   # the largest accumulator and count of an untuned direct pass
+    (270, 65535, 1.0, False, False),  # one past that accumulator: the sort
+    (269, 5000, 1.0, True, False),    # masses: the sort
+])
+def test_where_untuned_direct_passes_end(gp, dims, n, mass, masses, direct):
+    rng = np.random.default_rng(dims)
+    pos = rng.random((n, 3)).astype(np.float32)
+    m = rng.random(n).astype(np.float32) if masses else None
+    with gp.Context(dims, 8, timing=True) as ctx:
+        ctx.deposit(0, 1.0, pos, m, mass)
+        got = ctx.read_field(0)
+        stages = ctx.stage_times()
+        assert ("direct_deposit" in stages) == direct and ("dep_tile" in stages) != direct
+        ctx.set_engine(gp.api.ENGINE_SORTED)
+        ctx.zero(0)
+        ctx.deposit(0, 1.0, pos, m, mass)
+        assert np.array_equal(ctx.read_field(0), got)
