@@ -46,6 +46,7 @@ for dims, n in ((64, 5000), (75, 4001), (75, 70001), (100, 70001)):
 print("wide ok")
 """
 
+
 def test_direct_passes_64bit_indices():
     r = subprocess.run([sys.executable, "-c", _DIRECT.format(root=ROOT)],
                        env={**os.environ, "GENPK_WIDE_INDEX": "1"}, capture_output=True,
