@@ -279,9 +279,11 @@ void acc_overwritten(genpk_ctx *ctx, size_t bytes)
 #define GENPK_CUDA(call)                                                                      \
     do {                                                                                      \
         cudaError_t e_ = (call);                                                              \
-        if (e_ != cudaSuccess)                                                                \
+        if (e_ != cudaSuccess) {                                                              \
+            cudaGetLastError(); /* reported here, and not again by a later launch's check */  \
             return fail(ctx, e_ == cudaErrorMemoryAllocation ? GENPK_ERR_NOMEM : GENPK_ERR_CUDA, \
                         std::string(#call) + ": " + cudaGetErrorString(e_));                  \
+        }                                                                                     \
     } while (0)
 
 #define GENPK_CUFFT(call)                                                                     \
@@ -1784,6 +1786,7 @@ int ctx_create(int64_t dims, int nrbins, int nfields, unsigned flags, genpk_ctx 
     do {                                                                                      \
         cudaError_t e_ = (call);                                                              \
         if (e_ != cudaSuccess) {                                                              \
+            cudaGetLastError();                                                               \
             ctx->err = std::string(#call) + ": " + cudaGetErrorString(e_);                    \
             return bail(e_ == cudaErrorMemoryAllocation ? GENPK_ERR_NOMEM : GENPK_ERR_CUDA);  \
         }                                                                                     \

@@ -92,3 +92,24 @@ def test_context_stays_usable_after_a_timeout(gp):
     ok = cr > 0
     rel = np.abs(p[ok] - pr[ok]) / np.abs(pr[ok])
     assert rel.max() <= 1e-5, rel.max()
+
+
+@pytest.mark.parametrize("how", ["context", "spectrum"])
+def test_an_allocation_that_fails_is_reported_once(gp, how):
+    """A grid that does not fit is refused; the calls after it do not report it
+    again."""
+    import torch
+    from genpk_gb300 import synth
+    dpos = synth.uniform(1 << 20, 1.0, seed=1, device="cuda")
+    rng = np.random.default_rng(1)
+    f = rng.standard_normal((16, 16, 9)) + 0j
+    with gp.Context(16, 4) as ctx, gp.Context(64, 4) as other:
+        with pytest.raises(gp.GenPKError):
+            gp.Context(4096, 8, nfields=4)  # 1.1 TB
+        if how == "context":
+            other.deposit(0, 1.0, dpos, None, 1.0)
+            assert abs(other.read_field(0).sum() / (1 << 20) - 1) < 1e-5
+        else:
+            ctx.load_spectrum(0, f)
+            assert (ctx.power(0, 0, 1.0, 1.0)[0] >= 0).all()
+    assert torch.cuda.is_available()
