@@ -46,7 +46,8 @@
 // the accumulator, xfft.cu k_zfft).  The grid is therefore bit-identical to
 // the sorted engine's, in either mode, and independent of summation order.
 // The accumulator is zeroed before each pass: by a memset here, or already by
-// the binning x pass of the spectrum that used its previous contents.
+// what used its previous contents: the binning pass of the spectrum, or
+// k_direct_convert.
 #include "bulk.cuh"
 #include "common.cuh"
 #include "internal.h"
@@ -1181,8 +1182,8 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// Pass constants for the window engine (one thread), as k_sort_scan forms
-// them for the sorted engine: pass mass, fixed-point shift s (the largest |mass|
+// Pass constants for the window engine and direct passes (one thread), as scan_box
+// and k_bin_sort form them for the sorted engine: pass mass, fixed-point shift s (the largest |mass|
 // maps into [2^27, 2^28) units of 2^-s) and the pass mean in fixed point,
 // rounded to 24 significant bits (an empty cell then reads back exactly 0).
 // nparts = 0: uniform mass umass; else the sum of nparts partial sums.
@@ -1477,7 +1478,7 @@ cudaError_t deposit_window_pass(const DepositGeom &g, const DepositArgs &a, int 
     };
     cudaError_t err;
     // (max_mass_bits and alt_sum are zero here: the pass that used them last
-    // zeroed them, in k_window_prep / k_sort_scan and the finishing kernels)
+    // zeroed them, in k_window_prep / scan_box / k_bin_sort and the finishing kernels)
     const double n3 = (double)g.grid.dims * g.grid.dims * g.grid.dims;
     WinParams p = make_win_params(g, a, chunk);
     if (a.masses) {

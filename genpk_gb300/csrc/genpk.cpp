@@ -509,11 +509,11 @@ constexpr int kTuneReps = 2;
 // The deposit autotuner for particle orders without spatial coherence.  On
 // the first clean pass of a density band (and mass kind) it runs the pass once
 // per candidate -- the sorted engine with tiles 8^3, 16x16x8 and 16^3, and
-// (with_stream) the stream engine, whose reductions go straight to the accumulator -- timed with CUDA
-// events, and keeps the fastest.  (Measured on uniform random particles: the
-// stream engine is 2-2.6x faster at 1e6 particles, where the sort's fixed
-// costs dominate, about even at 3e7 on a 128^3 grid, and 1.75x slower at 3e7
-// on a 256^3 grid, whose accumulator exceeds the L2.)  Every candidate writes
+// (with_stream) the direct pass, whose reductions go straight to the accumulator
+// -- timed with CUDA events, and keeps the fastest.  (Uniform random particles, us,
+// direct and the best sort: 100 k on 128^3 20 and 24, 1.9 M 61 and 58; 100 k on
+// 256^3 39 and 86, 1.5 M 175 and 108; 2 M on 512^3 472 and 774, 6.2 M with masses
+// 1199 and 977; 8 M on 1024^3 4839 and 5606.)  Every candidate writes
 // the same grid (the sums are exact), so the trials only cost time: each
 // overwrites the clean grid and starts the field's running sums, and the error
 // counters are put back before the next.  The chosen candidate then runs as
@@ -655,10 +655,12 @@ const genpk_ctx::Tuned *find_tuned(const genpk_ctx *ctx, int64_t n, bool var, bo
 // 0.141 at 2^19 on 256^3, 0.175 and 0.155 at 2^20; 0.67 and 0.83 at 2^20 on
 // 512^3, 0.88 and 0.86 at 2^21.  (Both sides have become faster since; the line
 // stays, for a spectrum's last bits follow it.)
-// Particles with masses on 512^3 are stars in the order of a snapshot's cells:
-// direct adds find neighbours in the L2 and are the faster up to where windows
-// hold them (with the own passes 1.09 ms at 1.2 M and 1.24 at 4 M, sorted with
-// cuFFT 1.53 and 1.64; from 5 M on they are windows).
+// With masses on 512^3 the line lies higher: stars in the order of a snapshot's
+// cells kept the stream mode and the own passes there before the rule (with the
+// own passes 1.09 ms a spectrum at 1.2 M and 1.24 at 4 M, sorted with cuFFT 1.53
+// and 1.64; from 5 M on they are windows).  In random order, where sort and cuFFT
+// took 1.74 ms at 2.16 M, 1.80 at 4 M and 1.89 at 6.2 M, it is 1.34, 1.64 and
+// 1.78: direct passes to about 4.5 M, then the sort, with the own passes.
 int64_t own_transform_limit(int64_t dims, bool masses)
 {
     return dims <= 128   ? (int64_t)3 << 19

@@ -118,10 +118,11 @@ struct TileShape {
 };
 bool deposit_tile_supported(int tx, int ty, int tz);
 TileShape deposit_default_tile(int dims, int64_t n);
-// Particles a sort CTA takes at a time.
+// Particles a CTA of the counting sort takes at a time.
 constexpr int kSortChunkParticles = 4096;
-// Sort CTAs of a pass: two per SM (one where the per-CTA tile histogram leaves
-// no room for two), and no more than one per chunk.
+// Sort CTAs of a pass.  A binned pass (deposit_binned): one per SM, and no more
+// than one per 1024 particles.  Else two per SM (one where the per-CTA tile
+// histogram leaves no room for two), and no more than one per chunk.
 int deposit_sort_ctas(const DepositGeom &g, int64_t n, int num_sms);
 size_t deposit_hist_smem(const DepositGeom &g);
 size_t deposit_cursor_words(const DepositGeom &g);
@@ -171,7 +172,8 @@ struct GroupLayout {
 GroupLayout deposit_group_layout(int nbox, const GroupBox *boxes, int sort_ctas);
 // Scratch elements a grouped pass needs beyond deposit_scratch_sizes per box:
 // tile_start nbox x (ntiles + 1), totals nbox x ntiles (zeroed once), cursor
-// nbox x deposit_cursor_words, sorted rec0[nbox], mass_part cta0[nbox].  Requires
+// nbox x deposit_cursor_words, sorted rec0[nbox], mass_part 2 cta0[nbox] (masses,
+// then corner partials).  Requires
 // deposit_shared_hist(g), nbox <= kMaxGroupBoxes and rec0[nbox] < 2^32.
 // bad_out (device-visible, one word per box, may be null) receives each box's
 // count of skipped particles, and the status word is zeroed for the next pass.

@@ -1,14 +1,15 @@
 // spectrum.cu -- fused CIC deconvolution + log-k shell binning over the
 // half-complex spectrum (the GPU counterpart of powerspectrum.c:35-111).
 //
-// Work split (k_bin, in bin_rows.cuh): each warp takes a contiguous block of (i, j) rows of N/2+1
-// modes, walked in pieces of 32*RP modes with the next piece's loads in
-// flight.  Every lane bins a contiguous run of RP modes; bins only grow along a
+// Work split (k_bin, in bin_rows.cuh): each warp takes a contiguous block of
+// (i, j) rows of N/2+1 modes, walked in pieces of 32*RP modes with the next
+// piece's loads in flight.  Every lane bins a contiguous run of RP modes; bins only grow along a
 // run, so a lane keeps one FP32 running sum per spectrum pair and compares
 // |k|^2 with the next threshold held in a register.  The lanes' open sums are
 // combined at the end of a piece by a segmented warp scan over their bins (no
 // atomics); a bin completed inside a run (only where bins are narrower than a
-// run) goes to the warp's FP32 histogram with a shared atomic.  Every 16 rows
+// run) goes to the warp's FP32 histogram: with a shared atomic for one spectrum,
+// by a plain add with the lanes in step for several.  Every 16 rows
 // the touched bins are promoted into the warp's FP64 histogram.  At the end
 // the CTA sums its warps in a fixed order and writes one FP64 partial
 // histogram; k_bin_finalize sums the partials of all CTAs in a fixed order and

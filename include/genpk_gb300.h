@@ -230,7 +230,8 @@ int genpk_set_deposit_tile(genpk_ctx *ctx, int tile_x, int tile_y, int tile_z);
  *          cell, where windows merge few adds.  (Chosen automatically for
  *          particles in no order, it takes its form without the merges; passes
  *          of fewer than 65536 such particles take that too where the
- *          accumulator is small, and count as SORTED.)
+ *          accumulator is small, and count as SORTED.)  A uniform mass below
+ *          2^-73 takes that form in WINDOW and STREAM passes as well.
  *  AUTO (default): from a sample of particle chunks, STREAM or WINDOW when the
  *          order is coherent (by window cells per particle), else SORTED. */
 #define GENPK_ENGINE_AUTO 0
